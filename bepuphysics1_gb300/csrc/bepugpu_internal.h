@@ -165,13 +165,17 @@ void PlanGroups(const GroupPolicy& pol, const int32_t* a, const int32_t* b, cons
 bepugpu_status LaunchGroups(Context* ctx, Scene* s, const StepParams& p, uint32_t flags, bool count,
                             int* launches = nullptr);
 bool SplitGroupPrologue(const Scene* s, uint32_t flags);
+bepugpu_status LaunchPrestepped(Context* ctx, Scene* s, const StepParams& p, uint32_t flags, bool count,
+                                const GroupTables& t, int* launches);  // the groups' launches after it
 // The split prologue's default: scenes whose groups hold joints and at least
-// this many constraints.  Measured on GB300: joint chains (151,073 bodies,
-// 196,608 joints) step 7 % faster split, 12 % with the added joint types;
-// contact-only groups (the 65,536-box pile, towers) 7-13 % slower, the group
-// CTA's own pass over its bodies and manifolds being cheaper there than two
-// more launches and the copy of the solve lanes.
-constexpr int32_t kSplitPrologueConstraints = 8192;
+// this many constraints.  Measured on GB300, in-kernel against split: chains
+// of 16 capsules step in 98 and 82 us at 417 constraints, 112 and 100 us at
+// 1,671, 121 and 106 us at 8,347; with the added joint types 217 and 186 us at
+// 1,671.  Smaller scenes gain too, but keep the step at one launch per kind of
+// group.  Contact-only groups (the 65,536-box pile, towers) are 7-13 % slower
+// split, the group CTA's own pass over its bodies and manifolds being cheaper
+// there than two more launches and the copy of the solve lanes.
+constexpr int32_t kSplitPrologueConstraints = 1024;
 // Joints (joints.cu): record checks, upload into the scene's joint slots, and
 // the accumulated impulses back into records.
 bepugpu_status CheckJointRecords(Context* ctx, const bepugpu_joint* joints, uint32_t nj, int32_t bodies);

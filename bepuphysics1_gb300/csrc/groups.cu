@@ -21,19 +21,9 @@
 
 #include "../../include/bepugpu.h"
 #include "bepugpu_internal.h"
-#include "groups_device.cuh"
-#include "solver_device.cuh"
+#include "groups_launch.cuh"
 
 namespace bepugpu {
-
-template <bool kCensus, bool kShared, int kJoints>
-__global__ void k_groups(ManifoldSoA m, BodySoA b, JointSoA j, StepParams p, uint32_t flags, GroupTables t,
-                         int groupBase, int Bc, int Lc, int Jc, unsigned long long* census, bool nonConvex,
-                         bool prestepped) {
-    extern __shared__ float4 smem[];
-    const GroupDesc g = t.groups[groupBase + blockIdx.x];
-    GroupStep<kCensus, kShared, kJoints>(m, b, j, p, flags, t, g, Bc, Lc, Jc, smem, census, nonConvex, prestepped);
-}
 
 // The group step's first stages as grid-wide launches (the split prologue):
 // the contact refresh of the groups' manifold slots [s0, s1) beside the
@@ -52,8 +42,22 @@ __global__ void k_group_refresh_force(ManifoldSoA m, BodySoA b, StepParams p, co
         if (flags & (BEPUGPU_STEP_FORCES | BEPUGPU_STEP_DEACTIVATION)) StartBodyStep(b, list[t - nm], p, flags);
     }
 }
-__global__ void k_group_prestep(ManifoldSoA m, BodySoA b, StepParams p, int s0, int s1) {
-    const int s = s0 + blockIdx.x * blockDim.x + threadIdx.x;
+// kJoints as k_groups': the joint slots [j0, j1) take the launch's first
+// blocks, so a warp runs either joints or manifolds.  A joint's prestep is a
+// long divergent chain (a quarter of the group kernel's cycles on joint
+// chains, its warps half empty): one thread per joint over the whole grid,
+// reading and writing global lanes, and the lanes copied into the group's
+// shared memory after, took the 196,608-joint chains from 290 to 268 us a step
+// and 384 chains of the added types from 216 to 194 us.
+template <int kJoints>
+__global__ void k_group_prestep(ManifoldSoA m, BodySoA b, JointSoA j, StepParams p, int j0, int j1, int jointBlocks,
+                                int s0, int s1) {
+    if (kJoints && (int)blockIdx.x < jointBlocks) {
+        const int q = j0 + blockIdx.x * blockDim.x + threadIdx.x;
+        if (q < j1) PrestepJoint<kJoints == 2>(j, b, q, p);
+        return;
+    }
+    const int s = s0 + (blockIdx.x - jointBlocks) * blockDim.x + threadIdx.x;
     if (s < s1) PrestepManifold(m, b, s, p);
 }
 
@@ -314,54 +318,6 @@ bepugpu_status Scene::UploadGroups(Context* ctx) {
     return BEPUGPU_OK;
 }
 
-namespace {
-int ClassThreads(const GroupClass& c, int override_) {
-    if (override_ > 0) return override_;
-    int t = ((c.maxColourMembers + 31) / 32) * 32;
-    return std::min(std::max(t, 32), 256);
-}
-
-template <bool kShared, int kJoints>
-bepugpu_status LaunchClass(Context* ctx, Scene* s, const GroupClass& c, const StepParams& p, uint32_t flags,
-                           bool count, GroupTables t, bool prestepped, int* launches) {
-    if (c.end <= c.begin) return BEPUGPU_OK;
-    const int Bc = std::max(c.maxLocal, 1), Lc = std::max(c.maxManifolds, 1), Jc = std::max(c.maxJoints, 1);
-    const bool nonConvex = s->groupPlan.nonConvexLanes;
-    size_t smemBytes = GroupSmemBytes(kShared, Bc, Lc, kJoints ? Jc : 0, nonConvex);
-    cudaError_t e = cudaSuccess;
-    if (smemBytes > 48 * 1024) {
-        e = cudaFuncSetAttribute(k_groups<false, kShared, kJoints>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smemBytes);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_groups<true, kShared, kJoints>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smemBytes);
-        if (e != cudaSuccess) {
-            ctx->SetError("group kernel shared memory %zu bytes: %s", smemBytes, cudaGetErrorString(e));
-            return BEPUGPU_CUDA_ERROR;
-        }
-    }
-    const int threads = ClassThreads(c, s->groupThreadsOverride);
-    const unsigned blocks = (unsigned)(c.end - c.begin);
-    // the thread's last error must be this launch's own
-    const cudaError_t earlier = cudaGetLastError();
-    if (count)
-        k_groups<true, kShared, kJoints><<<blocks, threads, smemBytes, s->stream>>>(
-            s->m, s->b, s->j, p, flags, t, c.begin, Bc, Lc, Jc, s->Census(), nonConvex, prestepped);
-    else
-        k_groups<false, kShared, kJoints><<<blocks, threads, smemBytes, s->stream>>>(
-            s->m, s->b, s->j, p, flags, t, c.begin, Bc, Lc, Jc, nullptr, nonConvex, prestepped);
-    if (launches) (*launches)++;
-    e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        ctx->SetError("group kernel launch (%u CTAs of %d threads, %zu bytes of shared memory): %s%s%s", blocks,
-                      threads, smemBytes, cudaGetErrorString(e), earlier != cudaSuccess ? "; earlier error: " : "",
-                      earlier != cudaSuccess ? cudaGetErrorString(earlier) : "");
-        return BEPUGPU_CUDA_ERROR;
-    }
-    return BEPUGPU_OK;
-}
-}  // namespace
-
 bool SplitGroupPrologue(const Scene* s, uint32_t flags) {
     const GroupPlan& g = s->groupPlan;
     if (g.groups.empty() || !(flags & BEPUGPU_STEP_SOLVE)) return false;
@@ -380,35 +336,27 @@ bepugpu_status LaunchGroups(Context* ctx, Scene* s, const StepParams& p, uint32_
     t.colourOffsets = s->groupColourOffsetsDev;
     t.jointRefs = s->groupJointRefsDev;
     t.jointColourOffsets = s->groupJointColourOffsetsDev;
-    const bool split = SplitGroupPrologue(s, flags);
-    if (split) {
-        // every group's manifold slots follow the sweep part's; its bodies are the body list
-        const int s0 = g.globalCount, s1 = g.groups.back().mEnd, nb = g.groups.back().bEnd;
-        const int T = 128;
-        const cudaError_t earlier = cudaGetLastError();
-        if (s1 - s0 + nb > 0)
-            k_group_refresh_force<<<(s1 - s0 + nb + T - 1) / T, T, 0, s->stream>>>(s->m, s->b, p, t.bodies, nb, s0,
-                                                                                    s1, flags);
-        if (s1 > s0) k_group_prestep<<<(s1 - s0 + T - 1) / T, T, 0, s->stream>>>(s->m, s->b, p, s0, s1);
-        if (launches) *launches += (s1 - s0 + nb > 0) + (s1 > s0);
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) {
-            ctx->SetError("group prologue launch: %s%s%s", cudaGetErrorString(e),
-                          earlier != cudaSuccess ? "; earlier error: " : "",
-                          earlier != cudaSuccess ? cudaGetErrorString(earlier) : "");
-            return BEPUGPU_CUDA_ERROR;
-        }
+    if (!SplitGroupPrologue(s, flags)) return LaunchClasses<false>(ctx, s, p, flags, count, t, launches);
+    // every group's slots follow the sweep part's; its bodies are the body list
+    const int s0 = g.globalCount, s1 = g.groups.back().mEnd, nb = g.groups.back().bEnd;
+    const int j0 = g.jointGlobalCount, j1 = g.groups.back().jEnd;
+    const int T = 128, jointBlocks = (j1 - j0 + T - 1) / T, manifoldBlocks = (s1 - s0 + T - 1) / T;
+    const cudaError_t earlier = cudaGetLastError();
+    if (s1 - s0 + nb > 0)
+        k_group_refresh_force<<<(s1 - s0 + nb + T - 1) / T, T, 0, s->stream>>>(s->m, s->b, p, t.bodies, nb, s0, s1,
+                                                                                flags);
+    auto prestep = jointBlocks == 0 ? k_group_prestep<0> : (s->addedJointTypes ? k_group_prestep<2> : k_group_prestep<1>);
+    if (jointBlocks + manifoldBlocks > 0)
+        prestep<<<jointBlocks + manifoldBlocks, T, 0, s->stream>>>(s->m, s->b, s->j, p, j0, j1, jointBlocks, s0, s1);
+    if (launches) *launches += (s1 - s0 + nb > 0) + (jointBlocks + manifoldBlocks > 0);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        ctx->SetError("group prologue launch: %s%s%s", cudaGetErrorString(e),
+                      earlier != cudaSuccess ? "; earlier error: " : "",
+                      earlier != cudaSuccess ? cudaGetErrorString(earlier) : "");
+        return BEPUGPU_CUDA_ERROR;
     }
-    bepugpu_status st = LaunchClass<true, false>(ctx, s, g.shared, p, flags, count, t, split, launches);
-    if (st == BEPUGPU_OK) st = LaunchClass<false, false>(ctx, s, g.global, p, flags, count, t, split, launches);
-    if (s->addedJointTypes) {
-        if (st == BEPUGPU_OK) st = LaunchClass<true, 2>(ctx, s, g.sharedJoints, p, flags, count, t, split, launches);
-        if (st == BEPUGPU_OK) st = LaunchClass<false, 2>(ctx, s, g.globalJoints, p, flags, count, t, split, launches);
-    } else {
-        if (st == BEPUGPU_OK) st = LaunchClass<true, 1>(ctx, s, g.sharedJoints, p, flags, count, t, split, launches);
-        if (st == BEPUGPU_OK) st = LaunchClass<false, 1>(ctx, s, g.globalJoints, p, flags, count, t, split, launches);
-    }
-    return st;
+    return LaunchPrestepped(ctx, s, p, flags, count, t, launches);
 }
 
 }  // namespace bepugpu

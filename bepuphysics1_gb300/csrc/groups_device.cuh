@@ -67,17 +67,16 @@ __host__ __device__ constexpr size_t GroupSmemBytes(bool shared, int bodies, int
 // contact friction lanes (GroupManifoldLanes); a NONCONVEX manifold keeps its
 // friction direction and impulse in lanes 12-15 (the sliding lanes it does not
 // use), its prestep angular A in lanes 16-19 and angular B in lanes 25-28.
-// prestepped: the group's bodies went through the candidacy and force updates
-// and its manifolds through the refresh and the prestep in grid-wide launches
-// before this one (k_group_refresh_force, k_group_prestep), so the step starts
-// by copying bodies and manifold solve lanes into shared memory; the group's
-// joints are prestepped here as without it.
-template <bool kCensus, bool kShared, int kJoints>
+// kPrestepped: the group's bodies went through the candidacy and force updates,
+// its manifolds through the refresh and the prestep and its joints through
+// theirs in grid-wide launches before this one (k_group_refresh_force,
+// k_group_prestep), so the step starts by copying bodies and solve lanes into
+// shared memory and the kernel holds none of the prestep's code.
+template <bool kCensus, bool kShared, int kJoints, bool kPrestepped = false>
 __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b, const JointSoA& jt,
                                           const StepParams& p, uint32_t flags, const GroupTables& t,
                                           const GroupDesc& g, int Bc, int Lc, int Jc, float4* smem,
-                                          unsigned long long* census, bool nonConvex = false,
-                                          bool prestepped = false) {
+                                          unsigned long long* census, bool nonConvex = false) {
     const int nLocal = g.bEnd - g.bBegin, nm = g.mEnd - g.mBegin;
     GroupBodies bv;
     bv.pos = smem;
@@ -137,7 +136,7 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
     // sleeping island skips the force update and reads as not dynamic for the
     // rest of the step: pos.w = 0 in shared memory.
     int asleepAll = b.islandOf != nullptr;
-    if (prestepped) {
+    if (kPrestepped) {
         // Bodies, then (shared lanes) every solve lane the prestep wrote, as
         // asynchronous copies; a sleeping body's pos.w is cleared after them.
         for (int i = tid; i < nLocal; i += T) {
@@ -192,6 +191,14 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
             for (int j = tid; j < nm; j += T)
                 atomicAdd(census + 3, 288ull + 112ull * (unsigned long long)(m.head[g.mBegin + j].z & 0xff));
         }
+        if (kJoints)  // consecutive threads, consecutive slots of a lane
+            for (int q = tid; q < nj; q += T) {
+                const int s = g.jBegin + q;
+#pragma unroll
+                for (int k = 0; k < kJSolveLanes; k++) CopyAsync16(&jl.L(k, q), &jt.L(k, s));
+                CopyAsync8(jl.state + q, jt.state + s);
+                CopyAsync8(jRefs + q, t.jointRefs + s);
+            }
         CopyAsyncWait();
         for (int i = tid; i < nLocal; i += T) {
             const bool asleep = IslandAsleep(b, t.bodies[g.bBegin + i]);
@@ -231,7 +238,7 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
     // of its islands would have woken it), no body to move.
     if (__syncthreads_and(asleepAll)) return;
     // Refresh, lanes in, prestep: a thread keeps the same manifolds throughout.
-    if (!prestepped) {
+    if (!kPrestepped) {
         for (int j = tid; j < nm; j += T) {
             const int s = g.mBegin + j;
             int2 r = t.refs[s];
@@ -257,7 +264,7 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
             }
         }
     }
-    if (kJoints && (flags & BEPUGPU_STEP_SOLVE))
+    if (kJoints && !kPrestepped && (flags & BEPUGPU_STEP_SOLVE))
         for (int q = tid; q < nj; q += T) {
             const int2 r = t.jointRefs[g.jBegin + q];
             jRefs[q] = r;
