@@ -462,33 +462,23 @@ __global__ void k_prestep(ManifoldSoA m, BodySoA b, StepParams p) {
     if (s < m.count) PrestepManifold(m, b, s, p);
 }
 
-__device__ __forceinline__ void LoadPair(const BodySoA& b, int4 h, BodyState& A, BodyState& B) {
-    if (h.x >= 0) LoadBody(b, h.x, A);
-    if (h.y >= 0) LoadBody(b, h.y, B);
-}
-__device__ __forceinline__ void StorePair(const BodySoA& b, int4 h, uint32_t st, const BodyState& A,
-                                          const BodyState& B) {
-    if (st & kDynA) StoreVelocity(b, h.x, A);
-    if (st & kDynB) StoreVelocity(b, h.y, B);
-}
-
 __device__ __forceinline__ void WarmSlot(const ManifoldSoA& m, const BodySoA& b, int s) {
     uint2 state = m.state[s];
     if (!(state.x & kGroupActive)) return;
     int4 h = m.head[s];
     BodyState A, B;
-    LoadPair(b, h, A, B);
-    WarmStartManifold(m, s, A, B, state.x, h.z & 0xff);
-    StorePair(b, h, state.x, A, B);
+    LoadVisit(GlobalBodies{b}, h.x, h.y, state.x, A, B);
+    WarmStartManifold(m, s, A, B, state);
+    StoreVisit(GlobalBodies{b}, h.x, h.y, state.x, A, B);
 }
 __device__ __forceinline__ void SolveSlot(const ManifoldSoA& m, const BodySoA& b, int s, const StepParams& p) {
     uint2 state = m.state[s];
     if (!(state.x & kGroupActive)) return;
     int4 h = m.head[s];
     BodyState A, B;
-    LoadPair(b, h, A, B);
-    SolveManifold(m, s, A, B, state, h.z & 0xff, p);
-    StorePair(b, h, state.x, A, B);
+    LoadVisit(GlobalBodies{b}, h.x, h.y, state.x, A, B);
+    SolveManifold(m, s, A, B, state, p);
+    StoreVisit(GlobalBodies{b}, h.x, h.y, state.x, A, B);
     m.state[s] = state;
 }
 
@@ -505,17 +495,19 @@ __global__ void k_solve(ManifoldSoA m, BodySoA b, StepParams p, int begin, int e
     int4 h = make_int4(0, 0, 0, 0);
     if (s < end) {
         h = m.head[s];
+        // a superset of the active children: the contacts', sliding and twist
+        const uint32_t flags = (uint32_t)h.z >> 8 & kManifoldNonConvex ? kContactFriction : 0u;
         const int count = h.z & 0xff;
-        LoadSolveLanes(m, s, count, count > 0, L);
+        LoadSolveLanes(m, s, flags, count ? 0xff000000u | ((~0u << (4 * count)) & 0xffffu) : ~0u, L);
     }
     WaitForPrerequisites();
     if (s >= end) return;
     uint2 state = m.state[s];
     if (!(state.x & kGroupActive)) return;
     BodyState A, B;
-    LoadPair(b, h, A, B);
-    SolveManifold(m, s, A, B, state, h.z & 0xff, p, &L);
-    StorePair(b, h, state.x, A, B);
+    LoadVisit(GlobalBodies{b}, h.x, h.y, state.x, A, B);
+    SolveManifold(m, s, A, B, state, p, &L);
+    StoreVisit(GlobalBodies{b}, h.x, h.y, state.x, A, B);
     m.state[s] = state;
 }
 
@@ -529,11 +521,9 @@ __device__ __forceinline__ void WarmJointSlot(const JointSoA& j, const BodySoA& 
     if (!(st.x & kGroupActive)) return;
     int4 h = j.head[s];
     BodyState A, B;
-    LoadJointVelocityV(GlobalBodies{b}, h.x, A);
-    LoadJointVelocityV(GlobalBodies{b}, h.y, B);
+    LoadVisit(GlobalBodies{b}, h.x, h.y, st.x, A, B);
     WarmJoint<kAdded>(j, s, A, B, st.x, h.z & 0xff);
-    if (st.x & kDynA) StoreVelocity(b, h.x, A);
-    if (st.x & kDynB) StoreVelocity(b, h.y, B);
+    StoreVisit(GlobalBodies{b}, h.x, h.y, st.x, A, B);
 }
 template <bool kAdded>
 __device__ __forceinline__ void SolveJointSlot(const JointSoA& j, const BodySoA& b, int s, const StepParams& p) {
@@ -541,11 +531,9 @@ __device__ __forceinline__ void SolveJointSlot(const JointSoA& j, const BodySoA&
     if (!(st.x & kGroupActive)) return;
     int4 h = j.head[s];
     BodyState A, B;
-    LoadJointVelocityV(GlobalBodies{b}, h.x, A);
-    LoadJointVelocityV(GlobalBodies{b}, h.y, B);
+    LoadVisit(GlobalBodies{b}, h.x, h.y, st.x, A, B);
     SolveJoint<kAdded>(j, s, A, B, st, h.z & 0xff, p);
-    if (st.x & kDynA) StoreVelocity(b, h.x, A);
-    if (st.x & kDynB) StoreVelocity(b, h.y, B);
+    StoreVisit(GlobalBodies{b}, h.x, h.y, st.x, A, B);
     j.state[s] = st;
 }
 template <bool kAdded>

@@ -282,11 +282,9 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
                     if (!(st.x & kGroupActive)) continue;
                     const int2 r = jRefs[q];
                     BodyState A, B;
-                    LoadJointVelocityV(bv, r.x, A);
-                    LoadJointVelocityV(bv, r.y, B);
+                    LoadVisit(bv, r.x, r.y, st.x, A, B);
                     WarmJoint<kJoints == 2>(jl, q, A, B, st.x, JointType(st.x));
-                    if (st.x & kDynA) StoreVelocityV(bv, r.x, A);
-                    if (st.x & kDynB) StoreVelocityV(bv, r.y, B);
+                    StoreVisit(bv, r.x, r.y, st.x, A, B);
                 }
             for (int j = co[c] + tid; j < co[c + 1]; j += T) {
                 const int sl = lbase + j;
@@ -294,11 +292,9 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
                 if (!(st.x & kGroupActive)) continue;
                 int2 r = kShared ? sRefs[j] : t.refs[g.mBegin + j];
                 BodyState A, B;
-                if (r.x != -1) LoadBodyV(bv, r.x, A);
-                if (r.y != -1) LoadBodyV(bv, r.y, B);
-                WarmStartManifold(ml, sl, A, B, st.x, ml.head[sl].z & 0xff);
-                if (st.x & kDynA) StoreVelocityV(bv, r.x, A);
-                if (st.x & kDynB) StoreVelocityV(bv, r.y, B);
+                LoadVisit(bv, r.x, r.y, st.x, A, B);
+                WarmStartManifold(ml, sl, A, B, st);
+                StoreVisit(bv, r.x, r.y, st.x, A, B);
             }
             __syncthreads();
         }
@@ -310,11 +306,9 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
                         if (!(st.x & kGroupActive)) continue;
                         const int2 r = jRefs[q];
                         BodyState A, B;
-                        LoadJointVelocityV(bv, r.x, A);
-                        LoadJointVelocityV(bv, r.y, B);
+                        LoadVisit(bv, r.x, r.y, st.x, A, B);
                         SolveJoint<kJoints == 2>(jl, q, A, B, st, JointType(st.x), p);
-                        if (st.x & kDynA) StoreVelocityV(bv, r.x, A);
-                        if (st.x & kDynB) StoreVelocityV(bv, r.y, B);
+                        StoreVisit(bv, r.x, r.y, st.x, A, B);
                         jl.state[q] = st;
                     }
                 for (int j = co[c] + tid; j < co[c + 1]; j += T) {
@@ -322,19 +316,17 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
                     uint2 st = ml.state[sl];
                     if (!(st.x & kGroupActive)) continue;
                     int2 r = kShared ? sRefs[j] : t.refs[g.mBegin + j];
-                    const int count = ml.head[sl].z & 0xff;
                     BodyState A, B;
-                    if (r.x != -1) LoadBodyV(bv, r.x, A);
-                    if (r.y != -1) LoadBodyV(bv, r.y, B);
+                    LoadVisit(bv, r.x, r.y, st.x, A, B);
                     if (kCensus) {  // algorithmic bytes of the visit: 76 d + 136 + 48 c
+                        const int count = ml.head[sl].z & 0xff;
                         int d = ((st.x & kDynA) ? 1 : 0) + ((st.x & kDynB) ? 1 : 0);
                         atomicAdd(census, 76ull * d + 136ull + 48ull * count);
                         atomicAdd(census + 1, 1ull);
                         atomicAdd(census + 2, (unsigned long long)count);
                     }
-                    SolveManifold(ml, sl, A, B, st, count, p);
-                    if (st.x & kDynA) StoreVelocityV(bv, r.x, A);
-                    if (st.x & kDynB) StoreVelocityV(bv, r.y, B);
+                    SolveManifold(ml, sl, A, B, st, p);
+                    StoreVisit(bv, r.x, r.y, st.x, A, B);
                     ml.state[sl] = st;
                 }
                 __syncthreads();

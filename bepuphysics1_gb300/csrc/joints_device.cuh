@@ -104,6 +104,7 @@ enum : uint32_t {
 // iterations << 16.  Word y: 4-bit zero-impulse streaks of the three
 // children.
 enum : uint32_t {
+    kChildShift = 1,
     kJMinActive = 1u << 4,
     kJMaxActive = 1u << 5,
     kJTypeShift = 9,
@@ -368,36 +369,20 @@ __device__ __forceinline__ float4 JQuatBetween(float3 v1, float3 v2) {
     }
     return JQNormalize(q);
 }
-// Velocity-only view for the warm start and the solve.
-template <class V>
-__device__ __forceinline__ void LoadJointVelocityV(const V& bv, int r, BodyState& s) {
-    if (r == -1) {
-        s.vx = s.vy = s.vz = 0.f; s.invMass = 0.f;
-        s.wx = s.wy = s.wz = 0.f;
-        s.I11 = s.I12 = s.I13 = s.I21 = s.I22 = s.I23 = s.I31 = s.I32 = s.I33 = 0.f;
-        return;
-    }
-    LoadBodyV(bv, r, s);
-}
-
 // PointOnLineJoint's impulse on both connections (SolveIteration and
 // ExclusiveUpdate, PointOnLineJoint.cs:318-355, 440-463).  Lanes: kJOA rA,
 // kJOB rB, kJM0 / kJM1 the world restricted axes; the angular jacobians are
 // their cross products with rA and rB, recomputed as the reference computed them.
 __device__ __forceinline__ void ApplyPointOnLine(float4 oa, float4 ob, float4 m0, float4 m1, float x, float y,
-                                                 bool dynA, bool dynB, BodyState& A, BodyState& B) {
+                                                 BodyState& A, BodyState& B) {
     const float3 rA = JXYZ(oa), rB = JXYZ(ob), ax1 = JXYZ(m0), ax2 = JXYZ(m1);
     float ix = ax1.x * x + ax2.x * y, iy = ax1.y * x + ax2.y * y, iz = ax1.z * x + ax2.z * y;
-    if (dynA) {
-        const float3 a1 = JCross(rA, ax1), a2 = JCross(rA, ax2);
-        ApplyLinear(A, ix, iy, iz);
-        ApplyAngular(A, x * a1.x + y * a2.x, x * a1.y + y * a2.y, x * a1.z + y * a2.z);
-    }
-    if (dynB) {
-        const float3 b1 = JCross(ax1, rB), b2 = JCross(ax2, rB);
-        ApplyLinear(B, -ix, -iy, -iz);
-        ApplyAngular(B, x * b1.x + y * b2.x, x * b1.y + y * b2.y, x * b1.z + y * b2.z);
-    }
+    const float3 a1 = JCross(rA, ax1), a2 = JCross(rA, ax2);
+    ApplyLinear(A, ix, iy, iz);
+    ApplyAngular(A, x * a1.x + y * a2.x, x * a1.y + y * a2.y, x * a1.z + y * a2.z);
+    const float3 b1 = JCross(ax1, rB), b2 = JCross(ax2, rB);
+    ApplyLinear(B, -ix, -iy, -iz);
+    ApplyAngular(B, x * b1.x + y * b2.x, x * b1.y + y * b2.y, x * b1.z + y * b2.z);
 }
 
 // ------------------------------------------------------------- prestep --
@@ -1358,75 +1343,61 @@ __device__ __forceinline__ void PrestepJoint(const JointSoA& j, const BodySoA& b
 template <bool kAdded>
 __device__ __forceinline__ void WarmJointChildren(const JointSoA& j, int s, BodyState& A, BodyState& B, uint32_t st,
                                                   int type) {
-    const bool dynA = st & kDynA, dynB = st & kDynB;
     const float4 acc0 = j.L(kJACC0, s), acc1 = j.L(kJACC1, s);
     if (kAdded && (st & (1u << kChildShift)) && IsPointOnLineType(type)) {
         // PointOnLineJoint.ExclusiveUpdate (PointOnLineJoint.cs:440-463)
-        ApplyPointOnLine(j.L(kJOA, s), j.L(kJOB, s), j.L(kJM0, s), j.L(kJM1, s), acc0.x, acc0.y, dynA, dynB, A, B);
+        ApplyPointOnLine(j.L(kJOA, s), j.L(kJOB, s), j.L(kJM0, s), j.L(kJM1, s), acc0.x, acc0.y, A, B);
     } else if (kAdded && (st & (1u << kChildShift)) && IsPointOnPlaneType(type)) {
         // PointOnPlaneJoint.ExclusiveUpdate (PointOnPlaneJoint.cs:308-328)
         const float4 m0 = j.L(kJM0, s), m1 = j.L(kJM1, s), m2 = j.L(kJM2, s);
         const float a = acc0.x;
         const float ix = m0.x * a, iy = m0.y * a, iz = m0.z * a;
-        if (dynA) {
-            ApplyLinear(A, ix, iy, iz);
-            ApplyAngular(A, m1.x * a, m1.y * a, m1.z * a);
-        }
-        if (dynB) {
-            ApplyLinear(B, -ix, -iy, -iz);
-            ApplyAngular(B, m2.x * a, m2.y * a, m2.z * a);
-        }
+        ApplyLinear(A, ix, iy, iz);
+        ApplyAngular(A, m1.x * a, m1.y * a, m1.z * a);
+        ApplyLinear(B, -ix, -iy, -iz);
+        ApplyAngular(B, m2.x * a, m2.y * a, m2.z * a);
     } else if (kAdded && (st & (1u << kChildShift)) && IsDistanceType(type)) {
         // DistanceJoint / DistanceLimit.ExclusiveUpdate (DistanceJoint.cs:354-380)
         const float4 m0 = j.L(kJM0, s), m1 = j.L(kJM1, s), m2 = j.L(kJM2, s);
         const float a = acc0.x;
-        if (dynA) {
-            ApplyLinear(A, m0.x * a, m0.y * a, m0.z * a);
-            ApplyAngular(A, m1.x * a, m1.y * a, m1.z * a);
-        }
-        if (dynB) {
-            ApplyLinear(B, -m0.x * a, -m0.y * a, -m0.z * a);
-            ApplyAngular(B, m2.x * a, m2.y * a, m2.z * a);
-        }
+        ApplyLinear(A, m0.x * a, m0.y * a, m0.z * a);
+        ApplyAngular(A, m1.x * a, m1.y * a, m1.z * a);
+        ApplyLinear(B, -m0.x * a, -m0.y * a, -m0.z * a);
+        ApplyAngular(B, m2.x * a, m2.y * a, m2.z * a);
     } else if (st & (1u << kChildShift)) {
         // BallSocketJoint.ExclusiveUpdate (BallSocketJoint.cs:285-311)
         const float3 offA = JXYZ(j.L(kJOA, s)), offB = JXYZ(j.L(kJOB, s));
         const float3 acc = make_float3(acc0.x, acc0.y, acc0.z);
-        if (dynA) {
-            float3 lin = make_float3(-acc.x, -acc.y, -acc.z);
-            ApplyLinear(A, lin.x, lin.y, lin.z);
-            float3 t = JCross(offA, lin);
-            ApplyAngular(A, t.x, t.y, t.z);
-        }
-        if (dynB) {
-            ApplyLinear(B, acc.x, acc.y, acc.z);
-            float3 t = JCross(offB, acc);
-            ApplyAngular(B, t.x, t.y, t.z);
-        }
+        float3 lin = make_float3(-acc.x, -acc.y, -acc.z);
+        ApplyLinear(A, lin.x, lin.y, lin.z);
+        const float3 ta = JCross(offA, lin), tb = JCross(offB, acc);
+        ApplyAngular(A, ta.x, ta.y, ta.z);
+        ApplyLinear(B, acc.x, acc.y, acc.z);
+        ApplyAngular(B, tb.x, tb.y, tb.z);
     }
     if (kAdded && (st & (2u << kChildShift)) && IsTwistType(type)) {
         // TwistJoint.ExclusiveUpdate (TwistJoint.cs:302-317)
         const float4 w1 = j.L(kJW1, s);
         const float a = acc0.w;
-        if (dynA) ApplyAngular(A, -w1.x * a, -w1.y * a, -w1.z * a);
-        if (dynB) ApplyAngular(B, w1.x * a, w1.y * a, w1.z * a);
+        ApplyAngular(A, -w1.x * a, -w1.y * a, -w1.z * a);
+        ApplyAngular(B, w1.x * a, w1.y * a, w1.z * a);
     } else if (kAdded && (st & (2u << kChildShift)) && IsNoRotationType(type)) {
         // NoRotationJoint.ExclusiveUpdate (NoRotationJoint.cs:245-259)
-        if (dynA) ApplyAngular(A, acc0.w, acc1.x, acc1.y);
-        if (dynB) ApplyAngular(B, -acc0.w, -acc1.x, -acc1.y);
+        ApplyAngular(A, acc0.w, acc1.x, acc1.y);
+        ApplyAngular(B, -acc0.w, -acc1.x, -acc1.y);
     } else if (kAdded && (st & (2u << kChildShift)) && IsSwivelType(type)) {
         // SwivelHingeAngularJoint.ExclusiveUpdate (SwivelHingeAngularJoint.cs:272-287)
         const float4 w1 = j.L(kJW1, s);
         const float a = acc0.w;
-        if (dynA) ApplyAngular(A, w1.x * a, w1.y * a, w1.z * a);
-        if (dynB) ApplyAngular(B, -w1.x * a, -w1.y * a, -w1.z * a);
+        ApplyAngular(A, w1.x * a, w1.y * a, w1.z * a);
+        ApplyAngular(B, -w1.x * a, -w1.y * a, -w1.z * a);
     } else if (st & (2u << kChildShift)) {
         // RevoluteAngularJoint.ExclusiveUpdate (RevoluteAngularJoint.cs:291-310)
         const float3 c1 = JXYZ(j.L(kJW1, s)), c2 = JXYZ(j.L(kJW2, s));
         float ix = c1.x * acc0.w + c2.x * acc1.x, iy = c1.y * acc0.w + c2.y * acc1.x,
               iz = c1.z * acc0.w + c2.z * acc1.x;
-        if (dynA) ApplyAngular(A, ix, iy, iz);
-        if (dynB) ApplyAngular(B, -ix, -iy, -iz);
+        ApplyAngular(A, ix, iy, iz);
+        ApplyAngular(B, -ix, -iy, -iz);
     }
     if (st & (4u << kChildShift)) {
         const float4 l0 = j.L(kJL0, s);
@@ -1439,8 +1410,8 @@ __device__ __forceinline__ void WarmJointChildren(const JointSoA& j, int s, Body
         } else if (kAdded && IsAngularMotorType(type)) {
             // AngularMotor.ExclusiveUpdate (AngularMotor.cs:314-326), SingleEntityAngularMotor's
             // (:215-218; B is the world there)
-            if (dynA) ApplyAngular(A, acc0.x, acc0.y, acc0.z);
-            if (dynB) ApplyAngular(B, -acc0.x, -acc0.y, -acc0.z);
+            ApplyAngular(A, acc0.x, acc0.y, acc0.z);
+            ApplyAngular(B, -acc0.x, -acc0.y, -acc0.z);
         } else if (kAdded && IsSpeedLimitType(type)) {
             // ExclusiveUpdate (MaximumLinearVelocityConstraint.cs:195-199): no warm start, the
             // accumulated impulse starts the iterations from zero
@@ -1449,55 +1420,43 @@ __device__ __forceinline__ void WarmJointChildren(const JointSoA& j, int s, Body
             // LinearAxisMotor.ExclusiveUpdate (LinearAxisMotor.cs:370-390)
             const float4 jaa = j.L(kJL1, s), jab = j.L(kJL2, s);
             const float a = acc1.y;
-            if (dynA) {
-                ApplyLinear(A, l0.x * a, l0.y * a, l0.z * a);
-                ApplyAngular(A, jaa.x * a, jaa.y * a, jaa.z * a);
-            }
-            if (dynB) {
-                ApplyLinear(B, -l0.x * a, -l0.y * a, -l0.z * a);
-                ApplyAngular(B, jab.x * a, jab.y * a, jab.z * a);
-            }
+            ApplyLinear(A, l0.x * a, l0.y * a, l0.z * a);
+            ApplyAngular(A, jaa.x * a, jaa.y * a, jaa.z * a);
+            ApplyLinear(B, -l0.x * a, -l0.y * a, -l0.z * a);
+            ApplyAngular(B, jab.x * a, jab.y * a, jab.z * a);
         } else if (kAdded && (type == BEPUGPU_JOINT_TWIST_LIMIT || type == BEPUGPU_JOINT_ELLIPSE_SWING_LIMIT ||
                               type == BEPUGPU_JOINT_REVOLUTE_MOTOR || type == BEPUGPU_JOINT_TWIST_MOTOR)) {
             // TwistLimit.ExclusiveUpdate (TwistLimit.cs:368-383), EllipseSwingLimit's (:310-325),
             // RevoluteMotor's (RevoluteMotor.cs:292-307), TwistMotor's (TwistMotor.cs:255-270)
             const float a = acc1.y;
-            if (dynA) ApplyAngular(A, l0.x * a, l0.y * a, l0.z * a);
-            if (dynB) ApplyAngular(B, -l0.x * a, -l0.y * a, -l0.z * a);
+            ApplyAngular(A, l0.x * a, l0.y * a, l0.z * a);
+            ApplyAngular(B, -l0.x * a, -l0.y * a, -l0.z * a);
         } else if (kAdded && IsLinearLimitType(type)) {
             // LinearAxisLimit.ExclusiveUpdate (LinearAxisLimit.cs:449-466)
             const int k0 = LinearLimitLane(type);
             const float4 ja = j.L(k0, s), jaa = j.L(k0 + 1, s), jab = j.L(k0 + 2, s);
             const float a = acc1.z;
-            if (dynA) {
-                ApplyLinear(A, ja.x * a, ja.y * a, ja.z * a);
-                ApplyAngular(A, jaa.x * a, jaa.y * a, jaa.z * a);
-            }
-            if (dynB) {
-                ApplyLinear(B, -ja.x * a, -ja.y * a, -ja.z * a);
-                ApplyAngular(B, jab.x * a, jab.y * a, jab.z * a);
-            }
+            ApplyLinear(A, ja.x * a, ja.y * a, ja.z * a);
+            ApplyAngular(A, jaa.x * a, jaa.y * a, jaa.z * a);
+            ApplyLinear(B, -ja.x * a, -ja.y * a, -ja.z * a);
+            ApplyAngular(B, jab.x * a, jab.y * a, jab.z * a);
         } else if (type == BEPUGPU_JOINT_SWING_LIMIT) {
             // SwingLimit.ExclusiveUpdate (SwingLimit.cs:333-347)
             float ix = l0.x * acc1.y, iy = l0.y * acc1.y, iz = l0.z * acc1.y;
-            if (dynA) ApplyAngular(A, ix, iy, iz);
-            if (dynB) ApplyAngular(B, -ix, -iy, -iz);
+            ApplyAngular(A, ix, iy, iz);
+            ApplyAngular(B, -ix, -iy, -iz);
         } else {
             // RevoluteLimit.ExclusiveUpdate (RevoluteLimit.cs:577-620)
             const float4 l1 = j.L(kJL1, s);
             const bool minOn = st & kJMinActive, maxOn = st & kJMaxActive;
-            if (dynA) {
-                float ix = 0.f, iy = 0.f, iz = 0.f;
-                if (minOn) { ix = l0.x * acc1.y; iy = l0.y * acc1.y; iz = l0.z * acc1.y; }
-                if (maxOn) { ix = ix + l1.x * acc1.z; iy = iy + l1.y * acc1.z; iz = iz + l1.z * acc1.z; }
-                ApplyAngular(A, ix, iy, iz);
-            }
-            if (dynB) {
-                float ix = 0.f, iy = 0.f, iz = 0.f;
-                if (minOn) { ix = -l0.x * acc1.y; iy = -l0.y * acc1.y; iz = -l0.z * acc1.y; }
-                if (maxOn) { ix = ix + -l1.x * acc1.z; iy = iy + -l1.y * acc1.z; iz = iz + -l1.z * acc1.z; }
-                ApplyAngular(B, ix, iy, iz);
-            }
+            float ix = 0.f, iy = 0.f, iz = 0.f;
+            if (minOn) { ix = l0.x * acc1.y; iy = l0.y * acc1.y; iz = l0.z * acc1.y; }
+            if (maxOn) { ix = ix + l1.x * acc1.z; iy = iy + l1.y * acc1.z; iz = iz + l1.z * acc1.z; }
+            ApplyAngular(A, ix, iy, iz);
+            ix = iy = iz = 0.f;
+            if (minOn) { ix = -l0.x * acc1.y; iy = -l0.y * acc1.y; iz = -l0.z * acc1.y; }
+            if (maxOn) { ix = ix + -l1.x * acc1.z; iy = iy + -l1.y * acc1.z; iz = iz + -l1.z * acc1.z; }
+            ApplyAngular(B, ix, iy, iz);
         }
     }
 }
@@ -1527,18 +1486,13 @@ template <bool kAdded>
 __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, BodyState& A, BodyState& B,
                                                    uint32_t& st, uint32_t& zeros, int& activeConstraints, int type,
                                                    const StepParams& p) {
-    const bool dynA = st & kDynA, dynB = st & kDynB;
     auto account = [&](int c, float r) {
-        uint32_t z = (zeros >> (4 * c)) & 0xfu;
-        if (r < p.minimumImpulse) {
-            z++;
-            if ((int)z > p.minimumIterationCount) st &= ~(1u << (kChildShift + c));
-            else activeConstraints++;
-        } else {
-            z = 0;
-            activeConstraints++;
-        }
-        zeros = (zeros & ~(0xfu << (4 * c))) | ((z & 0xfu) << (4 * c));
+        const uint32_t nibble = 0xfu << (4 * c);
+        const bool still = r < p.minimumImpulse;
+        zeros = (zeros & ~nibble) | (still ? (zeros + (1u << (4 * c))) & nibble : 0u);
+        const bool stop = still && (int)((zeros >> (4 * c)) & 0xfu) > p.minimumIterationCount;
+        st = stop ? st & ~(1u << (kChildShift + c)) : st;
+        activeConstraints += stop ? 0 : 1;
     };
     float4 acc0 = j.L(kJACC0, s), acc1 = j.L(kJACC1, s);
     if (kAdded && (st & (1u << kChildShift)) && IsPointOnLineType(type)) {
@@ -1557,7 +1511,7 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
         const float x = lx * m0.w + ly * m2.x, y = lx * m1.w + ly * m2.y;  // Matrix2x2.Transform
         acc0.x = x + acc0.x;
         acc0.y = y + acc0.y;
-        ApplyPointOnLine(oa, ob, m0, m1, x, y, dynA, dynB, A, B);
+        ApplyPointOnLine(oa, ob, m0, m1, x, y, A, B);
         account(0, fabsf(x) + fabsf(y));
     } else if (kAdded && (st & (1u << kChildShift)) && IsPointOnPlaneType(type)) {
         // PointOnPlaneJoint.SolveIteration (PointOnPlaneJoint.cs:212-243)
@@ -1572,14 +1526,10 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
         const float lambda = m0.w * (vd + m1.w + oa.w * acc0.x);
         acc0.x += lambda;
         const float ix = m0.x * lambda, iy = m0.y * lambda, iz = m0.z * lambda;
-        if (dynA) {
-            ApplyLinear(A, ix, iy, iz);
-            ApplyAngular(A, m1.x * lambda, m1.y * lambda, m1.z * lambda);
-        }
-        if (dynB) {
-            ApplyLinear(B, -ix, -iy, -iz);
-            ApplyAngular(B, m2.x * lambda, m2.y * lambda, m2.z * lambda);
-        }
+        ApplyLinear(A, ix, iy, iz);
+        ApplyAngular(A, m1.x * lambda, m1.y * lambda, m1.z * lambda);
+        ApplyLinear(B, -ix, -iy, -iz);
+        ApplyAngular(B, m2.x * lambda, m2.y * lambda, m2.z * lambda);
         account(0, lambda);  // signed, as the reference returns it
     } else if (kAdded && (st & (1u << kChildShift)) && IsDistanceType(type)) {
         // DistanceJoint.SolveIteration (DistanceJoint.cs:226-268) /
@@ -1603,14 +1553,10 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
             acc0.x = Maxf(acc0.x + lambda, 0);
             lambda = acc0.x - previous;
         }
-        if (dynA) {
-            ApplyLinear(A, m0.x * lambda, m0.y * lambda, m0.z * lambda);
-            ApplyAngular(A, m1.x * lambda, m1.y * lambda, m1.z * lambda);
-        }
-        if (dynB) {
-            ApplyLinear(B, bx * lambda, by * lambda, bz * lambda);
-            ApplyAngular(B, m2.x * lambda, m2.y * lambda, m2.z * lambda);
-        }
+        ApplyLinear(A, m0.x * lambda, m0.y * lambda, m0.z * lambda);
+        ApplyAngular(A, m1.x * lambda, m1.y * lambda, m1.z * lambda);
+        ApplyLinear(B, bx * lambda, by * lambda, bz * lambda);
+        ApplyAngular(B, m2.x * lambda, m2.y * lambda, m2.z * lambda);
         account(0, fabsf(lambda));
     } else if (st & (1u << kChildShift)) {
         // BallSocketJoint.SolveIteration (BallSocketJoint.cs:318-372)
@@ -1631,15 +1577,11 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
         acc0.x = acc0.x + tx;
         acc0.y = acc0.y + ty;
         acc0.z = acc0.z + tz;
-        if (dynA) {
-            float nx = -tx, ny = -ty, nz = -tz;
-            ApplyLinear(A, nx, ny, nz);
-            ApplyAngular(A, oa.y * nz - oa.z * ny, oa.z * nx - oa.x * nz, oa.x * ny - oa.y * nx);
-        }
-        if (dynB) {
-            ApplyLinear(B, tx, ty, tz);
-            ApplyAngular(B, ob.y * tz - ob.z * ty, ob.z * tx - ob.x * tz, ob.x * ty - ob.y * tx);
-        }
+        float nx = -tx, ny = -ty, nz = -tz;
+        ApplyLinear(A, nx, ny, nz);
+        ApplyAngular(A, oa.y * nz - oa.z * ny, oa.z * nx - oa.x * nz, oa.x * ny - oa.y * nx);
+        ApplyLinear(B, tx, ty, tz);
+        ApplyAngular(B, ob.y * tz - ob.z * ty, ob.z * tx - ob.x * tz, ob.x * ty - ob.y * tx);
         account(0, fabsf(tx) + fabsf(ty) + fabsf(tz));
     }
     if (kAdded && (st & (2u << kChildShift)) && IsTwistType(type)) {
@@ -1652,8 +1594,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
         float lambda = -(velocityA + velocityB) + w2.x - softness * acc0.w;
         lambda *= w1.w;
         acc0.w += lambda;
-        if (dynA) ApplyAngular(A, jax * lambda, jay * lambda, jaz * lambda);
-        if (dynB) ApplyAngular(B, w1.x * lambda, w1.y * lambda, w1.z * lambda);
+        ApplyAngular(A, jax * lambda, jay * lambda, jaz * lambda);
+        ApplyAngular(B, w1.x * lambda, w1.y * lambda, w1.z * lambda);
         account(1, fabsf(lambda));
     } else if (kAdded && (st & (2u << kChildShift)) && IsNoRotationType(type)) {
         // NoRotationJoint.SolveIteration (NoRotationJoint.cs:160-187)
@@ -1670,8 +1612,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
         acc0.w = tx + acc0.w;
         acc1.x = ty + acc1.x;
         acc1.y = tz + acc1.y;
-        if (dynA) ApplyAngular(A, tx, ty, tz);
-        if (dynB) ApplyAngular(B, -tx, -ty, -tz);
+        ApplyAngular(A, tx, ty, tz);
+        ApplyAngular(B, -tx, -ty, -tz);
         account(1, fabsf(tx) + fabsf(ty) + fabsf(tz));
     } else if (kAdded && (st & (2u << kChildShift)) && IsSwivelType(type)) {
         // SwivelHingeAngularJoint.SolveIteration (SwivelHingeAngularJoint.cs:193-220)
@@ -1683,8 +1625,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
         float lambda = -(velocityA + velocityB) - w2.x - softness * acc0.w;
         lambda *= w1.w;
         acc0.w += lambda;
-        if (dynA) ApplyAngular(A, w1.x * lambda, w1.y * lambda, w1.z * lambda);
-        if (dynB) ApplyAngular(B, jbx * lambda, jby * lambda, jbz * lambda);
+        ApplyAngular(A, w1.x * lambda, w1.y * lambda, w1.z * lambda);
+        ApplyAngular(B, jbx * lambda, jby * lambda, jbz * lambda);
         account(1, fabsf(lambda));
     } else if (st & (2u << kChildShift)) {
         // RevoluteAngularJoint.SolveIteration (RevoluteAngularJoint.cs:313-356)
@@ -1703,8 +1645,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
         acc0.w = acc0.w + tx;
         acc1.x = acc1.x + ty;
         float ix = w1.x * tx + w2.x * ty, iy = w1.y * tx + w2.y * ty, iz = w1.z * tx + w2.z * ty;
-        if (dynA) ApplyAngular(A, ix, iy, iz);
-        if (dynB) ApplyAngular(B, -ix, -iy, -iz);
+        ApplyAngular(A, ix, iy, iz);
+        ApplyAngular(B, -ix, -iy, -iz);
         account(1, fabsf(tx) + fabsf(ty));
     }
     if (kAdded && (st & (4u << kChildShift)) && IsLinearLimitType(type)) {
@@ -1724,14 +1666,10 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
         const float previous = acc1.z;
         acc1.z = (st & kJMinActive) ? Minf(acc1.z + lambda, 0) : Maxf(acc1.z + lambda, 0);
         lambda = acc1.z - previous;
-        if (dynA) {
-            ApplyLinear(A, ja.x * lambda, ja.y * lambda, ja.z * lambda);
-            ApplyAngular(A, jaa.x * lambda, jaa.y * lambda, jaa.z * lambda);
-        }
-        if (dynB) {
-            ApplyLinear(B, bx * lambda, by * lambda, bz * lambda);
-            ApplyAngular(B, jab.x * lambda, jab.y * lambda, jab.z * lambda);
-        }
+        ApplyLinear(A, ja.x * lambda, ja.y * lambda, ja.z * lambda);
+        ApplyAngular(A, jaa.x * lambda, jaa.y * lambda, jaa.z * lambda);
+        ApplyLinear(B, bx * lambda, by * lambda, bz * lambda);
+        ApplyAngular(B, jab.x * lambda, jab.y * lambda, jab.z * lambda);
         account(2, fabsf(lambda));
     } else if (st & (4u << kChildShift)) {
         const float4 l0 = j.L(kJL0, s), l2 = j.L(kJL2, s);
@@ -1794,8 +1732,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
                 ly = acc0.y - py;
                 lz = acc0.z - pz;
             }
-            if (dynA) ApplyAngular(A, lx, ly, lz);
-            if (dynB) ApplyAngular(B, -lx, -ly, -lz);
+            ApplyAngular(A, lx, ly, lz);
+            ApplyAngular(B, -lx, -ly, -lz);
             account(2, fabsf(lx) + fabsf(ly) + fabsf(lz));
         } else if (kAdded && IsSpeedLimitType(type)) {
             // MaximumLinearSpeedConstraint / MaximumAngularSpeedConstraint.SolveIteration
@@ -1865,14 +1803,10 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
             const float previous = acc1.y;
             acc1.y = Clampf(acc1.y + lambda, -maxForceDt, maxForceDt);
             lambda = acc1.y - previous;
-            if (dynA) {
-                ApplyLinear(A, l0.x * lambda, l0.y * lambda, l0.z * lambda);
-                ApplyAngular(A, jaa.x * lambda, jaa.y * lambda, jaa.z * lambda);
-            }
-            if (dynB) {
-                ApplyLinear(B, bx * lambda, by * lambda, bz * lambda);
-                ApplyAngular(B, jab.x * lambda, jab.y * lambda, jab.z * lambda);
-            }
+            ApplyLinear(A, l0.x * lambda, l0.y * lambda, l0.z * lambda);
+            ApplyAngular(A, jaa.x * lambda, jaa.y * lambda, jaa.z * lambda);
+            ApplyLinear(B, bx * lambda, by * lambda, bz * lambda);
+            ApplyAngular(B, jab.x * lambda, jab.y * lambda, jab.z * lambda);
             account(2, fabsf(lambda));
         } else if (kAdded && (type == BEPUGPU_JOINT_REVOLUTE_MOTOR || type == BEPUGPU_JOINT_TWIST_MOTOR)) {
             // RevoluteMotor.SolveIteration (RevoluteMotor.cs:309-340), TwistMotor's (TwistMotor.cs:226-253)
@@ -1884,8 +1818,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
             const float previous = acc1.y;
             acc1.y = Clampf(acc1.y + lambda, -l2.w, l2.w);
             lambda = acc1.y - previous;
-            if (dynA) ApplyAngular(A, l0.x * lambda, l0.y * lambda, l0.z * lambda);
-            if (dynB) ApplyAngular(B, nx * lambda, ny * lambda, nz * lambda);
+            ApplyAngular(A, l0.x * lambda, l0.y * lambda, l0.z * lambda);
+            ApplyAngular(B, nx * lambda, ny * lambda, nz * lambda);
             account(2, fabsf(lambda));
         } else if (kAdded && type == BEPUGPU_JOINT_ELLIPSE_SWING_LIMIT) {
             // EllipseSwingLimit.SolveIteration (EllipseSwingLimit.cs:327-357)
@@ -1897,8 +1831,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
             const float previous = acc1.y;
             acc1.y = Minf(acc1.y + lambda, 0);
             lambda = acc1.y - previous;
-            if (dynA) ApplyAngular(A, l0.x * lambda, l0.y * lambda, l0.z * lambda);
-            if (dynB) ApplyAngular(B, nx * lambda, ny * lambda, nz * lambda);
+            ApplyAngular(A, l0.x * lambda, l0.y * lambda, l0.z * lambda);
+            ApplyAngular(B, nx * lambda, ny * lambda, nz * lambda);
             account(2, fabsf(lambda));
         } else if (kAdded && type == BEPUGPU_JOINT_TWIST_LIMIT) {
             // TwistLimit.SolveIteration (TwistLimit.cs:200-236)
@@ -1910,8 +1844,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
             const float previous = acc1.y;
             acc1.y = Maxf(acc1.y + lambda, 0);
             lambda = acc1.y - previous;
-            if (dynA) ApplyAngular(A, l0.x * lambda, l0.y * lambda, l0.z * lambda);
-            if (dynB) ApplyAngular(B, nx * lambda, ny * lambda, nz * lambda);
+            ApplyAngular(A, l0.x * lambda, l0.y * lambda, l0.z * lambda);
+            ApplyAngular(B, nx * lambda, ny * lambda, nz * lambda);
             account(2, fabsf(lambda));
         } else if (type == BEPUGPU_JOINT_SWING_LIMIT) {
             // SwingLimit.SolveIteration (SwingLimit.cs:211-243)
@@ -1923,8 +1857,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
             acc1.y = Maxf(acc1.y + lambda, 0);
             lambda = acc1.y - previous;
             float ix = l0.x * lambda, iy = l0.y * lambda, iz = l0.z * lambda;
-            if (dynA) ApplyAngular(A, ix, iy, iz);
-            if (dynB) ApplyAngular(B, -ix, -iy, -iz);
+            ApplyAngular(A, ix, iy, iz);
+            ApplyAngular(B, -ix, -iy, -iz);
             account(2, fabsf(lambda));
         } else {
             // RevoluteLimit.SolveIteration (RevoluteLimit.cs:211-283)
@@ -1939,8 +1873,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
                 float previous = acc1.y;
                 acc1.y = Maxf(acc1.y + lambda, 0);
                 lambda = acc1.y - previous;
-                if (dynA) ApplyAngular(A, l0.x * lambda, l0.y * lambda, l0.z * lambda);
-                if (dynB) ApplyAngular(B, nx * lambda, ny * lambda, nz * lambda);
+                ApplyAngular(A, l0.x * lambda, l0.y * lambda, l0.z * lambda);
+                ApplyAngular(B, nx * lambda, ny * lambda, nz * lambda);
                 lambdaTotal += fabsf(lambda);
             }
             if (st & kJMaxActive) {
@@ -1952,8 +1886,8 @@ __device__ __forceinline__ void SolveJointChildren(const JointSoA& j, int s, Bod
                 float previous = acc1.z;
                 acc1.z = Maxf(acc1.z + lambda, 0);
                 lambda = acc1.z - previous;
-                if (dynA) ApplyAngular(A, l1.x * lambda, l1.y * lambda, l1.z * lambda);
-                if (dynB) ApplyAngular(B, nx * lambda, ny * lambda, nz * lambda);
+                ApplyAngular(A, l1.x * lambda, l1.y * lambda, l1.z * lambda);
+                ApplyAngular(B, nx * lambda, ny * lambda, nz * lambda);
                 lambdaTotal += fabsf(lambda);
             }
             account(2, lambdaTotal);

@@ -254,11 +254,9 @@ __global__ void __launch_bounds__(kThreads) k_step_noalloc(bepugpu_body* bodies,
                 if (!(st.x & kGroupActive)) continue;
                 int4 h = v.m.head[s];
                 BodyState A, B;
-                if (h.x >= 0) LoadBody(v.b, h.x, A);
-                if (h.y >= 0) LoadBody(v.b, h.y, B);
-                WarmStartManifold(v.m, s, A, B, st.x, h.z & 0xff);
-                if (st.x & kDynA) StoreVelocity(v.b, h.x, A);
-                if (st.x & kDynB) StoreVelocity(v.b, h.y, B);
+                LoadVisit(GlobalBodies{v.b}, h.x, h.y, st.x, A, B);
+                WarmStartManifold(v.m, s, A, B, st);
+                StoreVisit(GlobalBodies{v.b}, h.x, h.y, st.x, A, B);
             }
             __syncthreads();
         }
@@ -269,11 +267,9 @@ __global__ void __launch_bounds__(kThreads) k_step_noalloc(bepugpu_body* bodies,
                     if (!(st.x & kGroupActive)) continue;
                     int4 h = v.m.head[s];
                     BodyState A, B;
-                    if (h.x >= 0) LoadBody(v.b, h.x, A);
-                    if (h.y >= 0) LoadBody(v.b, h.y, B);
-                    SolveManifold(v.m, s, A, B, st, h.z & 0xff, p);
-                    if (st.x & kDynA) StoreVelocity(v.b, h.x, A);
-                    if (st.x & kDynB) StoreVelocity(v.b, h.y, B);
+                    LoadVisit(GlobalBodies{v.b}, h.x, h.y, st.x, A, B);
+                    SolveManifold(v.m, s, A, B, st, p);
+                    StoreVisit(GlobalBodies{v.b}, h.x, h.y, st.x, A, B);
                     v.m.state[s] = st;
                 }
                 __syncthreads();

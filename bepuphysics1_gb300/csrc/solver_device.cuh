@@ -75,21 +75,24 @@ enum : uint32_t {
     kCandidate = 8u
 };
 
-// Manifold state bits (word x of the uint2 state).
+// Manifold state: word x of the uint2.
 enum : uint32_t {
     kGroupActive = 1u << 0,       // ConvexContactManifoldConstraint.isActiveInSolver
-    kChildShift = 1,              // bits 1..6: pen0..pen3, sliding, twist isActiveInSolver
-    kSlidingBit = 1u << 5,
-    kTwistBit = 1u << 6,
+    kContactFriction = 1u << 1,   // NONCONVEX: children 4..7 are the contacts' friction constraints
     kDynA = 1u << 7,              // entityADynamic as computed in Update
     kDynB = 1u << 8,
-    kHasA = 1u << 9,              // entity A is not null
-    kHasB = 1u << 10,
-    kFricShift = 11,              // NONCONVEX: bits 11..14, contact friction 0..3 isActiveInSolver
     kIterShift = 16               // bits 16..31: group currentIterations
 };
-// Word y: 4-bit iterationsAtZeroImpulse per child: pen0..3, then sliding and
-// twist (convex) or contact friction 0..3 (NONCONVEX).
+// Word y: a nibble per child -- penetration 0..3, then sliding and twist
+// (convex) or contact friction 0..3 (NONCONVEX) -- with its
+// iterationsAtZeroImpulse, or 15 when it is not active in the solver.  A child
+// stops when the count passes minimumIterationCount (at most 14), so an active
+// one holds 0..14.
+constexpr uint32_t kChildOff = 0xfu;
+constexpr int kSlidingChild = 4, kTwistChild = 5;
+__device__ __forceinline__ bool ChildOn(uint32_t children, int c) {
+    return (children & (kChildOff << (4 * c))) != (kChildOff << (4 * c));
+}
 constexpr uint32_t kManifoldNonConvex = 8u;  // BEPUGPU_MANIFOLD_NONCONVEX, in head.z >> 8
 
 struct ManifoldSoA {
@@ -157,21 +160,19 @@ struct GlobalBodies {
     }
 };
 
-template <class V>
-__device__ __forceinline__ void LoadBodyV(const V& bv, int r, BodyState& s) {
-    float4 v = bv.Vlin(r), w = bv.Vang(r), a = bv.Inv0(r), c = bv.Inv1(r);
+__device__ __forceinline__ void MakeBody(float4 v, float4 w, float4 a, float4 c, BodyState& s) {
     s.vx = v.x; s.vy = v.y; s.vz = v.z; s.invMass = v.w;
     s.wx = w.x; s.wy = w.y; s.wz = w.z; s.I33 = w.w;
     s.I11 = a.x; s.I12 = a.y; s.I13 = a.z; s.I21 = a.w;
     s.I22 = c.x; s.I23 = c.y; s.I31 = c.z; s.I32 = c.w;
 }
 template <class V>
+__device__ __forceinline__ void LoadBodyV(const V& bv, int r, BodyState& s) {
+    MakeBody(bv.Vlin(r), bv.Vang(r), bv.Inv0(r), bv.Inv1(r), s);
+}
+template <class V>
 __device__ __forceinline__ void StoreVelocityV(const V& bv, int r, const BodyState& s) {
     bv.SetVelocity(r, make_float4(s.vx, s.vy, s.vz, s.invMass), make_float4(s.wx, s.wy, s.wz, s.I33));
-}
-__device__ __forceinline__ void LoadBody(const BodySoA& b, int i, BodyState& s) { LoadBodyV(GlobalBodies{b}, i, s); }
-__device__ __forceinline__ void StoreVelocity(const BodySoA& b, int i, const BodyState& s) {
-    StoreVelocityV(GlobalBodies{b}, i, s);
 }
 // EntityBase.ApplyLinearImpulse (EntityBase.cs:754-761)
 __device__ __forceinline__ void ApplyLinear(BodyState& s, float x, float y, float z) {
@@ -552,18 +553,24 @@ __device__ __forceinline__ void PrestepManifoldIO(const ManifoldSoA& mi, int si,
         }
     };
     if (!groupActive) {
-        mo.state[so] = make_uint2(0u, 0u);
+        mo.state[so] = make_uint2(0u, ~0u);
         carryState();
         return;
     }
     st |= kGroupActive;
-    for (int k = 0; k < count; k++) st |= 1u << (kChildShift + k);
-    if (count > 0) st |= kSlidingBit | kTwistBit;
+    uint32_t children = ~0u << (4 * count);  // count penetration children, sliding and twist
+    if (count > 0) children &= ~((kChildOff << (4 * kSlidingChild)) | (kChildOff << (4 * kTwistChild)));
+    if (count < 4) {  // the friction limits sum all four lanes
+        float4 acc = mi.penacc[si];
+        if (count < 1) acc.x = 0.f;
+        if (count < 2) acc.y = 0.f;
+        if (count < 3) acc.z = 0.f;
+        acc.w = 0.f;
+        mo.penacc[so] = acc;
+    }
     bool dynA = hasA && A.dynamic, dynB = hasB && B.dynamic;
     if (dynA) st |= kDynA;
     if (dynB) st |= kDynB;
-    if (hasA) st |= kHasA;
-    if (hasB) st |= kHasB;
     float4 mat = mi.mat[si];
     const float kinetic = mat.x, staticF = mat.y, bounciness = mat.z;
     float updateRate = p.updateRate;
@@ -627,7 +634,7 @@ __device__ __forceinline__ void PrestepManifoldIO(const ManifoldSoA& mi, int si,
         mo.pj2[k * capo + so] = make_float4(aBx, aBy, aBz, v2i);
     }
     if (count == 0) {
-        mo.state[so] = make_uint2(st, 0u);
+        mo.state[so] = make_uint2(st, ~0u);
         carryState();
         return;
     }
@@ -636,7 +643,8 @@ __device__ __forceinline__ void PrestepManifoldIO(const ManifoldSoA& mi, int si,
         // after the penetration children, each contact's ContactFrictionConstraint.Update
         // (ContactFrictionConstraint.cs:147-256).  The friction direction and impulse come
         // from mi; they go to mo with the prestep products.
-        st &= ~(kSlidingBit | kTwistBit);
+        st |= kContactFriction;
+        children |= 0xffff0000u;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             if (k >= count) break;
@@ -677,7 +685,7 @@ __device__ __forceinline__ void PrestepManifoldIO(const ManifoldSoA& mi, int si,
                 mo.cfr[k * capo + so] = fr;
                 continue;  // no direction: isActiveInSolver = false for this step
             }
-            st |= 1u << (kFricShift + k);
+            children &= ~(kChildOff << (16 + 4 * k));
             const float lx = fr.x, ly = fr.y, lz = fr.z;
             const float aAx = (ray * lz) - (raz * ly), aAy = (raz * lx) - (rax * lz), aAz = (rax * ly) - (ray * lx);
             const float aBx = (ly * rbz) - (lz * rby), aBy = (lz * rbx) - (lx * rbz), aBz = (lx * rby) - (ly * rbx);
@@ -698,7 +706,7 @@ __device__ __forceinline__ void PrestepManifoldIO(const ManifoldSoA& mi, int si,
             mo.cfa[k * capo + so] = make_float4(aAx, aAy, aAz, -1 / (entryA + entryB));
             mo.cfb[k * capo + so] = make_float4(aBx, aBy, aBz, friction);
         }
-        mo.state[so] = make_uint2(st, 0u);
+        mo.state[so] = make_uint2(st, children);
         return;
     }
 
@@ -873,7 +881,7 @@ __device__ __forceinline__ void PrestepManifoldIO(const ManifoldSoA& mi, int si,
     mo.s6[so] = make_float4(aB11, aB12, aB13, tfriction);
     mo.s7[so] = make_float4(aB21, aB22, aB23, 0.f);
     mo.lever[so] = make_float4(lev[0], lev[1], lev[2], lev[3]);
-    mo.state[so] = make_uint2(st, 0u);
+    mo.state[so] = make_uint2(st, children);
 }
 template <class V>
 __device__ __forceinline__ void PrestepManifoldV(const ManifoldSoA& m, const V& bv, int s, int ra, int rb,
@@ -885,82 +893,97 @@ __device__ __forceinline__ void PrestepManifold(const ManifoldSoA& m, const Body
     PrestepManifoldV(m, GlobalBodies{b}, s, h.x, h.y, p);
 }
 
+// A body of a visit.  One that is not dynamic enters with inverse mass and
+// inertia zero, so an impulse leaves its velocity as it is and the children
+// apply theirs to both bodies without asking (it is not stored); no entity
+// enters as zeros.
+template <class V>
+__device__ __forceinline__ void LoadVisitBody(const V& bv, int r, bool dynamic, BodyState& s) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v = zero, w = zero, a = zero, c = zero;
+    if (r != -1) {
+        v = bv.Vlin(r);
+        w = bv.Vang(r);
+    }
+    if (dynamic) {
+        a = bv.Inv0(r);
+        c = bv.Inv1(r);
+    } else {
+        v.w = w.w = 0.f;
+    }
+    MakeBody(v, w, a, c, s);
+}
+template <class V>
+__device__ __forceinline__ void LoadVisit(const V& bv, int ra, int rb, uint32_t st, BodyState& A, BodyState& B) {
+    LoadVisitBody(bv, ra, st & kDynA, A);
+    LoadVisitBody(bv, rb, st & kDynB, B);
+}
+template <class V>
+__device__ __forceinline__ void StoreVisit(const V& bv, int ra, int rb, uint32_t st, const BodyState& A,
+                                           const BodyState& B) {
+    if (st & kDynA) StoreVelocityV(bv, ra, A);
+    if (st & kDynB) StoreVelocityV(bv, rb, B);
+}
+// A's impulse along a child's jacobians, and B's (its linear jacobian is A's negated).
+__device__ __forceinline__ void ApplyImpulse(BodyState& A, BodyState& B, float impulse, float4 linear, float4 angularA,
+                                             float4 angularB) {
+    const float lx = impulse * linear.x, ly = impulse * linear.y, lz = impulse * linear.z;
+    ApplyLinear(A, lx, ly, lz);
+    ApplyAngular(A, impulse * angularA.x, impulse * angularA.y, impulse * angularA.z);
+    ApplyLinear(B, -lx, -ly, -lz);
+    ApplyAngular(B, impulse * angularB.x, impulse * angularB.y, impulse * angularB.z);
+}
+// The relative velocity along a child's jacobians: A's part plus B's (the
+// reference skips a missing entity's part, which is zero here).
+__device__ __forceinline__ float VelocityAlong(const BodyState& A, const BodyState& B, float4 linear, float4 angularA,
+                                               float4 angularB) {
+    const float a = A.vx * linear.x + A.vy * linear.y + A.vz * linear.z + A.wx * angularA.x + A.wy * angularA.y +
+                    A.wz * angularA.z;
+    const float b = -B.vx * linear.x - B.vy * linear.y - B.vz * linear.z + B.wx * angularB.x + B.wy * angularB.y +
+                    B.wz * angularB.z;
+    return a + b;
+}
+
 // Warm start: ConvexContactManifoldConstraint.ExclusiveUpdate
 // (ConvexContactManifoldConstraint.cs:186-192) with the children's
 // ExclusiveUpdate bodies (ContactPenetrationConstraint.cs:240-271,
 // SlidingFrictionTwoAxis.cs:447-482, TwistFrictionConstraint.cs:182-204).
-template <class Body>
-__device__ __forceinline__ void WarmStartManifold(const ManifoldSoA& m, int s, Body& A, Body& B, uint32_t st,
-                                                  int count) {
+__device__ __forceinline__ void WarmStartManifold(const ManifoldSoA& m, int s, BodyState& A, BodyState& B,
+                                                  uint2 state) {
     const int cap = m.capacity;
-    bool dynA = st & kDynA, dynB = st & kDynB;
+    const uint32_t children = state.y;
     float4 acc4 = m.penacc[s];
     const float accs[4] = {acc4.x, acc4.y, acc4.z, acc4.w};
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        if (k >= count) break;
-        if (!(st & (1u << (kChildShift + k)))) continue;
-        float4 j0 = m.pj0[k * cap + s], j1 = m.pj1[k * cap + s], j2 = m.pj2[k * cap + s];
-        float acc = accs[k];
-        float lx = acc * j0.x, ly = acc * j0.y, lz = acc * j0.z;
-        if (dynA) {
-            ApplyLinear(A, lx, ly, lz);
-            ApplyAngular(A, acc * j1.x, acc * j1.y, acc * j1.z);
-        }
-        if (dynB) {
-            ApplyLinear(B, -lx, -ly, -lz);
-            ApplyAngular(B, acc * j2.x, acc * j2.y, acc * j2.z);
-        }
+        if (!ChildOn(children, k)) continue;
+        ApplyImpulse(A, B, accs[k], m.pj0[k * cap + s], m.pj1[k * cap + s], m.pj2[k * cap + s]);
     }
-    if (st & (0xfu << kFricShift)) {
+    if (state.x & kContactFriction) {
         // ContactFrictionConstraint.ExclusiveUpdate (ContactFrictionConstraint.cs:258-289)
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            if (k >= count) break;
-            if (!(st & (1u << (kFricShift + k)))) continue;
+            if (!ChildOn(children, 4 + k)) continue;
             const float4 fr = m.cfr[k * cap + s];
-            const float acc = fr.w;
-            const float lx = acc * fr.x, ly = acc * fr.y, lz = acc * fr.z;
-            if (dynA) {
-                const float4 fa = m.cfa[k * cap + s];
-                ApplyLinear(A, lx, ly, lz);
-                ApplyAngular(A, acc * fa.x, acc * fa.y, acc * fa.z);
-            }
-            if (dynB) {
-                const float4 fb = m.cfb[k * cap + s];
-                ApplyLinear(B, -lx, -ly, -lz);
-                ApplyAngular(B, acc * fb.x, acc * fb.y, acc * fb.z);
-            }
+            ApplyImpulse(A, B, fr.w, fr, m.cfa[k * cap + s], m.cfb[k * cap + s]);
         }
         return;
     }
-    if (count == 0) return;
+    if (!ChildOn(children, kSlidingChild)) return;  // no contacts
     float4 f = m.fricacc[s];
-    if (st & kSlidingBit) {
-        float ax = f.x, ay = f.y;
-        float4 L1 = m.saxis[s], L2 = m.s3[s], A1 = m.s4[s], A2 = m.s5[s], B1 = m.s6[s], B2 = m.s7[s];
-        float lx = ax * L1.x + ay * L2.x;
-        float ly = ax * L1.y + ay * L2.y;
-        float lz = ax * L1.z + ay * L2.z;
-        if (dynA) {
-            float gx = ax * A1.x + ay * A2.x, gy = ax * A1.y + ay * A2.y, gz = ax * A1.z + ay * A2.z;
-            ApplyLinear(A, lx, ly, lz);
-            ApplyAngular(A, gx, gy, gz);
-        }
-        if (dynB) {
-            float gx = ax * B1.x + ay * B2.x, gy = ax * B1.y + ay * B2.y, gz = ax * B1.z + ay * B2.z;
-            ApplyLinear(B, -lx, -ly, -lz);
-            ApplyAngular(B, gx, gy, gz);
-        }
-    }
-    if (st & kTwistBit) {
-        float4 j0 = m.pj0[s];  // twist axis = contact 0 normal = -linearA of penetration 0
-        float nx = -j0.x, ny = -j0.y, nz = -j0.z;
-        float t = f.z;
-        float gx = t * nx, gy = t * ny, gz = t * nz;
-        if (dynA) ApplyAngular(A, gx, gy, gz);
-        if (dynB) ApplyAngular(B, -gx, -gy, -gz);
-    }
+    float ax = f.x, ay = f.y;
+    float4 L1 = m.saxis[s], L2 = m.s3[s], A1 = m.s4[s], A2 = m.s5[s], B1 = m.s6[s], B2 = m.s7[s];
+    float lx = ax * L1.x + ay * L2.x;
+    float ly = ax * L1.y + ay * L2.y;
+    float lz = ax * L1.z + ay * L2.z;
+    ApplyLinear(A, lx, ly, lz);
+    ApplyAngular(A, ax * A1.x + ay * A2.x, ax * A1.y + ay * A2.y, ax * A1.z + ay * A2.z);
+    ApplyLinear(B, -lx, -ly, -lz);
+    ApplyAngular(B, ax * B1.x + ay * B2.x, ax * B1.y + ay * B2.y, ax * B1.z + ay * B2.z);
+    float4 j0 = m.pj0[s];  // twist axis = contact 0 normal = -linearA of penetration 0
+    const float gx = f.z * -j0.x, gy = f.z * -j0.y, gz = f.z * -j0.z;
+    ApplyAngular(A, gx, gy, gz);
+    ApplyAngular(B, -gx, -gy, -gz);
 }
 
 // Programmatic dependent launch: a sweep kernel lets the next one start its
@@ -970,204 +993,173 @@ __device__ __forceinline__ void WarmStartManifold(const ManifoldSoA& m, int s, B
 __device__ __forceinline__ void LetDependentsLaunch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void WaitForPrerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// The prestep products a solve visit reads; none of them change during the
-// sweeps, so a sweep kernel may load them before the sweep it follows ends.
+// The prestep products the active children of a visit read (children: the
+// state's word y; it may name more than are active).  None of them change
+// during the sweeps, so a sweep may load them before the one it follows ends.
 struct SolveLanes {
     float4 J0[4], J1[4], J2[4];
     float4 S0, S1, L1, L2, A1, A2, B1, B2, LEV;
 };
-__device__ __forceinline__ void LoadSolveLanes(const ManifoldSoA& m, int s, int count, bool friction,
+__device__ __forceinline__ void LoadSolveLanes(const ManifoldSoA& m, int s, uint32_t st, uint32_t children,
                                                SolveLanes& L) {
     const int cap = m.capacity;
+    const bool friction = !(st & kContactFriction);
+    const bool sliding = friction && ChildOn(children, kSlidingChild), twist = friction && ChildOn(children, kTwistChild);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        if (k < count) {
-            L.J0[k] = m.pj0[k * cap + s];
+        const bool on = ChildOn(children, k);
+        if (on || (k == 0 && twist)) L.J0[k] = m.pj0[k * cap + s];
+        if (on) {
             L.J1[k] = m.pj1[k * cap + s];
             L.J2[k] = m.pj2[k * cap + s];
         }
     }
-    if (friction) {
+    if (sliding) {
         L.S0 = m.s0[s]; L.S1 = m.s1[s]; L.L1 = m.saxis[s]; L.L2 = m.s3[s];
-        L.A1 = m.s4[s]; L.A2 = m.s5[s]; L.B1 = m.s6[s]; L.B2 = m.s7[s];
-        L.LEV = m.lever[s];
+        L.A1 = m.s4[s]; L.B2 = m.s7[s];
     }
+    if (sliding || twist) {
+        L.A2 = m.s5[s];
+        L.B1 = m.s6[s];
+    }
+    if (twist) L.LEV = m.lever[s];
 }
 
 // One solver visit of a manifold: Solver.UnsafeSolveIteration (Solver.cs:285-314)
 // -> ConvexContactManifoldConstraint.SolveIteration (:199-212) ->
 // SolverGroup.SolveUpdateable (SolverGroup.cs:117-150) on each child.
 // Children solve strictly in order: they are a Gauss-Seidel sequence.
-// pre: the visit's lanes already loaded (LoadSolveLanes with friction = count > 0), or null.
-template <class Body>
-__device__ __forceinline__ void SolveManifold(const ManifoldSoA& m, int s, Body& A, Body& B, uint2& state,
-                                              int count, const StepParams& p, const SolveLanes* pre = nullptr) {
+// pre: the visit's lanes already loaded (LoadSolveLanes), or null.
+// A visit is bound by the children's dependent chains and instruction issue
+// (a warp or two per scheduler), so it holds no branch but a child's own: both
+// bodies take every impulse (LoadVisitBody), and the children's bookkeeping is
+// one word operation at the end instead of a branch and a nibble update each.
+// One warp alone, all six children active, lanes in shared memory: 3,109 ->
+// 2,118 cycles a visit (915 -> 806 instructions, 87 -> 33 of them branches);
+// the 65,536-box pile's group launch 84.8 -> 73.4 us.  Packed two-wide FP32
+// (add / fma.rn.f32x2) measured the same as these scalar chains: the pipe runs
+// both at the same rate, and the pairs cost as many moves as they save.
+__device__ __forceinline__ void SolveManifold(const ManifoldSoA& m, int s, BodyState& A, BodyState& B, uint2& state,
+                                              const StepParams& p, const SolveLanes* pre = nullptr) {
     const int cap = m.capacity;
-    uint32_t st = state.x, zeros = state.y;
+    uint32_t st = state.x, children = state.y;
     // UnsafeSolveIteration on the group
     uint32_t iter = (st >> kIterShift) + 1;
     st = (st & 0xffffu) | (iter << kIterShift);
     if (!((int)iter <= p.iterationLimit && (int)iter <= p.maximumIterationCount)) {
-        state = make_uint2(st & ~kGroupActive, zeros);
+        state = make_uint2(st & ~kGroupActive, children);
         return;
     }
-    bool hasA = st & kHasA, hasB = st & kHasB;  // kinematic partners' velocities still enter
-    bool dynA = st & kDynA, dynB = st & kDynB;
-    int activeConstraints = 0;
     // Every load of the visit is issued before the sequential solves start.
     float4 acc4 = m.penacc[s];
     float accs[4] = {acc4.x, acc4.y, acc4.z, acc4.w};
     SolveLanes Lv;
     if (pre) Lv = *pre;
-    else LoadSolveLanes(m, s, count, (st & (kSlidingBit | kTwistBit)) != 0, Lv);
-    const float4 *J0 = Lv.J0, *J1 = Lv.J1, *J2 = Lv.J2;
+    else LoadSolveLanes(m, s, st, children, Lv);
     float4 f = m.fricacc[s];
-    const float4 S0 = Lv.S0, S1 = Lv.S1, L1 = Lv.L1, L2 = Lv.L2, A1 = Lv.A1, A2 = Lv.A2, B1 = Lv.B1, B2 = Lv.B2,
-                 LEV = Lv.LEV;
-    // SolveUpdateable bookkeeping for child c (its zero-impulse nibble) given
-    // its |impulse|; `bit` is its activity bit.
-    auto accountBit = [&](int c, uint32_t bit, float r) {
-        uint32_t z = (zeros >> (4 * c)) & 0xfu;
-        if (r < p.minimumImpulse) {
-            z++;
-            if ((int)z > p.minimumIterationCount) st &= ~bit;
-            else activeConstraints++;
-        } else {
-            z = 0;
-            activeConstraints++;
-        }
-        zeros = (zeros & ~(0xfu << (4 * c))) | ((z & 0xfu) << (4 * c));
-    };
-    auto account = [&](int c, float r) { accountBit(c, 1u << (kChildShift + c), r); };
+    const uint32_t on = children;  // the children this visit solves
+    // SolveUpdateable's bookkeeping (SolverGroup.cs:117-150): a child whose
+    // |impulse| is below the minimum is marked by a one in its nibble here;
+    // all children's counts follow at the end.
+    uint32_t still = 0;
+    auto account = [&](int c, float r) { still |= r < p.minimumImpulse ? 1u << (4 * c) : 0u; };
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        if (k >= count) break;
-        if (!(st & (1u << (kChildShift + k)))) continue;
+        if (!ChildOn(on, k)) continue;
         // child currentIterations equals the group's here; the cap passed above
-        const float4 j0 = J0[k], j1 = J1[k], j2 = J2[k];
-        float lx = j0.x, ly = j0.y, lz = j0.z, bias = j0.w, softness = j1.w, v2i = j2.w;
-        float rv = 0;
-        if (hasA) rv = A.vx * lx + A.vy * ly + A.vz * lz + A.wx * j1.x + A.wy * j1.y + A.wz * j1.z;
-        if (hasB) rv += -B.vx * lx - B.vy * ly - B.vz * lz + B.wx * j2.x + B.wy * j2.y + B.wz * j2.z;
-        float lambda = (rv - bias + softness * accs[k]) * v2i;
-        float prev = accs[k];
+        const float4 j0 = Lv.J0[k], j1 = Lv.J1[k], j2 = Lv.J2[k];
+        const float bias = j0.w, softness = j1.w, v2i = j2.w;
+        float lambda = (VelocityAlong(A, B, j0, j1, j2) - bias + softness * accs[k]) * v2i;
+        const float prev = accs[k];
         accs[k] = Maxf(0, accs[k] + lambda);
         lambda = accs[k] - prev;
-        float ix = lambda * lx, iy = lambda * ly, iz = lambda * lz;
-        if (dynA) {
-            ApplyLinear(A, ix, iy, iz);
-            ApplyAngular(A, lambda * j1.x, lambda * j1.y, lambda * j1.z);
-        }
-        if (dynB) {
-            ApplyLinear(B, -ix, -iy, -iz);
-            ApplyAngular(B, lambda * j2.x, lambda * j2.y, lambda * j2.z);
-        }
+        ApplyImpulse(A, B, lambda, j0, j1, j2);
         account(k, fabsf(lambda));
     }
-    if (st & (0xfu << kFricShift)) {
+    if (st & kContactFriction) {
         // NONCONVEX: each contact's ContactFrictionConstraint.SolveIteration
         // (ContactFrictionConstraint.cs:95-143), after every penetration child.
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            if (k >= count) break;
-            const uint32_t bit = 1u << (kFricShift + k);
-            if (!(st & bit)) continue;
+            if (!ChildOn(on, 4 + k)) continue;
             float4 fr = m.cfr[k * cap + s];
             const float4 fa = m.cfa[k * cap + s], fb = m.cfb[k * cap + s];
-            float velocity = 0;
-            if (hasA)
-                velocity += A.vx * fr.x + A.vy * fr.y + A.vz * fr.z + A.wx * fa.x + A.wy * fa.y + A.wz * fa.z;
-            if (hasB)
-                velocity += -B.vx * fr.x - B.vy * fr.y - B.vz * fr.z + B.wx * fb.x + B.wy * fb.y + B.wz * fb.z;
-            float lambda = velocity * fa.w;
+            float lambda = VelocityAlong(A, B, fr, fa, fb) * fa.w;
             const float prev = fr.w, maxForce = fb.w * accs[k];
             fr.w = Clampf(fr.w + lambda, -maxForce, maxForce);
             lambda = fr.w - prev;
-            const float ix = lambda * fr.x, iy = lambda * fr.y, iz = lambda * fr.z;
-            if (dynA) {
-                ApplyLinear(A, ix, iy, iz);
-                ApplyAngular(A, lambda * fa.x, lambda * fa.y, lambda * fa.z);
-            }
-            if (dynB) {
-                ApplyLinear(B, -ix, -iy, -iz);
-                ApplyAngular(B, lambda * fb.x, lambda * fb.y, lambda * fb.z);
-            }
-            accountBit(4 + k, bit, fabsf(lambda));
+            ApplyImpulse(A, B, lambda, fr, fa, fb);
+            account(4 + k, fabsf(lambda));
             m.cfr[k * cap + s] = fr;
         }
-    }
-    if (st & kSlidingBit) {
-        // SlidingFrictionTwoAxis.SolveIteration (SlidingFrictionTwoAxis.cs:155-234)
-        float dvx = 0, dvy = 0, dvz = 0;
-        if (hasA) {
-            dvx = A.vx + (A.wy * S0.z) - (A.wz * S0.y);
-            dvy = A.vy + (A.wz * S0.x) - (A.wx * S0.z);
-            dvz = A.vz + (A.wx * S0.y) - (A.wy * S0.x);
-        }
-        if (hasB) {
+    } else {
+        // The friction limits sum all four lanes' impulses: the prestep clears
+        // those past the contact count.
+        if (ChildOn(on, kSlidingChild)) {
+            // SlidingFrictionTwoAxis.SolveIteration (SlidingFrictionTwoAxis.cs:155-234)
+            const float4 S0 = Lv.S0, S1 = Lv.S1, L1 = Lv.L1, L2 = Lv.L2, A1 = Lv.A1, A2 = Lv.A2, B1 = Lv.B1, B2 = Lv.B2;
+            float dvx = A.vx + (A.wy * S0.z) - (A.wz * S0.y);
+            float dvy = A.vy + (A.wz * S0.x) - (A.wx * S0.z);
+            float dvz = A.vz + (A.wx * S0.y) - (A.wy * S0.x);
             dvx += -B.vx - (B.wy * S1.z) + (B.wz * S1.y);
             dvy += -B.vy - (B.wz * S1.x) + (B.wx * S1.z);
             dvz += -B.vz - (B.wx * S1.y) + (B.wy * S1.x);
-        }
-        float lxv = dvx * L1.x + dvy * L1.y + dvz * L1.z;
-        float lyv = dvx * L2.x + dvy * L2.y + dvz * L2.z;
-        float x = lxv;
-        lxv = x * S1.w + lyv * L2.w;   // M11, M21
-        lyv = x * L1.w + lyv * A1.w;   // M12, M22
-        float px = f.x, py = f.y;
-        f.x += lxv;
-        f.y += lyv;
-        float length = f.x * f.x + f.y * f.y;
-        float maximumFrictionForce = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (k < count) maximumFrictionForce += accs[k];
-        maximumFrictionForce *= S0.w;
-        if (length > maximumFrictionForce * maximumFrictionForce) {
-            length = maximumFrictionForce / SqrtOfFloat(length);
-            f.x *= length;
-            f.y *= length;
-        }
-        lxv = f.x - px;
-        lyv = f.y - py;
-        float gx = lxv * L1.x + lyv * L2.x, gy = lxv * L1.y + lyv * L2.y, gz = lxv * L1.z + lyv * L2.z;
-        if (dynA) {
+            float lxv = dvx * L1.x + dvy * L1.y + dvz * L1.z;
+            float lyv = dvx * L2.x + dvy * L2.y + dvz * L2.z;
+            float x = lxv;
+            lxv = x * S1.w + lyv * L2.w;   // M11, M21
+            lyv = x * L1.w + lyv * A1.w;   // M12, M22
+            float px = f.x, py = f.y;
+            f.x += lxv;
+            f.y += lyv;
+            float length = f.x * f.x + f.y * f.y;
+            float maximumFrictionForce = accs[0] + accs[1] + accs[2] + accs[3];
+            maximumFrictionForce *= S0.w;
+            if (length > maximumFrictionForce * maximumFrictionForce) {
+                length = maximumFrictionForce / SqrtOfFloat(length);
+                f.x *= length;
+                f.y *= length;
+            }
+            lxv = f.x - px;
+            lyv = f.y - py;
+            float gx = lxv * L1.x + lyv * L2.x, gy = lxv * L1.y + lyv * L2.y, gz = lxv * L1.z + lyv * L2.z;
             ApplyLinear(A, gx, gy, gz);
             ApplyAngular(A, lxv * A1.x + lyv * A2.x, lxv * A1.y + lyv * A2.y, lxv * A1.z + lyv * A2.z);
-        }
-        if (dynB) {
             ApplyLinear(B, -gx, -gy, -gz);
             ApplyAngular(B, lxv * B1.x + lyv * B2.x, lxv * B1.y + lyv * B2.y, lxv * B1.z + lyv * B2.z);
+            account(kSlidingChild, fabsf(lxv) + fabsf(lyv));
         }
-        account(4, fabsf(lxv) + fabsf(lyv));
+        if (ChildOn(on, kTwistChild)) {
+            // TwistFrictionConstraint.SolveIteration (TwistFrictionConstraint.cs:65-107)
+            const float4 j0 = Lv.J0[0], lev = Lv.LEV;
+            const float v2i = Lv.A2.w, friction = Lv.B1.w;
+            const float nx = -j0.x, ny = -j0.y, nz = -j0.z;
+            float lambda = A.wx * nx + A.wy * ny + A.wz * nz;
+            lambda -= B.wx * nx + B.wy * ny + B.wz * nz;
+            lambda *= v2i;
+            float prev = f.z;
+            float maximumFrictionForce = lev.x * accs[0] + lev.y * accs[1] + lev.z * accs[2] + lev.w * accs[3];
+            maximumFrictionForce *= friction;
+            f.z = Clampf(f.z + lambda, -maximumFrictionForce, maximumFrictionForce);
+            lambda = f.z - prev;
+            float gx = lambda * nx, gy = lambda * ny, gz = lambda * nz;
+            ApplyAngular(A, gx, gy, gz);
+            ApplyAngular(B, -gx, -gy, -gz);
+            account(kTwistChild, fabsf(lambda));
+        }
     }
-    if (st & kTwistBit) {
-        // TwistFrictionConstraint.SolveIteration (TwistFrictionConstraint.cs:65-107)
-        const float4 j0 = J0[0], lev = LEV;
-        float v2i = A2.w, friction = B1.w;
-        float nx = -j0.x, ny = -j0.y, nz = -j0.z;
-        float lambda = 0;
-        if (hasA) lambda = A.wx * nx + A.wy * ny + A.wz * nz;
-        if (hasB) lambda -= B.wx * nx + B.wy * ny + B.wz * nz;
-        lambda *= v2i;
-        float prev = f.z;
-        const float levs[4] = {lev.x, lev.y, lev.z, lev.w};
-        float maximumFrictionForce = 0;
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (k < count) maximumFrictionForce += levs[k] * accs[k];
-        maximumFrictionForce *= friction;
-        f.z = Clampf(f.z + lambda, -maximumFrictionForce, maximumFrictionForce);
-        lambda = f.z - prev;
-        float gx = lambda * nx, gy = lambda * ny, gz = lambda * nz;
-        if (dynA) ApplyAngular(A, gx, gy, gz);
-        if (dynB) ApplyAngular(B, -gx, -gy, -gz);
-        account(5, fabsf(lambda));
-    }
-    if (activeConstraints <= 0) st &= ~kGroupActive;
+    // A still child's count goes up, a moving one's starts again, a stopped
+    // one keeps its 15; a count that passes minimumIterationCount -- one more
+    // than it, since the child was active -- becomes 15.
+    const uint32_t off = children & (children >> 1) & (children >> 2) & (children >> 3) & 0x11111111u;
+    children = (children & (off * 15u)) | ((children & (still * 15u)) + still);
+    const uint32_t x = children ^ (still * ((uint32_t)p.minimumIterationCount + 1u));
+    const uint32_t stop = still & ~(x | (x >> 1) | (x >> 2) | (x >> 3));
+    children |= stop * 15u;
+    if (children == ~0u) st &= ~kGroupActive;
     m.penacc[s] = make_float4(accs[0], accs[1], accs[2], accs[3]);
     m.fricacc[s] = f;
-    state = make_uint2(st, zeros);
+    state = make_uint2(st, children);
 }
 
 }  // namespace bepugpu
