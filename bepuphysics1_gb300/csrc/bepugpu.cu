@@ -468,7 +468,9 @@ __device__ __forceinline__ void WarmSlot(const ManifoldSoA& m, const BodySoA& b,
     int4 h = m.head[s];
     BodyState A, B;
     LoadVisit(GlobalBodies{b}, h.x, h.y, state.x, A, B);
-    WarmStartManifold(m, s, A, B, state);
+    SolveLanes L;
+    LoadSolveLanes(m, s, state.x, state.y, L);
+    WarmStartManifold(m, s, A, B, state, L);
     StoreVisit(GlobalBodies{b}, h.x, h.y, state.x, A, B);
 }
 __device__ __forceinline__ void SolveSlot(const ManifoldSoA& m, const BodySoA& b, int s, const StepParams& p) {
@@ -482,9 +484,25 @@ __device__ __forceinline__ void SolveSlot(const ManifoldSoA& m, const BodySoA& b
     m.state[s] = state;
 }
 
+// A colour's warm start: everything but the bodies' velocities is loaded
+// before the previous colour's ends (the warm start changes nothing else).
 __global__ void k_warm(ManifoldSoA m, BodySoA b, int begin, int end) {
-    int s = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < end) WarmSlot(m, b, s);
+    LetDependentsLaunch();
+    const int s = begin + blockIdx.x * blockDim.x + threadIdx.x;
+    int4 h = make_int4(0, 0, 0, 0);
+    uint2 state = make_uint2(0u, 0u);
+    SolveLanes L;
+    if (s < end) {
+        h = m.head[s];
+        state = m.state[s];
+        if (state.x & kGroupActive) LoadSolveLanes(m, s, state.x, state.y, L);
+    }
+    WaitForPrerequisites();
+    if (!(state.x & kGroupActive)) return;
+    BodyState A, B;
+    LoadVisit(GlobalBodies{b}, h.x, h.y, state.x, A, B);
+    WarmStartManifold(m, s, A, B, state, L);
+    StoreVisit(GlobalBodies{b}, h.x, h.y, state.x, A, B);
 }
 // A colour sweep: the visit's prestep lanes load before the previous sweep
 // ends (they do not change during the sweeps); state, impulses and bodies after.
@@ -812,6 +830,8 @@ bepugpu_status Scene::Allocate(Context* ctx, uint32_t nb, uint32_t nm, uint32_t 
     L.groupJointRefs = take(8 * J); L.groupJointOffsets = take(4 * (2 * (M + J) + 2));
     L.bodyRecords = take(sizeof(bepugpu_body) * B);
     L.shape = take(16 * B); L.genSlots = take(4 * M);
+    L.flowChunks = take(8 * M); L.flowVisit = take(8 * M); L.flowDegree = take(4 * B); L.flowBegin = take(4 * (B + 1));
+    L.flowCsr = take(8 * M); L.flowLin = take(16 * B); L.flowAng = take(16 * B);
     arenaBytes = bytes;
     // The arena and the staging buffer are blocks of the context's heap, like
     // the ones a restore takes after a spill.
@@ -877,6 +897,10 @@ void Scene::Rebase() {
     bodyRecords = (bepugpu_body*)(base + L.bodyRecords);
     shape = (float4*)(base + L.shape);
     genSlotsDev = (int32_t*)(base + L.genSlots);
+    flow.chunks = (int2*)(base + L.flowChunks); flow.visit = (int2*)(base + L.flowVisit);
+    flow.degree = (int32_t*)(base + L.flowDegree); flow.csrBegin = (int32_t*)(base + L.flowBegin);
+    flow.csr = (int32_t*)(base + L.flowCsr); flow.lin = (float4*)(base + L.flowLin);
+    flow.ang = (float4*)(base + L.flowAng);
 }
 
 // Moves the arena to pinned host memory and gives the scene's heap blocks
@@ -1119,7 +1143,10 @@ bepugpu_status Scene::BuildGraph(Context* ctx, const StepParams& p, uint32_t fla
         launchesPerStep++;
     }
     CK(cudaEventRecordWithFlags(evPhase[2], stream, cudaEventRecordExternal));
-    if (solve) {
+    const bool flows = solve && !nj;  // manifolds alone: the sweeps in one launch (flow.cu)
+    const bool flowWarm = flows && flow.chunkCount <= kFlowWarmChunks;
+    if (solve && !flowWarm) {
+        bool after = false;  // the first one follows the prestep, whose lanes it loads: no early start
         for (int c = 0; c < colours; c++) {
             int b0 = manifoldOffsets[c], b1 = manifoldOffsets[c + 1];
             int j0 = nj ? jointOffsets[c] : 0, j1 = nj ? jointOffsets[c + 1] : 0;
@@ -1127,13 +1154,25 @@ bepugpu_status Scene::BuildGraph(Context* ctx, const StepParams& p, uint32_t fla
                 warmMixed<<<Blocks(b1 - b0 + j1 - j0, T), T, 0, stream>>>(ms, b, js, b0, b1, j0, j1);
                 launchesPerStep++;
             } else if (b1 > b0) {
-                k_warm<<<Blocks(b1 - b0, T), T, 0, stream>>>(ms, b, b0, b1);
+                if (after) CK(LaunchAfterSweep(k_warm, Blocks(b1 - b0, T), T, stream, ms, b, b0, b1));
+                else k_warm<<<Blocks(b1 - b0, T), T, 0, stream>>>(ms, b, b0, b1);
                 launchesPerStep++;
             }
+            after = after || b1 - b0 + j1 - j0 > 0;
         }
     }
     CK(cudaEventRecordWithFlags(evPhase[3], stream, cudaEventRecordExternal));
-    if (solve) {
+    if (flows) {
+        int flowLaunches = 0;
+        bepugpu_status fs = LaunchFlow(ctx, this, p, flowWarm, &flowLaunches);
+        if (fs != BEPUGPU_OK) {
+            cudaGraph_t dropped;
+            cudaStreamEndCapture(stream, &dropped);
+            if (dropped) cudaGraphDestroy(dropped);
+            return fs;
+        }
+        launchesPerStep += flowLaunches;
+    } else if (solve) {
         for (int it = 0; it < p.iterationLimit; it++)
             for (int c = 0; c < colours; c++) {
                 int b0 = manifoldOffsets[c], b1 = manifoldOffsets[c + 1];
@@ -1407,6 +1446,7 @@ void bepugpu_destroy(bepugpu_context* c) {
     ShutdownServers(ctx);  // their workers step these scenes
     ctx->batch.reset();
     ctx->scenes.clear();
+    if (ctx->flowError) cudaFreeHost(ctx->flowError);
     delete ctx;
 }
 
@@ -1451,7 +1491,7 @@ bepugpu_status bepugpu_synchronize(bepugpu_context* c) {
             }
         }
     }
-    return BEPUGPU_OK;
+    return FlowStatus(ctx);
 }
 
 bepugpu_status bepugpu_scene_create(bepugpu_context* c, uint32_t nb, uint32_t nm, uint32_t nj, int32_t* out) {
@@ -1637,6 +1677,10 @@ bepugpu_status bepugpu_upload_constraints(bepugpu_context* c, int32_t id, const 
     {
         bepugpu_status gst = s->UploadGroups(ctx);
         if (gst != BEPUGPU_OK) return gst;
+    }
+    {
+        bepugpu_status fst = s->UploadFlow(ctx, a.data() + nj, bb.data() + nj);
+        if (fst != BEPUGPU_OK) return fst;
     }
     s->hostSlotOf = plan.slotOf;
     s->maxBodyReferenced = -1;
@@ -1853,7 +1897,7 @@ bepugpu_status bepugpu_step_state(bepugpu_context* c, int32_t id, bepugpu_body_s
     st = QueueStateDownload(ctx, s, bodies, nb, man, nm);
     CK(cudaStreamSynchronize(s->stream));
     s->asyncPending = false;
-    return st;
+    return st == BEPUGPU_OK ? FlowStatus(ctx) : st;
 }
 
 bepugpu_status bepugpu_download_state(bepugpu_context* c, int32_t id, bepugpu_body_state* bodies, uint32_t nb,
@@ -1871,7 +1915,7 @@ bepugpu_status bepugpu_download_state(bepugpu_context* c, int32_t id, bepugpu_bo
     }
     st = QueueStateDownload(ctx, s, bodies, nb, man, nm);
     CK(cudaStreamSynchronize(s->stream));
-    return st;
+    return st == BEPUGPU_OK ? FlowStatus(ctx) : st;
 }
 
 bepugpu_status bepugpu_update_bodies(bepugpu_context* c, int32_t id, const bepugpu_body* bodies, uint32_t n) {

@@ -176,6 +176,30 @@ bepugpu_status LaunchPrestepped(Context* ctx, Scene* s, const StepParams& p, uin
 // split, the group CTA's own pass over its bodies and manifolds being cheaper
 // there than two more launches and the copy of the solve lanes.
 constexpr int32_t kSplitPrologueConstraints = 1024;
+// The barrier-free sweeps' tables (flow.cu), for the manifold slots outside
+// island groups.
+struct FlowTables {
+    int2* chunks;             // slots [x, y) of one colour, at most 32, colour-major
+    int2* visit;              // per slot: its place among its bodies A's and B's visits of a sweep, -1 none
+    int32_t* degree;          // per body: visits of a sweep
+    int32_t* csrBegin;        // per body: its entries of csr, bodies + 1
+    int32_t* csr;             // slot << 1 | end (0 A, 1 B), ascending
+    float4 *lin, *ang;        // per body: velocity, w = visits so far (bits)
+    int* error;
+    int chunkCount;
+};
+// The solve sweeps of the slots outside groups, after their prestep and, with
+// `warm`, their warm start: two launches.
+bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool warm, int* launches);
+// Scenes of more chunks than this (four for each of the 8 warps a GB300 SM
+// holds of k_flow) warm-start in a launch per colour, whose smaller kernel
+// keeps more loads in flight.  Measured in a step, in the flow launch against
+// per colour: 82,000 manifolds 7.8 and 8.0 ms (four frames of a settling heap
+// of 16 colours), 188,667 manifolds 325 and 332 us, 425,999 754 and 744 us,
+// 757,861 1,388 and 1,354 us.
+constexpr int kFlowWarmChunks = 4864;
+// TIMEOUT when a wait of a finished flow launch ran out (and clears it).
+bepugpu_status FlowStatus(Context* ctx);
 // Joints (joints.cu): record checks, upload into the scene's joint slots, and
 // the accumulated impulses back into records.
 bepugpu_status CheckJointRecords(Context* ctx, const bepugpu_joint* joints, uint32_t nj, int32_t bodies);
@@ -241,6 +265,7 @@ struct ArenaLayout {
     size_t groupJointRefs, groupJointOffsets;
     size_t bodyRecords;
     size_t shape, genSlots;
+    size_t flowChunks, flowVisit, flowDegree, flowBegin, flowCsr, flowLin, flowAng;
 };
 
 struct Server;
@@ -308,6 +333,13 @@ struct Scene {
         g.count = groupPlan.globalCount;
         return g;
     }
+    FlowTables flow{};
+    // flow.cu: the tables from the constraint upload's records (bodies a, b
+    // per manifold record), or from update_pairs' sorted (body, entry) keys.
+    bepugpu_status UploadFlow(Context* ctx, const int32_t* a, const int32_t* b);
+    bepugpu_status UploadFlowChunks(Context* ctx);
+    bepugpu_status BuildFlowOnDevice(Context* ctx, const unsigned long long* entries, int count, const int2* ends,
+                                     const int* slots);
     int SweepColours() const { return manifoldOffsets.empty() ? 0 : (int)manifoldOffsets.size() - 1; }
     uint32_t maxBodies = 0, maxManifolds = 0, maxJoints = 0;
     DeviceHeap* heap = nullptr;     // the owning context's heap: arena and staging blocks
@@ -437,6 +469,8 @@ struct Context {
     float lastMs = 0.f;
     int batchThreads = 0;  // threads per CTA of batched launches, 0 = from the groups' colour sizes
     uint64_t batchEpoch = 0;  // batched calls so far (Scene::batchStamp)
+    int* flowError = nullptr;   // page-locked: a flow launch's wait ran out (flow.cu)
+    int flowBlocksPerSm = 0;
     std::vector<bepugpu_server*> servers;  // live servers: shut down before the scenes go
     void SetError(const char* fmt, ...);
 };

@@ -293,7 +293,9 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
                 int2 r = kShared ? sRefs[j] : t.refs[g.mBegin + j];
                 BodyState A, B;
                 LoadVisit(bv, r.x, r.y, st.x, A, B);
-                WarmStartManifold(ml, sl, A, B, st);
+                SolveLanes L;
+                LoadSolveLanes(ml, sl, st.x, st.y, L);
+                WarmStartManifold(ml, sl, A, B, st, L);
                 StoreVisit(bv, r.x, r.y, st.x, A, B);
             }
             __syncthreads();

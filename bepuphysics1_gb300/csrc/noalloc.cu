@@ -255,7 +255,9 @@ __global__ void __launch_bounds__(kThreads) k_step_noalloc(bepugpu_body* bodies,
                 int4 h = v.m.head[s];
                 BodyState A, B;
                 LoadVisit(GlobalBodies{v.b}, h.x, h.y, st.x, A, B);
-                WarmStartManifold(v.m, s, A, B, st);
+                SolveLanes L;
+                LoadSolveLanes(v.m, s, st.x, st.y, L);
+                WarmStartManifold(v.m, s, A, B, st, L);
                 StoreVisit(GlobalBodies{v.b}, h.x, h.y, st.x, A, B);
             }
             __syncthreads();

@@ -347,6 +347,7 @@ struct DeviceColouring {
     int* colour;
     int* order;
     int* slotOf;
+    const unsigned long long* entries = nullptr;  // (dynamic body << 32 | entry), sorted, 2 n of them (~0: none)
     int colours = 0;
     std::vector<int32_t> offsets;
 };
@@ -362,6 +363,7 @@ static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, i
     if (n == 0) return BEPUGPU_OK;
     const size_t padded = PaddedSize((size_t)2 * n);
     auto* entries = c.take<unsigned long long>(padded);
+    out.entries = entries;
     auto* at = c.take<int2>(n);
     int* counters = c.take<int>(64);
     k_colour_entries<<<(n + T - 1) / T, T, 0, st>>>(ends, n, s->b, entries, out.colour);
@@ -564,6 +566,11 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
         CK(cudaMemcpyAsync(plan.slotOf.data(), col.slotOf, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
     }
     s->manifoldOffsets = col.offsets;
+    s->flow.chunkCount = 0;
+    if (n) {
+        bepugpu_status fs = s->BuildFlowOnDevice(ctx, col.entries, 2 * n, rec.ends, col.slotOf);
+        if (fs != BEPUGPU_OK) return fs;
+    }
     s->jointOffsets.assign(col.colours + 1, 0);
     s->hostSlotOf = plan.slotOf;
     s->m.count = n;

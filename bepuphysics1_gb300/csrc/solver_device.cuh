@@ -944,48 +944,6 @@ __device__ __forceinline__ float VelocityAlong(const BodyState& A, const BodySta
     return a + b;
 }
 
-// Warm start: ConvexContactManifoldConstraint.ExclusiveUpdate
-// (ConvexContactManifoldConstraint.cs:186-192) with the children's
-// ExclusiveUpdate bodies (ContactPenetrationConstraint.cs:240-271,
-// SlidingFrictionTwoAxis.cs:447-482, TwistFrictionConstraint.cs:182-204).
-__device__ __forceinline__ void WarmStartManifold(const ManifoldSoA& m, int s, BodyState& A, BodyState& B,
-                                                  uint2 state) {
-    const int cap = m.capacity;
-    const uint32_t children = state.y;
-    float4 acc4 = m.penacc[s];
-    const float accs[4] = {acc4.x, acc4.y, acc4.z, acc4.w};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        if (!ChildOn(children, k)) continue;
-        ApplyImpulse(A, B, accs[k], m.pj0[k * cap + s], m.pj1[k * cap + s], m.pj2[k * cap + s]);
-    }
-    if (state.x & kContactFriction) {
-        // ContactFrictionConstraint.ExclusiveUpdate (ContactFrictionConstraint.cs:258-289)
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            if (!ChildOn(children, 4 + k)) continue;
-            const float4 fr = m.cfr[k * cap + s];
-            ApplyImpulse(A, B, fr.w, fr, m.cfa[k * cap + s], m.cfb[k * cap + s]);
-        }
-        return;
-    }
-    if (!ChildOn(children, kSlidingChild)) return;  // no contacts
-    float4 f = m.fricacc[s];
-    float ax = f.x, ay = f.y;
-    float4 L1 = m.saxis[s], L2 = m.s3[s], A1 = m.s4[s], A2 = m.s5[s], B1 = m.s6[s], B2 = m.s7[s];
-    float lx = ax * L1.x + ay * L2.x;
-    float ly = ax * L1.y + ay * L2.y;
-    float lz = ax * L1.z + ay * L2.z;
-    ApplyLinear(A, lx, ly, lz);
-    ApplyAngular(A, ax * A1.x + ay * A2.x, ax * A1.y + ay * A2.y, ax * A1.z + ay * A2.z);
-    ApplyLinear(B, -lx, -ly, -lz);
-    ApplyAngular(B, ax * B1.x + ay * B2.x, ax * B1.y + ay * B2.y, ax * B1.z + ay * B2.z);
-    float4 j0 = m.pj0[s];  // twist axis = contact 0 normal = -linearA of penetration 0
-    const float gx = f.z * -j0.x, gy = f.z * -j0.y, gz = f.z * -j0.z;
-    ApplyAngular(A, gx, gy, gz);
-    ApplyAngular(B, -gx, -gy, -gz);
-}
-
 // Programmatic dependent launch: a sweep kernel lets the next one start its
 // preamble (griddepcontrol.launch_dependents) and waits for the previous one's
 // completion and memory (griddepcontrol.wait) before it reads what that one
@@ -1023,6 +981,49 @@ __device__ __forceinline__ void LoadSolveLanes(const ManifoldSoA& m, int s, uint
         L.B1 = m.s6[s];
     }
     if (twist) L.LEV = m.lever[s];
+}
+
+// Warm start: ConvexContactManifoldConstraint.ExclusiveUpdate
+// (ConvexContactManifoldConstraint.cs:186-192) with the children's
+// ExclusiveUpdate bodies (ContactPenetrationConstraint.cs:240-271,
+// SlidingFrictionTwoAxis.cs:447-482, TwistFrictionConstraint.cs:182-204).
+// L: the visit's lanes (LoadSolveLanes).
+__device__ __forceinline__ void WarmStartManifold(const ManifoldSoA& m, int s, BodyState& A, BodyState& B,
+                                                  uint2 state, const SolveLanes& L) {
+    const int cap = m.capacity;
+    const uint32_t children = state.y;
+    float4 acc4 = m.penacc[s];
+    const float accs[4] = {acc4.x, acc4.y, acc4.z, acc4.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (!ChildOn(children, k)) continue;
+        ApplyImpulse(A, B, accs[k], L.J0[k], L.J1[k], L.J2[k]);
+    }
+    if (state.x & kContactFriction) {
+        // ContactFrictionConstraint.ExclusiveUpdate (ContactFrictionConstraint.cs:258-289)
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (!ChildOn(children, 4 + k)) continue;
+            const float4 fr = m.cfr[k * cap + s];
+            ApplyImpulse(A, B, fr.w, fr, m.cfa[k * cap + s], m.cfb[k * cap + s]);
+        }
+        return;
+    }
+    if (!ChildOn(children, kSlidingChild)) return;  // no contacts
+    float4 f = m.fricacc[s];
+    float ax = f.x, ay = f.y;
+    const float4 L1 = L.L1, L2 = L.L2, A1 = L.A1, A2 = L.A2, B1 = L.B1, B2 = L.B2;
+    float lx = ax * L1.x + ay * L2.x;
+    float ly = ax * L1.y + ay * L2.y;
+    float lz = ax * L1.z + ay * L2.z;
+    ApplyLinear(A, lx, ly, lz);
+    ApplyAngular(A, ax * A1.x + ay * A2.x, ax * A1.y + ay * A2.y, ax * A1.z + ay * A2.z);
+    ApplyLinear(B, -lx, -ly, -lz);
+    ApplyAngular(B, ax * B1.x + ay * B2.x, ax * B1.y + ay * B2.y, ax * B1.z + ay * B2.z);
+    const float4 j0 = L.J0[0];  // twist axis = contact 0 normal = -linearA of penetration 0
+    const float gx = f.z * -j0.x, gy = f.z * -j0.y, gz = f.z * -j0.z;
+    ApplyAngular(A, gx, gy, gz);
+    ApplyAngular(B, -gx, -gy, -gz);
 }
 
 // One solver visit of a manifold: Solver.UnsafeSolveIteration (Solver.cs:285-314)
