@@ -21,6 +21,7 @@
 
 #include "../../include/bepugpu.h"
 #include "colouring.h"
+#include "grid_barrier.cuh"
 #include "solver_device.cuh"
 #include "bepugpu_internal.h"
 
@@ -573,39 +574,6 @@ __global__ void k_solve_mixed(ManifoldSoA m, BodySoA b, JointSoA j, StepParams p
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < je - jb) SolveJointSlot<kAdded>(j, b, jb + t, p);
     else if (mb + t - (je - jb) < me) SolveSlot(m, b, mb + t - (je - jb), p);
-}
-
-// Bounded grid barrier for the cooperative kernel.  Thread 0 of each block
-// arrives on a counter; the last arrival resets it and bumps the generation.
-// A wait that outlives kBarrierSpinLimit polls sets *err and the kernel returns.
-constexpr long long kBarrierSpinLimit = 1ll << 24;
-__device__ __forceinline__ bool GridBarrier(unsigned int* counter, volatile unsigned int* generation,
-                                            unsigned int& localGen, volatile int* err) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned int g = localGen;
-        __threadfence();
-        unsigned int arrived = atomicAdd(counter, 1u);
-        if (arrived == gridDim.x - 1) {
-            atomicExch(counter, 0u);
-            __threadfence();
-            atomicAdd((unsigned int*)generation, 1u);
-        } else {
-            long long spins = 0;
-            while (*generation == g) {
-                if (++spins > kBarrierSpinLimit) {
-                    *err = BEPUGPU_TIMEOUT;
-                    break;
-                }
-                if (*err) break;
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-    }
-    localGen++;
-    __syncthreads();
-    return *err == 0;
 }
 
 struct PersistentArgs {

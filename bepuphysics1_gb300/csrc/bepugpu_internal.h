@@ -27,13 +27,23 @@ struct BroadPhaseBuffers;
 void ReleaseBroadPhase(Scene* s);  // broadphase.cu
 struct Context;
 // broadphase.cu: the pair set into device memory (sorted 64-bit keys, lower
-// body << 32 | higher), the ascending bitonic sort of 64-bit keys it uses
-// (`padded` a power of two from PaddedSize), and a filler of largest keys.
+// body << 32 | higher).
 bepugpu_status RunBroadPhase(Context* ctx, Scene* s, float dt, unsigned& found);
 const unsigned long long* BroadPhasePairs(const Scene* s);
-size_t PaddedSize(size_t n);
-void SortKeys(unsigned long long* keys, size_t padded, cudaStream_t st);
-void FillKeys(unsigned long long* keys, size_t n, cudaStream_t st);
+// sort.cu: ascending stable sort of 64-bit keys by the bits a plan names --
+// lowBits from bit lowFrom on, then highBits from bit 32 on -- in one
+// cooperative launch.  `count` (device, null: capacity) keys, at most
+// `capacity`; `other` as large as `keys`; hist kSortHistWords words; *err is
+// set to TIMEOUT when a barrier's wait ran out.  Uses the scene's barrier words.
+struct SortDigits {
+    int passes;
+    int shift[10], bits[10];
+};
+constexpr int kSortBlocks = 64, kSortHistWords = kSortBlocks * 512;
+SortDigits SortPlan(int lowFrom, int lowBits, int highBits);
+int BitsFor(size_t values);  // bits that tell `values` values apart
+cudaError_t RadixSort(const Scene* s, unsigned long long* keys, unsigned long long* other, const unsigned* count,
+                      size_t capacity, const SortDigits& digits, unsigned* hist, int* err, cudaStream_t st);
 struct PairBuffers;                // pairs.cu
 void ReleasePairs(Scene* s);
 struct IslandBuffers;               // islands.cu
@@ -471,6 +481,7 @@ struct Context {
     uint64_t batchEpoch = 0;  // batched calls so far (Scene::batchStamp)
     int* flowError = nullptr;   // page-locked: a flow launch's wait ran out (flow.cu)
     int flowBlocksPerSm = 0;
+    int colourBlocksPerSm = 0;  // pairs.cu
     std::vector<bepugpu_server*> servers;  // live servers: shut down before the scenes go
     void SetError(const char* fmt, ...);
 };

@@ -18,14 +18,17 @@
 //   2. a body no wider than a cell enters every cell its box touches (at most
 //      eight) as a 64-bit key (cell code, body); wider bodies go to a short
 //      list;
-//   3. the keys are sorted (bitonic, the low 2048-element stages in shared
-//      memory), so each cell's bodies are contiguous;
+//   3. the keys are sorted (sort.cu) by the upper bits of their scrambled cell
+//      codes, about four values per body, so each cell's bodies lie in one
+//      short run -- the cells' order does not matter, so two passes are enough;
 //   4. a thread per key tests its body against the later keys of the same
 //      cell, and reports a pair only in the cell that holds the largest
 //      corner of the two boxes' minima -- a point of both boxes, so exactly
 //      one cell of each overlapping pair reports it;
-//   5. a thread per (wide body, body) tests the wide bodies against all;
-//   6. the pairs, as 64-bit keys, are sorted and copied back.
+//   5. threads over (wide body, body) test the wide bodies against all;
+//   6. the pairs, as 64-bit keys, are sorted.
+// The counts of entries, wide bodies and pairs stay on the device between the
+// launches; the host reads them once, at the end.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,13 +43,10 @@
 namespace bepugpu {
 namespace {
 
-constexpr int kSortBlock = 1024;            // threads of the shared-memory sort stages
-constexpr int kSortTile = 2 * kSortBlock;   // keys per shared-memory tile
-constexpr unsigned long long kNoKey = ~0ull;
-
 // Scalars of one call: [0] sum of box extents (float bits, atomics), [1]
-// bodies with a box, [2] wide-body count, [3] pair count, [4] cell entries.
-enum : int { kWExtent = 0, kWShaped, kWWide, kWPairs, kWEntries, kWords = 8 };
+// bodies with a box, [2] wide-body count, [3] pair count, [4] cell entries,
+// [5] status of the sorts' barriers.
+enum : int { kWExtent = 0, kWShaped, kWWide, kWPairs, kWEntries, kWError, kWords = 8 };
 
 // The bounding box of body i: lo.w = 0 (no shape), 1 (kinematic), 2 (dynamic).
 __device__ __forceinline__ float BoxOf(const BodySoA& b, const float4* __restrict__ shape, float dt, int i,
@@ -119,9 +119,13 @@ __device__ __forceinline__ float CellSize(const unsigned* words) {
 __device__ __forceinline__ int CellOf(float x, float inv) { return (int)floorf(x * inv); }
 // 10 bits per axis, wrapping: distinct cells far apart may share a code; the
 // overlap test keeps that from making pairs, and a box spans at most two
-// cells per axis, so it never meets the same code twice.
+// cells per axis, so it never meets the same code twice.  An odd factor
+// scrambles the 30 bits one to one: neighbouring cells differ in the upper
+// bits, which the entries are sorted by.
+constexpr int kCellCodeBits = 30;
 __device__ __forceinline__ unsigned CellCode(int x, int y, int z) {
-    return ((unsigned)(x & 1023) << 20) | ((unsigned)(y & 1023) << 10) | (unsigned)(z & 1023);
+    const unsigned code = ((unsigned)(x & 1023) << 20) | ((unsigned)(y & 1023) << 10) | (unsigned)(z & 1023);
+    return (code * 0x2545F491u) & ((1u << kCellCodeBits) - 1u);
 }
 
 // Cell entries of the bodies no wider than a cell; the wider ones to a list.
@@ -154,72 +158,6 @@ __global__ void k_bp_cells(const float4* __restrict__ lo, float4* __restrict__ h
                 if (at < keyCap) keys[at] = ((unsigned long long)CellCode(x, y, z) << 32) | (unsigned)i;
 }
 
-__global__ void k_fill_keys(unsigned long long* __restrict__ keys, size_t n) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) keys[i] = kNoKey;
-}
-
-// Bitonic stages with partner distance j >= kSortTile, one pair per thread.
-__global__ void k_bitonic_global(unsigned long long* __restrict__ keys, int j, int k) {
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;  // pair index
-    const unsigned i = 2 * t - (t & (j - 1));                   // lower element of the pair
-    const unsigned l = i + j;
-    const bool up = (i & k) == 0;
-    const unsigned long long a = keys[i], b = keys[l];
-    if ((a > b) == up) { keys[i] = b; keys[l] = a; }
-}
-// The stages of one k with j < kSortTile (all of them when k <= kSortTile: a
-// whole tile sort), in shared memory; each block owns one tile.
-__global__ void __launch_bounds__(kSortBlock) k_bitonic_tile(unsigned long long* __restrict__ keys, int kFrom,
-                                                             int kTo, int jFrom) {
-    __shared__ unsigned long long s[kSortTile];
-    const unsigned base = blockIdx.x * kSortTile;
-    const unsigned t = threadIdx.x;
-    s[t] = keys[base + t];
-    s[t + kSortBlock] = keys[base + t + kSortBlock];
-    __syncthreads();
-    for (int k = kFrom; k <= kTo; k <<= 1) {
-        for (int j = (k == kFrom ? jFrom : k >> 1); j > 0; j >>= 1) {
-            const unsigned i = 2 * t - (t & (j - 1));
-            const unsigned l = i + j;
-            const bool up = ((base + i) & k) == 0;
-            const unsigned long long a = s[i], b = s[l];
-            if ((a > b) == up) { s[i] = b; s[l] = a; }
-            __syncthreads();
-        }
-    }
-    keys[base + t] = s[t];
-    keys[base + t + kSortBlock] = s[t + kSortBlock];
-}
-
-}  // namespace
-
-// The power of two at or above n, at least one tile.
-size_t PaddedSize(size_t n) {
-    size_t p = kSortTile;
-    while (p < n) p <<= 1;
-    return p;
-}
-
-// Ascending bitonic sort of `padded` keys (a power of two, at least one
-// tile): each tile sorted in shared memory, then for every larger k the wide
-// stages in global memory and the narrow ones in shared memory.
-void SortKeys(unsigned long long* keys, size_t padded, cudaStream_t st) {
-    k_bitonic_tile<<<(unsigned)(padded / kSortTile), kSortBlock, 0, st>>>(keys, 2, kSortTile, 1);
-    for (size_t k = 2 * kSortTile; k <= padded; k <<= 1) {
-        for (size_t j = k >> 1; j >= kSortTile; j >>= 1)
-            k_bitonic_global<<<(unsigned)(padded / 2 / 256), 256, 0, st>>>(keys, (int)j, (int)k);
-        k_bitonic_tile<<<(unsigned)(padded / kSortTile), kSortBlock, 0, st>>>(keys, (int)k, (int)k, kSortTile / 2);
-    }
-}
-
-// keys[0, n) set to the largest key (sorts last).
-void FillKeys(unsigned long long* keys, size_t n, cudaStream_t st) {
-    if (n) k_fill_keys<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(keys, n);
-}
-
-namespace {
-
 // BoundingBox.Intersects (BoundingBox.cs:58-66) and the NoBroadPhase rule of
 // two kinematic bodies.
 __device__ __forceinline__ bool MakesPair(float4 la, float4 ha, float4 lb, float4 hb) {
@@ -234,46 +172,58 @@ __device__ __forceinline__ void Report(int a, int b, unsigned long long* __restr
     if (at < capacity) pairs[at] = ((unsigned long long)min(a, b) << 32) | (unsigned)max(a, b);
 }
 
-// One thread per sorted cell entry: the later entries of the same cell.
-__global__ void k_bp_cell_pairs(const unsigned long long* __restrict__ keys, unsigned entries,
-                                const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                const unsigned* __restrict__ words, unsigned long long* __restrict__ pairs,
-                                unsigned capacity, unsigned* __restrict__ count) {
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= entries) return;
-    const unsigned long long ki = keys[i];
-    const unsigned code = (unsigned)(ki >> 32);
-    const int a = (int)(ki & 0xffffffffu);
-    const float4 la = lo[a], ha = hi[a];
+// Threads over the sorted cell entries: each tests the later entries of its
+// cell.  A run of entries that agree in the upper `sortedBits` code bits may
+// hold several cells.
+__global__ void k_bp_cell_pairs(const unsigned long long* __restrict__ keys, const float4* __restrict__ lo,
+                                const float4* __restrict__ hi, unsigned* __restrict__ words, int sortedBits,
+                                unsigned long long* __restrict__ pairs, unsigned capacity) {
+    const unsigned entries = words[kWEntries];
     const float inv = 1.f / CellSize(words);
-    for (unsigned j = i + 1; j < entries; j++) {
-        const unsigned long long kj = keys[j];
-        if ((unsigned)(kj >> 32) != code) break;
-        const int b = (int)(kj & 0xffffffffu);
-        const float4 lb = lo[b], hb = hi[b];
-        if (!MakesPair(la, ha, lb, hb)) continue;
-        // report in the cell of the largest corner of the minima only
-        const unsigned home = CellCode(CellOf(fmaxf(la.x, lb.x), inv), CellOf(fmaxf(la.y, lb.y), inv),
-                                       CellOf(fmaxf(la.z, lb.z), inv));
-        if (home == code) Report(a, b, pairs, capacity, count);
+    const int drop = kCellCodeBits - sortedBits;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < entries; i += gridDim.x * blockDim.x) {
+        const unsigned long long ki = keys[i];
+        const unsigned code = (unsigned)(ki >> 32);
+        const int a = (int)(ki & 0xffffffffu);
+        const float4 la = lo[a], ha = hi[a];
+        for (unsigned j = i + 1; j < entries; j++) {
+            const unsigned long long kj = keys[j];
+            const unsigned other = (unsigned)(kj >> 32);
+            if (other >> drop != code >> drop) break;
+            if (other != code) continue;
+            const int b = (int)(kj & 0xffffffffu);
+            const float4 lb = lo[b], hb = hi[b];
+            if (!MakesPair(la, ha, lb, hb)) continue;
+            // report in the cell of the largest corner of the minima only
+            const unsigned home = CellCode(CellOf(fmaxf(la.x, lb.x), inv), CellOf(fmaxf(la.y, lb.y), inv),
+                                           CellOf(fmaxf(la.z, lb.z), inv));
+            if (home == code) Report(a, b, pairs, capacity, words + kWPairs);
+        }
     }
 }
 
-// One thread per (wide body, body): wide bodies against every other body
+// Threads over (wide body, body): wide bodies against every other body
 // (a pair of two wide bodies from the lower one only).
-__global__ void k_bp_wide_pairs(const int* __restrict__ wide, unsigned wideCount, int n,
-                                const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                const unsigned* __restrict__ words, unsigned long long* __restrict__ pairs,
-                                unsigned capacity, unsigned* __restrict__ count) {
-    const unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (unsigned long long)wideCount * n) return;
-    const int w = wide[t / n], b = (int)(t % n);
-    if (b == w) return;
-    const float4 lb = lo[b], hb = hi[b];
-    if (__float_as_int(lb.w) == 0) return;
-    const float4 la = lo[w], ha = hi[w];
-    if (hb.w != 0.f && b < w) return;  // two wide bodies: from the lower one
-    if (MakesPair(la, ha, lb, hb)) Report(w, b, pairs, capacity, count);
+__global__ void k_bp_wide_pairs(const int* __restrict__ wide, unsigned wideCap, int n, const float4* __restrict__ lo,
+                                const float4* __restrict__ hi, unsigned* __restrict__ words,
+                                unsigned long long* __restrict__ pairs, unsigned capacity) {
+    const unsigned long long work = (unsigned long long)min(words[kWWide], wideCap) * n;
+    for (unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; t < work;
+         t += (unsigned long long)gridDim.x * blockDim.x) {
+        const int w = wide[t / n], b = (int)(t % n);
+        if (b == w) continue;
+        const float4 lb = lo[b], hb = hi[b];
+        if (__float_as_int(lb.w) == 0) continue;
+        const float4 la = lo[w], ha = hi[w];
+        if (hb.w != 0.f && b < w) continue;  // two wide bodies: from the lower one
+        if (MakesPair(la, ha, lb, hb)) Report(w, b, pairs, capacity, words + kWPairs);
+    }
+}
+
+// Sorted keys as (lower, higher) records, the caller's layout.
+__global__ void k_bp_unpack(const unsigned long long* __restrict__ pairs, unsigned n, int2* __restrict__ out) {
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = make_int2((int)(pairs[i] >> 32), (int)(pairs[i] & 0xffffffffu));
 }
 
 }  // namespace
@@ -293,15 +243,19 @@ struct BroadPhaseBuffers {
     int* wide = nullptr;
     unsigned long long* keys = nullptr;   // cell entries
     unsigned long long* pairs = nullptr;  // (lower << 32) | higher, then sorted
+    unsigned long long* other = nullptr;  // the sorts' second buffer
     unsigned* words = nullptr;
-    size_t bodyCap = 0, keyCap = 0, pairCap = 0;
+    unsigned* hist = nullptr;             // the sorts' digit counts
+    size_t bodyCap = 0, keyCap = 0, pairCap = 0, otherCap = 0;
     ~BroadPhaseBuffers() {
         cudaFree(lo);
         cudaFree(hi);
         cudaFree(wide);
         cudaFree(keys);
         cudaFree(pairs);
+        cudaFree(other);
         cudaFree(words);
+        cudaFree(hist);
     }
 };
 
@@ -353,49 +307,48 @@ bepugpu_status RunBroadPhase(Context* ctx, Scene* s, float dt, unsigned& found) 
         bp.bodyCap = n;
         wideCap = n;
     }
-    size_t wordsCap = bp.words ? kWords : 0;
+    size_t wordsCap = bp.words ? kWords : 0, histCap = bp.hist ? kSortHistWords : 0;
     CK(Grow(bp.words, wordsCap, (size_t)kWords));
-    CK(Grow(bp.keys, bp.keyCap, PaddedSize((size_t)8 * n)));  // at most eight cells a body
-    CK(Grow(bp.pairs, bp.pairCap, PaddedSize((size_t)4 * n)));
+    CK(Grow(bp.hist, histCap, (size_t)kSortHistWords));
+    CK(Grow(bp.keys, bp.keyCap, (size_t)8 * n));  // at most eight cells a body
+    CK(Grow(bp.pairs, bp.pairCap, (size_t)4 * n));
+    CK(Grow(bp.other, bp.otherCap, std::max(bp.keyCap, bp.pairCap)));
     const cudaStream_t st = s->stream;
+    int* err = (int*)(bp.words + kWError);
+    // about four sorted code values per body: runs of an entry or two
+    const int cellBits = std::min(kCellCodeBits, std::max(12, BitsFor((size_t)4 * n)));
+    const int bodyBits = BitsFor((size_t)n);
     CK(cudaMemsetAsync(bp.words, 0, sizeof(unsigned) * kWords, st));
     k_bp_boxes<<<(n + 255) / 256, 256, 0, st>>>(s->b, s->shape, dt, bp.lo, bp.hi, bp.words);
     k_bp_cells<<<(n + 255) / 256, 256, 0, st>>>(bp.lo, bp.hi, n, bp.words, bp.keys, (unsigned)bp.keyCap, bp.wide,
                                                (unsigned)wideCap);
-    unsigned w[kWords];
-    CK(cudaMemcpyAsync(w, bp.words, sizeof(w), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    const unsigned entries = w[kWEntries], wideCount = std::min<unsigned>(w[kWWide], (unsigned)wideCap);
-    const size_t sortedEntries = PaddedSize(entries);
-    if (entries < sortedEntries)
-        k_fill_keys<<<(unsigned)((sortedEntries - entries + 255) / 256), 256, 0, st>>>(bp.keys + entries,
-                                                                                    sortedEntries - entries);
-    SortKeys(bp.keys, sortedEntries, st);
     CK(cudaGetLastError());
+    CK(RadixSort(s, bp.keys, bp.other, bp.words + kWEntries, bp.keyCap,
+                 SortPlan(32 + kCellCodeBits - cellBits, cellBits, 0), bp.hist, err, st));
+    // one thread per possible entry up to 16 blocks an SM
+    const int blocks = std::max(1, std::min((int)((8 * (size_t)n + 127) / 128), ctx->smCount * 16));
     for (int attempt = 0; attempt < 2; attempt++) {
-        CK(cudaMemsetAsync(bp.words + kWPairs, 0, sizeof(unsigned), st));
-        if (entries)
-            k_bp_cell_pairs<<<(entries + 127) / 128, 128, 0, st>>>(bp.keys, entries, bp.lo, bp.hi, bp.words,
-                                                                  bp.pairs, (unsigned)bp.pairCap,
-                                                                  bp.words + kWPairs);
-        const unsigned long long wideWork = (unsigned long long)wideCount * n;
-        if (wideWork)
-            k_bp_wide_pairs<<<(unsigned)((wideWork + 255) / 256), 256, 0, st>>>(
-                bp.wide, wideCount, n, bp.lo, bp.hi, bp.words, bp.pairs, (unsigned)bp.pairCap, bp.words + kWPairs);
+        if (attempt) CK(cudaMemsetAsync(bp.words + kWPairs, 0, sizeof(unsigned), st));
+        k_bp_cell_pairs<<<blocks, 128, 0, st>>>(bp.keys, bp.lo, bp.hi, bp.words, cellBits, bp.pairs,
+                                                (unsigned)bp.pairCap);
+        k_bp_wide_pairs<<<blocks, 128, 0, st>>>(bp.wide, (unsigned)wideCap, n, bp.lo, bp.hi, bp.words, bp.pairs,
+                                                (unsigned)bp.pairCap);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(&found, bp.words + kWPairs, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        // the pairs in ascending order
+        CK(RadixSort(s, bp.pairs, bp.other, bp.words + kWPairs, bp.pairCap, SortPlan(0, bodyBits, bodyBits), bp.hist,
+                     err, st));
+        unsigned w[kWords];
+        CK(cudaMemcpyAsync(w, bp.words, sizeof(w), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        if (PaddedSize(found) <= bp.pairCap) break;
-        CK(Grow(bp.pairs, bp.pairCap, PaddedSize(found)));  // too many pairs for the buffer: grow, test again
-    }
-    // the pairs in ascending order: pad with the largest key and sort
-    const size_t sortedPairs = PaddedSize(found);
-    if (found) {
-        if (sortedPairs > found)
-            k_fill_keys<<<(unsigned)((sortedPairs - found + 255) / 256), 256, 0, st>>>(bp.pairs + found,
-                                                                                      sortedPairs - found);
-        SortKeys(bp.pairs, sortedPairs, st);
-        CK(cudaGetLastError());
+        if (w[kWError]) {
+            cudaMemsetAsync(s->BarrierCounter(), 0, sizeof(unsigned), st);
+            ctx->SetError("broad phase: a sort's grid barrier wait ran out");
+            return BEPUGPU_TIMEOUT;
+        }
+        found = w[kWPairs];
+        if (found <= bp.pairCap) break;
+        CK(Grow(bp.pairs, bp.pairCap, (size_t)found));  // too many pairs for the buffer: grow, test again
+        CK(Grow(bp.other, bp.otherCap, bp.pairCap));
     }
     return BEPUGPU_OK;
 }
@@ -423,14 +376,11 @@ extern "C" bepugpu_status bepugpu_broad_phase(bepugpu_context* c, int32_t id, fl
     const cudaStream_t st = s->stream;
     BroadPhaseBuffers& bp = *s->broadPhase;
     const uint32_t nw = std::min<uint32_t>(found, max_pairs);
-    std::vector<unsigned long long> host(nw);
     if (nw) {
-        CK(cudaMemcpyAsync(host.data(), bp.pairs, sizeof(unsigned long long) * nw, cudaMemcpyDeviceToHost, st));
+        k_bp_unpack<<<(nw + 255) / 256, 256, 0, st>>>(bp.pairs, nw, (int2*)bp.other);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(pairs, bp.other, sizeof(int2) * nw, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-    }
-    for (uint32_t k = 0; k < nw; k++) {
-        pairs[2 * k] = (int32_t)(host[k] >> 32);
-        pairs[2 * k + 1] = (int32_t)(host[k] & 0xffffffffu);
     }
     *pair_count = found;
     return BEPUGPU_OK;

@@ -6,15 +6,16 @@
 // is recoloured on the device.
 //
 //   1. the broad phase leaves the pair keys sorted in device memory;
-//   2. each record looks its pair up in them (kept or dropped), each pair
-//      looks itself up in the sorted old keys (kept or new);
+//   2. the old records' keys go into a hash table, where each pair looks
+//      itself up: found, its records are kept, else it is new;
 //   3. prefix sums give the new list: the kept records in their order, then
 //      the new pairs ascending;
 //   4. the colouring -- the smallest colour no earlier entry sharing a dynamic
-//      body took, the host's greedy colouring in list order -- runs as rounds
-//      of Jones-Plassmann with the list index as priority: an entry takes its
+//      body took, the host's greedy colouring in list order -- runs as
+//      Jones-Plassmann with the list index as priority: an entry takes its
 //      colour once the entries before it at each of its dynamic bodies have
-//      theirs, which is exactly the greedy choice;
+//      theirs, which is exactly the greedy choice; one cooperative launch, the
+//      entries polling the ones before them;
 //   5. slots follow the colour-major order (a sort of (colour, index) keys) and
 //      the records' lanes move to them, new records start empty.
 #include <cuda_runtime.h>
@@ -86,31 +87,37 @@ __device__ __forceinline__ unsigned long long PairKey(int a, int b) {
     const int lo = min(a, b), hi = max(a, b);
     return ((unsigned long long)(unsigned)lo << 32) | (unsigned)hi;
 }
-__device__ __forceinline__ bool Contains(const unsigned long long* __restrict__ keys, int n, unsigned long long k) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (keys[mid] < k) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo < n && keys[lo] == k;
+// The hash table of the old records: open addressing over a power of two of
+// slots, at least twice the records; a slot is the record's key and, in rec,
+// its index.  Two records of one pair take a slot each.
+__device__ __forceinline__ unsigned HashOf(unsigned long long key, unsigned slots) {
+    return (unsigned)((key * 0x9E3779B97F4A7C15ull) >> 32) & (slots - 1);
 }
-
-// Old records: their keys in record order and a copy to sort.
-__global__ void k_old_keys(ManifoldSoA m, const int32_t* __restrict__ slotOf, int n, unsigned long long* key,
-                           unsigned long long* sorted) {
+__global__ void k_old_table(ManifoldSoA m, const int32_t* __restrict__ slotOf, int n, unsigned long long* table,
+                            int* rec, unsigned slots) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n) return;
     const int4 h = m.head[slotOf[r]];
-    key[r] = sorted[r] = PairKey(h.x, h.y);
+    const unsigned long long key = PairKey(h.x, h.y);
+    for (unsigned at = HashOf(key, slots);; at = (at + 1) & (slots - 1))
+        if (atomicCAS(table + at, ~0ull, key) == ~0ull) {
+            rec[at] = r;
+            return;
+        }
 }
-// kept[r]: record r's pair is still reported; fresh[p]: pair p is new.
-__global__ void k_membership(const unsigned long long* __restrict__ oldKey, int nOld,
-                             const unsigned long long* __restrict__ oldSorted, const unsigned long long* __restrict__ pairs,
-                             int nPairs, int* kept, int* fresh) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < nOld) kept[t] = Contains(pairs, nPairs, oldKey[t]) ? 1 : 0;
-    if (t < nPairs) fresh[t] = Contains(oldSorted, nOld, pairs[t]) ? 0 : 1;
+// fresh[p]: pair p is new; kept[r] (zero before): record r's pair is still reported.
+__global__ void k_membership(const unsigned long long* __restrict__ table, const int* __restrict__ rec, unsigned slots,
+                             const unsigned long long* __restrict__ pairs, int nPairs, int* kept, int* fresh) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= nPairs) return;
+    const unsigned long long key = pairs[p];
+    bool known = false;
+    for (unsigned at = HashOf(key, slots); table[at] != ~0ull; at = (at + 1) & (slots - 1))
+        if (table[at] == key) {
+            kept[rec[at]] = 1;
+            known = true;
+        }
+    fresh[p] = known ? 0 : 1;
 }
 
 // The new list: record i's bodies (A, B as the record keeps them), its flags
@@ -175,45 +182,73 @@ __global__ void k_colour_positions(const unsigned long long* __restrict__ entrie
     if (ends[i].x == body) at[i].x = k;
     else at[i].y = k;
 }
-// One round: an entry whose predecessors at both dynamic bodies are coloured
-// takes the smallest colour none of its predecessors has.
-__global__ void k_colour_round(const unsigned long long* __restrict__ entries, const int2* __restrict__ at, int n,
-                               int* colour, int* waiting) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || colour[i] >= 0) return;
-    const int2 pos = at[i];
-    const int ks[2] = {pos.x, pos.y};
-    for (int e = 0; e < 2; e++) {
-        const int k = ks[e];
-        if (k <= 0) continue;
-        if ((entries[k - 1] >> 32) != (entries[k] >> 32)) continue;
-        if (((volatile int*)colour)[(int)(entries[k - 1] & 0xffffffffu)] < 0) {
-            atomicAdd(waiting, 1);
-            return;
-        }
-    }
-    for (int base = 0;; base += 64) {
-        unsigned long long used = 0;
-        for (int e = 0; e < 2; e++) {
-            const int k = ks[e];
-            if (k < 0) continue;
-            const unsigned long long body = entries[k] >> 32;
-            for (int q = k - 1; q >= 0 && (entries[q] >> 32) == body; q--) {
-                const int c = colour[(int)(entries[q] & 0xffffffffu)] - base;
-                if (c >= 0 && c < 64) used |= 1ull << c;
+// The colouring: every entry waits until the entries before it at its dynamic
+// bodies are coloured, then takes the smallest colour none of them has.  A
+// thread takes its entries in list order and every thread is resident
+// (cooperative launch), so the first uncoloured entry is never waiting; only
+// the colours themselves pass between threads, each read past L1, and a stale
+// one reads as uncoloured.  A wait of kColourSpinLimit polls ends with *err.
+// Bound by the polls' trips through L2 along the longest chain: 82,000 entries
+// of a settling heap in 80 us, where rounds of a launch each took 32 launches
+// and 270 us.
+constexpr int kColourSpinLimit = 1 << 22;
+__device__ __forceinline__ int PeekColour(const int* colour, int i) { return *(volatile const int*)(colour + i); }
+__global__ void k_colour_entries_in_order(const unsigned long long* __restrict__ entries, const int2* __restrict__ at,
+                                          int n, int* colour, int* err) {
+    const int stride = gridDim.x * blockDim.x;
+    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 - (int)(threadIdx.x & 31) < n; i0 += stride) {
+        const int i = i0;
+        bool done = i >= n;
+        const int2 pos = done ? make_int2(-1, -1) : at[i];
+        const int ks[2] = {pos.x, pos.y};
+        for (int spins = 0; !__all_sync(0xffffffffu, done); spins++) {
+            if (spins > kColourSpinLimit) {
+                *(volatile int*)err = BEPUGPU_TIMEOUT;
+                return;
             }
-        }
-        if (used != ~0ull) {
-            colour[i] = base + __ffsll((long long)~used) - 1;
-            return;
+            if (done) continue;
+            int chosen = -1;
+            for (int base = 0; chosen < 0; base += 64) {
+                unsigned long long used = 0;
+                bool ready = true;
+                for (int e = 0; e < 2; e++) {
+                    const int k = ks[e];
+                    if (k < 0) continue;
+                    const unsigned long long body = entries[k] >> 32;
+                    for (int q = k - 1; ready && q >= 0 && (entries[q] >> 32) == body; q--) {
+                        const int c = PeekColour(colour, (int)(entries[q] & 0xffffffffu));
+                        ready = c >= 0;
+                        if (c >= base && c < base + 64) used |= 1ull << (c - base);
+                    }
+                }
+                if (!ready) break;
+                if (used != ~0ull) chosen = base + __ffsll((long long)~used) - 1;
+            }
+            if (chosen >= 0) {
+                *(volatile int*)(colour + i) = chosen;
+                done = true;
+            }
         }
     }
 }
+// Entries per colour; the colours up to kColourBins through shared memory.
+constexpr int kColourBins = 1024;
 __global__ void k_colour_count(const int* __restrict__ colour, int n, int* counts, int* maxColour) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    atomicAdd(counts + colour[i], 1);
-    atomicMax(maxColour, colour[i]);
+    __shared__ int bins[kColourBins];
+    __shared__ int top;
+    for (int k = threadIdx.x; k < kColourBins; k += blockDim.x) bins[k] = 0;
+    if (threadIdx.x == 0) top = 0;
+    __syncthreads();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int c = colour[i];
+        if (c < kColourBins) atomicAdd(bins + c, 1);
+        else atomicAdd(counts + c, 1);
+        atomicMax(&top, c);
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < kColourBins; k += blockDim.x)
+        if (bins[k]) atomicAdd(counts + k, bins[k]);
+    if (threadIdx.x == 0) atomicMax(maxColour, top);
 }
 __global__ void k_slot_keys(const int* __restrict__ colour, int n, unsigned long long* keys) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -361,57 +396,63 @@ static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, i
     out.colours = 0;
     out.offsets.assign(1, 0);
     if (n == 0) return BEPUGPU_OK;
-    const size_t padded = PaddedSize((size_t)2 * n);
-    auto* entries = c.take<unsigned long long>(padded);
-    out.entries = entries;
+    auto* entries = c.take<unsigned long long>(2 * (size_t)n);
+    auto* other = c.take<unsigned long long>(2 * (size_t)n);  // the sorts' second buffer
+    auto* keys = c.take<unsigned long long>(n);
     auto* at = c.take<int2>(n);
-    int* counters = c.take<int>(64);
+    unsigned* hist = c.take<unsigned>(kSortHistWords);
+    // counts[0, n]: entries per colour; then the highest colour, and the status words
+    int* counts = c.take<int>((size_t)n + 4);
+    int *maxColour = counts + n + 1, *err = counts + n + 2;
+    CK(cudaMemsetAsync(counts, 0, sizeof(int) * ((size_t)n + 4), st));
     k_colour_entries<<<(n + T - 1) / T, T, 0, st>>>(ends, n, s->b, entries, out.colour);
-    FillKeys(entries + 2 * (size_t)n, padded - 2 * (size_t)n, st);
-    SortKeys(entries, padded, st);
+    // by body alone: the entries start in list order and the sort is stable
+    // (entries of no dynamic body have every bit set: one value more than the bodies)
+    CK(RadixSort(s, entries, other, nullptr, 2 * (size_t)n, SortPlan(0, 0, BitsFor((size_t)s->b.count + 1)), hist, err,
+                 st));
+    out.entries = entries;
     CK(cudaMemsetAsync(at, 0xff, sizeof(int2) * n, st));
     k_colour_positions<<<(int)((2 * (size_t)n + T - 1) / T), T, 0, st>>>(entries, 2 * n, ends, at);
     CK(cudaGetLastError());
-    // Rounds in batches of 16.  An entry still waiting counts itself; a round
-    // with none waiting leaves every entry coloured (the ready ones took their
-    // colours in it), so a batch whose last count is zero ends the loop.
-    // Each round colours at least the lowest uncoloured entry: n rounds suffice.
-    constexpr int kBatch = 16;
-    for (int round = 0;; round += kBatch) {
-        if (round > n + kBatch) {
-            ctx->SetError("update_pairs: the colouring did not finish");
-            return BEPUGPU_CUDA_ERROR;
-        }
-        CK(cudaMemsetAsync(counters, 0, sizeof(int) * kBatch, st));
-        for (int k = 0; k < kBatch; k++)
-            k_colour_round<<<(n + T - 1) / T, T, 0, st>>>(entries, at, n, out.colour, counters + k);
-        CK(cudaGetLastError());
-        int waiting = 0;
-        CK(cudaMemcpyAsync(&waiting, counters + kBatch - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        if (waiting == 0) break;
+    if (!ctx->colourBlocksPerSm)
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->colourBlocksPerSm, k_colour_entries_in_order, T, 0));
+    {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)std::max(1, std::min((n + T - 1) / T, ctx->colourBlocksPerSm * ctx->smCount)));
+        cfg.blockDim = dim3(T);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        CK(cudaLaunchKernelEx(&cfg, k_colour_entries_in_order, (const unsigned long long*)entries, (const int2*)at, n,
+                              out.colour, err));
     }
-    // colour counts and offsets
-    int* counts = c.take<int>(n + 1);
-    int* maxColour = counters + 32;
-    CK(cudaMemsetAsync(counts, 0, sizeof(int) * (n + 1), st));
-    CK(cudaMemsetAsync(maxColour, 0, sizeof(int), st));
-    k_colour_count<<<(n + T - 1) / T, T, 0, st>>>(out.colour, n, counts, maxColour);
-    int top = 0;
-    CK(cudaMemcpyAsync(&top, maxColour, sizeof(int), cudaMemcpyDeviceToHost, st));
+    k_colour_count<<<std::min((n + T - 1) / T, ctx->smCount), T, 0, st>>>(out.colour, n, counts, maxColour);
+    CK(cudaGetLastError());
+    int tail[2];  // the highest colour, the status
+    const int listed = std::min(n, kColourBins);
+    std::vector<int32_t> hc(listed);
+    CK(cudaMemcpyAsync(tail, maxColour, sizeof(tail), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hc.data(), counts, sizeof(int) * listed, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    out.colours = top + 1;
-    std::vector<int32_t> hc(out.colours);
-    CK(cudaMemcpyAsync(hc.data(), counts, sizeof(int) * out.colours, cudaMemcpyDeviceToHost, st));
-    // slots: (colour, entry) keys sorted
-    const size_t paddedSlots = PaddedSize((size_t)n);
-    auto* keys = c.take<unsigned long long>(paddedSlots);
+    if (tail[1]) {
+        cudaMemsetAsync(s->BarrierCounter(), 0, sizeof(unsigned), st);
+        ctx->SetError("update_pairs: the colouring did not finish");
+        return BEPUGPU_TIMEOUT;
+    }
+    out.colours = tail[0] + 1;
+    if (out.colours > listed) {
+        hc.resize(out.colours);
+        CK(cudaMemcpyAsync(hc.data(), counts, sizeof(int) * out.colours, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+    }
+    // slots: entries sorted by colour, in list order inside one
     k_slot_keys<<<(n + T - 1) / T, T, 0, st>>>(out.colour, n, keys);
-    FillKeys(keys + n, paddedSlots - n, st);
-    SortKeys(keys, paddedSlots, st);
+    CK(RadixSort(s, keys, other, nullptr, (size_t)n, SortPlan(0, 0, BitsFor((size_t)out.colours)), hist, err, st));
     k_slots<<<(n + T - 1) / T, T, 0, st>>>(keys, n, out.slotOf, out.order);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(st));
     out.offsets.assign(out.colours + 1, 0);
     for (int k = 0; k < out.colours; k++) out.offsets[k + 1] = out.offsets[k] + hc[k];
     return BEPUGPU_OK;
@@ -480,10 +521,12 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
     PairBuffers& P = *s->pairs;
     // scratch: keys, flags and scans, the new list, the colouring, the moved lanes
     const int nMax = std::max(std::max(nPairs, nOld), 1);
-    const size_t want = 256 * 64 + sizeof(unsigned long long) * (2 * (size_t)nMax + PaddedSize(nMax) +
-                                                               PaddedSize(2 * (size_t)nMax) + PaddedSize(nMax)) +
-                        sizeof(int) * (14 * (size_t)nMax + 64) + sizeof(float4) * kLanes * (size_t)nMax +
-                        sizeof(int2) * 2 * (size_t)nMax;
+    unsigned tableSlots = 64;
+    while (tableSlots < 2 * (unsigned)nMax) tableSlots *= 2;
+    const size_t want = 256 * 64 + (sizeof(unsigned long long) + sizeof(int)) * (size_t)tableSlots +
+                        sizeof(unsigned long long) * 5 * (size_t)nMax +
+                        sizeof(int) * (14 * (size_t)nMax + 64 + kSortHistWords) +
+                        sizeof(float4) * kLanes * (size_t)nMax + sizeof(int2) * 2 * (size_t)nMax;
     if (P.blockBytes < want) {
         cudaFree(P.block);
         P.block = nullptr;
@@ -498,9 +541,8 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
     }
     Carve cv{(char*)P.block};
     const int T = 256;
-    auto* oldKey = cv.take<unsigned long long>(nMax);
-    const size_t paddedOld = PaddedSize(nMax);
-    auto* oldSorted = cv.take<unsigned long long>(paddedOld);
+    auto* table = cv.take<unsigned long long>(tableSlots);
+    int* tableRec = cv.take<int>(tableSlots);
     int* kept = cv.take<int>(nMax);
     int* keptAt = cv.take<int>(nMax);
     int* fresh = cv.take<int>(nMax);
@@ -508,13 +550,13 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
     int* scanScratch = cv.take<int>(2 * (size_t)nMax + 64);
     int* totals = cv.take<int>(2);
     NewRecords rec{cv.take<int2>(nMax), cv.take<uint32_t>(nMax), cv.take<int32_t>(nMax)};
+    CK(cudaMemsetAsync(table, 0xff, sizeof(unsigned long long) * tableSlots, st));
     if (nOld) {
-        k_old_keys<<<(nOld + T - 1) / T, T, 0, st>>>(s->m, s->slotOf, nOld, oldKey, oldSorted);
-        FillKeys(oldSorted + nOld, paddedOld - nOld, st);
-        SortKeys(oldSorted, paddedOld, st);
+        CK(cudaMemsetAsync(kept, 0, sizeof(int) * nOld, st));
+        k_old_table<<<(nOld + T - 1) / T, T, 0, st>>>(s->m, s->slotOf, nOld, table, tableRec, tableSlots);
     }
-    const int nt = std::max(nOld, nPairs);
-    if (nt) k_membership<<<(nt + T - 1) / T, T, 0, st>>>(oldKey, nOld, oldSorted, pairs, nPairs, kept, fresh);
+    if (nPairs)
+        k_membership<<<(nPairs + T - 1) / T, T, 0, st>>>(table, tableRec, tableSlots, pairs, nPairs, kept, fresh);
     CK(cudaGetLastError());
     bepugpu_status sr = ExclusiveScan(ctx, kept, keptAt, nOld, scanScratch, totals, st);
     if (sr != BEPUGPU_OK) return sr;
