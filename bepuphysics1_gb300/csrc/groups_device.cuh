@@ -77,6 +77,7 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
                                           const StepParams& p, uint32_t flags, const GroupTables& t,
                                           const GroupDesc& g, int Bc, int Lc, int Jc, float4* smem,
                                           unsigned long long* census, bool nonConvex = false) {
+    const int tid = threadIdx.x, T = blockDim.x;
     const int nLocal = g.bEnd - g.bBegin, nm = g.mEnd - g.mBegin;
     GroupBodies bv;
     bv.pos = smem;
@@ -127,8 +128,48 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
         jRefs = (int2*)(jl.state + Jc);
         jl.count = nj;
     }
-    const int tid = threadIdx.x, T = blockDim.x;
     const int lbase = kShared ? 0 : g.mBegin;  // slot of local manifold 0 in ml
+
+    // The manifolds' inputs into shared memory, as asynchronous copies that run
+    // under the bodies' update: each lies where its own prestep products go
+    // (PrestepManifoldIO), read by the thread that copied it.  The chain of
+    // refs, head and contact loads from L2 held up the refresh and the prestep:
+    // 26 of the 108 thousand cycles of a group of the 65,536-box pile, whose
+    // ten steps went from 1,022 to 993 us.
+    ManifoldSoA mi = m;  // inputs of local manifold j: at mBegin + j, or staged at j
+    const int ibase = kShared && !kPrestepped ? 0 : g.mBegin;
+    if (kShared && !kPrestepped) {
+        float4* lanes = smem + 6 * Bc;
+        mi = ml;
+        mi.cnrm = ml.pj0;
+        mi.offA = ml.pj1;
+        mi.offB = ml.pj2;
+        mi.cpos = lanes + (nonConvex ? 25 : 15) * Lc;
+        mi.saxis = lanes + 19 * Lc;
+        mi.mat = ml.lever;
+    }
+    auto stage = [&]() {
+        const int cap = m.capacity;
+        for (int j = tid; j < nm; j += T) {
+            const int s = g.mBegin + j;
+            CopyAsync16(mi.head + j, m.head + s);
+            CopyAsync8(sRefs + j, t.refs + s);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                CopyAsync16(mi.cnrm + k * Lc + j, m.cnrm + k * cap + s);
+                CopyAsync16(mi.offA + k * Lc + j, m.offA + k * cap + s);
+                CopyAsync16(mi.offB + k * Lc + j, m.offB + k * cap + s);
+                CopyAsync16(mi.cpos + k * Lc + j, m.cpos + k * cap + s);
+                if (nonConvex) CopyAsync16(mi.cfr + k * Lc + j, m.cfr + k * cap + s);
+            }
+            CopyAsync16(mi.mat + j, m.mat + s);
+            CopyAsync16(mi.saxis + j, m.saxis + s);
+            CopyAsync16(mi.penacc + j, m.penacc + s);
+            CopyAsync16(mi.fricacc + j, m.fricacc + s);
+        }
+    };
+    // with islands a sleeping group returns before it needs any of them
+    if (kShared && !kPrestepped && !b.islandOf) stage();
 
     // Bodies into shared memory, through the candidacy update
     // (SimulationIslandMember.cs:53-164) and the force update (EntityBase.cs:911-975).
@@ -237,23 +278,20 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
     // no manifold with an active entry (an active kinematic body touching one
     // of its islands would have woken it), no body to move.
     if (__syncthreads_and(asleepAll)) return;
+    if (kShared && !kPrestepped && b.islandOf) stage();
     // Refresh, lanes in, prestep: a thread keeps the same manifolds throughout.
     if (!kPrestepped) {
+        if (kShared) CopyAsyncWait();  // each thread its own copies
         for (int j = tid; j < nm; j += T) {
             const int s = g.mBegin + j;
-            int2 r = t.refs[s];
+            const int2 r = kShared ? sRefs[j] : t.refs[s];
             // with islands, a pair between two inactive entries is not refreshed (NarrowPhase.cs:300-332)
             auto entryActive = [&](int ref) {
                 return ref >= 0 ? bv.pos[ref].w != 0.f : (ref <= -2 && b.act[-2 - ref].y <= 0.f);
             };
             if ((flags & BEPUGPU_STEP_REFRESH_CONTACTS) && (!b.islandOf || entryActive(r.x) || entryActive(r.y)))
-                RefreshManifoldV(m, bv, s, r.x, r.y, p);
-            if (kShared) {
-                ml.penacc[j] = m.penacc[s];  // after the refresh, which may compact them
-                ml.fricacc[j] = m.fricacc[s];
-                sRefs[j] = r;
-            }
-            if (flags & BEPUGPU_STEP_SOLVE) PrestepManifoldIO(m, s, ml, lbase + j, bv, r.x, r.y, p);
+                RefreshManifoldIO(mi, ibase + j, m, bv, s, r.x, r.y, p);
+            if (flags & BEPUGPU_STEP_SOLVE) PrestepManifoldIO<kShared>(mi, ibase + j, ml, lbase + j, bv, r.x, r.y, p);
             if (kCensus) {
                 // Compulsory DRAM bytes of the step for this manifold.  Lanes in shared memory:
                 // head, refs, 3 input lanes per contact, material, axis and impulses read once,

@@ -398,19 +398,23 @@ __device__ __forceinline__ float3 QTransform(float vx, float vy, float vz, float
 // order-preserving removal of the contacts it queues.  Removed contacts lose
 // their accumulated impulse (ContactPenetrationConstraint.CleanUp, :65-75); a
 // manifold left empty clears sliding and twist (ConvexContactManifoldConstraint.cs:148-154).
+// A group kernel reads a staged copy of the manifold (mi at slot si) and
+// writes what the refresh changes to the copy and to the manifold (m at s);
+// the other paths pass the same arrays twice.
 template <class V>
-__device__ __forceinline__ void RefreshManifoldV(const ManifoldSoA& m, const V& bv, int s, int ra, int rb,
-                                                 const StepParams& p) {
-    int4 h = m.head[s];
+__device__ __forceinline__ void RefreshManifoldIO(const ManifoldSoA& mi, int si, const ManifoldSoA& m, const V& bv,
+                                                  int s, int ra, int rb, const StepParams& p) {
+    const bool staged = mi.head != m.head;
+    int4 h = mi.head[si];
     int count = h.z & 0xff;
     // narrow-phase manifolds (flag 4, BEPUGPU_MANIFOLD_GENERATED) are not refreshed
     if (count == 0 || ((h.z >> 8) & 4)) return;
-    int cap = m.capacity;
+    const int cap = m.capacity, capi = mi.capacity;
     float4 pa = make_float4(0, 0, 0, 0), qa = make_float4(0, 0, 0, 1);
     float4 pb = pa, qb = qa;
     if (ra != -1) { pa = bv.Pos(ra); qa = bv.Quat(ra); }
     if (rb != -1) { pb = bv.Pos(rb); qb = bv.Quat(rb); }
-    float4 acc = m.penacc[s];
+    float4 acc = mi.penacc[si];
     const float accs[4] = {acc.x, acc.y, acc.z, acc.w};
     // All contact loops are unrolled over the four lanes with a count guard so
     // per-contact values stay in registers.
@@ -420,9 +424,9 @@ __device__ __forceinline__ void RefreshManifoldV(const ManifoldSoA& m, const V& 
     for (int k = 0; k < 4; k++) {
         keep[k] = false;
         if (k < count) {
-            cn[k] = m.cnrm[k * cap + s];
-            oa[k] = m.offA[k * cap + s];
-            ob[k] = m.offB[k * cap + s];
+            cn[k] = mi.cnrm[k * capi + si];
+            oa[k] = mi.offA[k * capi + si];
+            ob[k] = mi.offB[k * capi + si];
             float3 ta = QTransform(oa[k].x, oa[k].y, oa[k].z, qa);
             float3 tb = QTransform(ob[k].x, ob[k].y, ob[k].z, qb);
             float ax = ta.x + pa.x, ay = ta.y + pa.y, az = ta.z + pa.z;  // RigidTransform.Transform
@@ -450,7 +454,9 @@ __device__ __forceinline__ void RefreshManifoldV(const ManifoldSoA& m, const V& 
     for (int k = 0; k < 4; k++) {
         if (!keep[k]) continue;
         m.cpos[kept * cap + s] = cp[k];
+        if (staged) mi.cpos[kept * capi + si] = cp[k];
         if (kept != k) {
+            if (staged) mi.cnrm[kept * capi + si] = cn[k];  // the prestep reads no offsets
             m.cnrm[kept * cap + s] = cn[k];
             m.offA[kept * cap + s] = oa[k];
             m.offB[kept * cap + s] = ob[k];
@@ -465,9 +471,14 @@ __device__ __forceinline__ void RefreshManifoldV(const ManifoldSoA& m, const V& 
         m.penacc[s] = make_float4(n0, n1, n2, n3);
         h.z = (h.z & ~0xff) | kept;
         m.head[s] = h;
+        if (staged) {
+            mi.penacc[si] = make_float4(n0, n1, n2, n3);
+            mi.head[si] = h;
+        }
         if (kept == 0) {
-            float4 f = m.fricacc[s];
+            float4 f = mi.fricacc[si];
             m.fricacc[s] = make_float4(0.f, 0.f, 0.f, f.w);
+            if (staged) mi.fricacc[si] = make_float4(0.f, 0.f, 0.f, f.w);
         }
         if (((uint32_t)h.z >> 8) & kManifoldNonConvex) {
             // NonConvexContactManifoldConstraint.RemoveContact (:139-166): each
@@ -478,12 +489,24 @@ __device__ __forceinline__ void RefreshManifoldV(const ManifoldSoA& m, const V& 
             for (int k = 0; k < 4; k++) {
                 if (k >= count) break;
                 if (!keep[k]) continue;
-                if (q != k) m.cfr[q * cap + s] = m.cfr[k * cap + s];
+                if (q != k) {
+                    const float4 fr = mi.cfr[k * capi + si];
+                    m.cfr[q * cap + s] = fr;
+                    if (staged) mi.cfr[q * capi + si] = fr;
+                }
                 q++;
             }
-            for (int k = kept; k < count; k++) m.cfr[k * cap + s] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = kept; k < count; k++) {
+                m.cfr[k * cap + s] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (staged) mi.cfr[k * capi + si] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
     }
+}
+template <class V>
+__device__ __forceinline__ void RefreshManifoldV(const ManifoldSoA& m, const V& bv, int s, int ra, int rb,
+                                                 const StepParams& p) {
+    RefreshManifoldIO(m, s, m, bv, s, ra, rb, p);
 }
 // An entry of the narrow phase is active (NarrowPhase.cs:300-332 updates a
 // pair while one of its entries is): a dynamic body while its island is
@@ -524,8 +547,10 @@ __device__ __forceinline__ void LoadPrestepBody(const V& bv, int r, PrestepBody&
 // Inputs (head, contacts, material, previous sliding axis) are read from
 // `mi` at slot `si`; products (Jacobians, friction lanes, state, head) are
 // written to `mo` at slot `so`.  The sweep path passes the same arrays twice;
-// a group kernel writes its products to shared memory.
-template <class V>
+// a group kernel writes its products to shared memory, over the staged inputs:
+// of contact k, cpos, cnrm and offsets are dead once pj0..pj2 of k are written
+// but for cpos, which lies under lanes written after its last use.
+template <bool kStaged = false, class V>
 __device__ __forceinline__ void PrestepManifoldIO(const ManifoldSoA& mi, int si, const ManifoldSoA& mo, int so,
                                                   const V& bv, int ra, int rb, const StepParams& p) {
     int4 h = mi.head[si];
@@ -541,6 +566,12 @@ __device__ __forceinline__ void PrestepManifoldIO(const ManifoldSoA& mi, int si,
     // BEPUGPU_MANIFOLD_ACTIVE = 1, BEPUGPU_MANIFOLD_SOLVER_RULE = 2
     bool groupActive = (mflags & 1u) && (mflags & 2u) && ((hasA && A.dynamic) || (hasB && B.dynamic));
     const bool nonConvex = mflags & kManifoldNonConvex;
+    // Contact k's normal once pj0 of k is written (over the staged one): its
+    // negated linear jacobian.
+    auto normalOf = [&](int k) {
+        const float4 n = kStaged ? mo.pj0[k * capo + so] : mi.cnrm[k * cap + si];
+        return kStaged ? make_float3(-n.x, -n.y, -n.z) : make_float3(n.x, n.y, n.z);
+    };
     // A manifold the sliding update skips keeps its axis, a NONCONVEX one its
     // contacts' friction state; lanes staged in shared memory must carry them
     // too (they are written back whole).
@@ -648,7 +679,8 @@ __device__ __forceinline__ void PrestepManifoldIO(const ManifoldSoA& mi, int si,
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             if (k >= count) break;
-            const float4 cp = mi.cpos[k * cap + si], cn = mi.cnrm[k * cap + si];
+            const float4 cp = mi.cpos[k * cap + si];
+            const float3 cn = normalOf(k);
             float4 fr = mi.cfr[k * cap + si];
             float rax = 0, ray = 0, raz = 0, rbx = 0, rby = 0, rbz = 0;  // the penetration child's ra, rb
             float vAx = 0, vAy = 0, vAz = 0, vBx = 0, vBy = 0, vBz = 0;
@@ -749,8 +781,8 @@ __device__ __forceinline__ void PrestepManifoldIO(const ManifoldSoA& mi, int si,
         vBx = vBx + B.vx; vBy = vBy + B.vy; vBz = vBz + B.vz;
     }
     float rvx = vAx - vBx, rvy = vAy - vBy, rvz = vAz - vBz;
-    float4 n0 = mi.cnrm[si];
-    float nx = n0.x, ny = n0.y, nz = n0.z;
+    const float3 n0 = normalOf(0);
+    const float nx = n0.x, ny = n0.y, nz = n0.z;
     float normalVelocityScalar = nx * rvx + ny * rvy + nz * rvz;
     rvx -= normalVelocityScalar * nx;
     rvy -= normalVelocityScalar * ny;

@@ -39,3 +39,32 @@ def test_iteration_counts(gpu_context, policy, minimum, maximum, iterations):
         errs, exact = p.compare()
         assert exact, errs
     p.close()
+
+
+@pytest.mark.parametrize("policy", [None, (0, 1024, 4096, 64, 0)], ids=["groups", "sweeps"])
+@pytest.mark.parametrize("spheres", [0.0, 0.4])
+def test_refresh_drops_contacts(gpu_context, policy, spheres):
+    """Bodies turned and pushed so that the refresh drops first, middle and last
+    contacts of a manifold: a group kernel compacts its staged copy and the
+    manifold, and the prestep reads the copy."""
+    b, m, _ = scenes.make_tower(260, seed=7, sphere_fraction=spheres)
+    b = b.copy()
+    rng = np.random.default_rng(4)
+    dyn = b["is_dynamic"] != 0
+    b["position"][dyn] += rng.uniform(-0.07, 0.07, (int(dyn.sum()), 3)).astype(np.float32)
+    q = b["orientation"]
+    q[dyn] += rng.normal(0, 0.06, (int(dyn.sum()), 4)).astype(np.float32)
+    q /= np.linalg.norm(q, axis=1, keepdims=True)
+    gpu_context.set_settings(default_settings())
+    p = Pair(gpu_context, b, m, group_policy=policy)
+    before = m["contact_count"]
+    for step in range(3):
+        p.step()
+        errs, exact = p.compare()
+        assert exact, errs
+        if step == 0:
+            after = p.gpu.download_constraints()[0]["contact_count"]
+            lost = before - after
+            assert ((lost > 0) & (after > 0)).sum() > 5 or spheres  # some manifolds keep a part
+            assert (lost > 0).sum() > 5
+    p.close()
