@@ -1132,7 +1132,7 @@ bepugpu_status Scene::BuildGraph(Context* ctx, const StepParams& p, uint32_t fla
     CK(cudaEventRecordWithFlags(evPhase[3], stream, cudaEventRecordExternal));
     if (flows) {
         int flowLaunches = 0;
-        bepugpu_status fs = LaunchFlow(ctx, this, p, flowWarm, &flowLaunches);
+        bepugpu_status fs = LaunchFlow(ctx, this, p, false, flowWarm, &flowLaunches);
         if (fs != BEPUGPU_OK) {
             cudaGraph_t dropped;
             cudaStreamEndCapture(stream, &dropped);

@@ -162,6 +162,11 @@ struct GroupPlan {
     bool groupJoints = false;  // some group holds joints
     bool nonConvexLanes = false;  // some group holds a NONCONVEX manifold: shared lanes have room for its friction
 };
+// The class of groups that keep their lanes in global memory, without joints,
+// when its largest group would not fit a CTA's shared memory whatever the
+// caller's budget: a one-scene step spreads those over the GPU, visit by visit
+// (flow.cu), instead of one CTA each.  Null: no such class.
+const GroupClass* FlowGroups(const GroupPlan& plan);
 // Shared memory a group may use: 96 bytes per body, plus 400 per manifold when
 // its solve lanes live there.
 constexpr size_t kGroupSmemBudget = 200 * 1024;
@@ -177,6 +182,8 @@ bepugpu_status LaunchGroups(Context* ctx, Scene* s, const StepParams& p, uint32_
 bool SplitGroupPrologue(const Scene* s, uint32_t flags);
 bepugpu_status LaunchPrestepped(Context* ctx, Scene* s, const StepParams& p, uint32_t flags, bool count,
                                 const GroupTables& t, int* launches);  // the groups' launches after it
+bepugpu_status LaunchFlowGroups(Context* ctx, Scene* s, const StepParams& p, uint32_t flags, const GroupTables& t,
+                                bool started, int* launches);
 // The split prologue's default: scenes whose groups hold joints and at least
 // this many constraints.  Measured on GB300, in-kernel against split: chains
 // of 16 capsules step in 98 and 82 us at 417 constraints, 112 and 100 us at
@@ -197,10 +204,12 @@ struct FlowTables {
     float4 *lin, *ang;        // per body: velocity, w = visits so far (bits)
     int* error;
     int chunkCount;
+    int groupChunkCount;      // chunks after those: the slots of FlowGroups
 };
-// The solve sweeps of the slots outside groups, after their prestep and, with
-// `warm`, their warm start: two launches.
-bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool warm, int* launches);
+// The solve sweeps of the slots outside groups, or (groups) of the island
+// groups that FlowGroups names, after their prestep and, with `warm`, their
+// warm start: two launches.
+bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool groups, bool warm, int* launches);
 // Scenes of more chunks than this (four for each of the 8 warps a GB300 SM
 // holds of k_flow) warm-start in a launch per colour, whose smaller kernel
 // keeps more loads in flight.  Measured in a step, in the flow launch against
@@ -347,7 +356,7 @@ struct Scene {
     // flow.cu: the tables from the constraint upload's records (bodies a, b
     // per manifold record), or from update_pairs' sorted (body, entry) keys.
     bepugpu_status UploadFlow(Context* ctx, const int32_t* a, const int32_t* b);
-    bepugpu_status UploadFlowChunks(Context* ctx);
+    bepugpu_status UploadFlowChunks(Context* ctx, const std::vector<int2>& groupChunks);
     bepugpu_status BuildFlowOnDevice(Context* ctx, const unsigned long long* entries, int count, const int2* ends,
                                      const int* slots);
     int SweepColours() const { return manifoldOffsets.empty() ? 0 : (int)manifoldOffsets.size() - 1; }

@@ -1,5 +1,6 @@
 // Colour sweeps without barriers: the warm start and the solve sweeps of the
-// manifolds outside island groups, ordered visit by visit.
+// manifolds outside island groups, and of islands too large for one CTA's
+// shared memory, ordered visit by visit.
 //
 // The colour-ordered Gauss-Seidel sequence only orders two visits when they
 // share a dynamic body.  A launch (or a grid barrier) per colour orders all of
@@ -35,6 +36,7 @@
 
 #include "../../include/bepugpu.h"
 #include "bepugpu_internal.h"
+#include "groups_device.cuh"
 #include "solver_device.cuh"
 
 namespace bepugpu {
@@ -107,9 +109,12 @@ struct FlowEnd {
 // After the prestep: numbers each body's manifolds that have anything to
 // solve (a manifold without an active child leaves its bodies as they are in
 // every sweep) in slot order, and gives the body's first one the turn.
-__global__ void k_flow_order(ManifoldSoA m, BodySoA b, FlowTables f, unsigned first, unsigned sweeps) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= b.count) return;
+// list (null: every body): the n bodies to number.
+__global__ void k_flow_order(ManifoldSoA m, BodySoA b, FlowTables f, const int32_t* __restrict__ list, int bodies,
+                             unsigned first, unsigned sweeps) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= bodies) return;
+    const int i = list ? list[q] : q;
     const int begin = f.csrBegin[i], end = f.csrBegin[i + 1];
     unsigned n = 0;
     for (int k = begin; k < end; k++) {
@@ -283,38 +288,64 @@ std::vector<int2> FlowChunks(const std::vector<int32_t>& colourOffsets) {
         }                                                                                     \
     } while (0)
 
+const GroupClass* FlowGroups(const GroupPlan& plan) {
+    const GroupClass& c = plan.global;
+    const bool large = c.end > c.begin &&
+                       GroupSmemBytes(true, c.maxLocal, c.maxManifolds, 0, plan.nonConvexLanes) > kGroupSmemBudget;
+    return large ? &c : nullptr;
+}
+
 bepugpu_status Scene::UploadFlow(Context* ctx, const int32_t* a, const int32_t* b) {
+    // slots [0, n) and [g0, g1)
     const int n = groupPlan.globalCount;
-    flow.chunkCount = 0;
-    if (n == 0) return BEPUGPU_OK;
-    std::vector<int32_t> recordOf(n, -1);
-    for (size_t i = 0; i < groupPlan.slotOf.size(); i++)
-        if (groupPlan.slotOf[i] < n) recordOf[groupPlan.slotOf[i]] = (int32_t)i;
+    const GroupClass* large = FlowGroups(groupPlan);
+    const int g0 = large ? groupPlan.groups[large->begin].mBegin : n, g1 = large ? groupPlan.groups[large->end - 1].mEnd : n;
+    flow.chunkCount = flow.groupChunkCount = 0;
+    if (n == 0 && g1 == g0) return BEPUGPU_OK;
+    std::vector<int32_t> recordOf(groupPlan.slotOf.size(), -1);
+    for (size_t i = 0; i < groupPlan.slotOf.size(); i++) recordOf[groupPlan.slotOf[i]] = (int32_t)i;
     const int nb = this->b.count;
     std::vector<int32_t> begin(nb + 1, 0);
     auto moving = [&](int32_t e) { return e >= 0 && hostDynamic[e]; };
-    for (int s = 0; s < n; s++) {
-        if (moving(a[recordOf[s]])) begin[a[recordOf[s]] + 1]++;
-        if (moving(b[recordOf[s]])) begin[b[recordOf[s]] + 1]++;
-    }
+    auto slots = [&](auto visit) {
+        for (int s = 0; s < n; s++) visit(s, a[recordOf[s]], b[recordOf[s]]);
+        for (int s = g0; s < g1; s++) visit(s, a[recordOf[s]], b[recordOf[s]]);
+    };
+    slots([&](int, int32_t x, int32_t y) {
+        if (moving(x)) begin[x + 1]++;
+        if (moving(y)) begin[y + 1]++;
+    });
     for (int i = 0; i < nb; i++) begin[i + 1] += begin[i];
     std::vector<int32_t> at(begin.begin(), begin.end() - 1), csr(begin[nb]);
-    for (int s = 0; s < n; s++) {
-        if (moving(a[recordOf[s]])) csr[at[a[recordOf[s]]]++] = s << 1;
-        if (moving(b[recordOf[s]])) csr[at[b[recordOf[s]]]++] = (s << 1) | 1;
+    slots([&](int s, int32_t x, int32_t y) {
+        if (moving(x)) csr[at[x]++] = s << 1;
+        if (moving(y)) csr[at[y]++] = (s << 1) | 1;
+    });
+    CK(cudaMemcpyAsync(flow.csrBegin, begin.data(), sizeof(int32_t) * begin.size(), cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(flow.csr, csr.data(), sizeof(int32_t) * csr.size(), cudaMemcpyHostToDevice, stream));
+    // the groups' chunks colour by colour over all of them
+    std::vector<int2> groupChunks;
+    for (int c = 0; large; c++) {
+        bool any = false;
+        for (int k = large->begin; k < large->end; k++) {
+            const GroupDesc& g = groupPlan.groups[k];
+            if (c >= g.cCount) continue;
+            any = true;
+            const int32_t* off = groupPlan.colourOffsets.data() + g.cBegin;
+            for (int32_t s = off[c]; s < off[c + 1]; s += 32)
+                groupChunks.push_back(make_int2(g.mBegin + s, g.mBegin + std::min(s + 32, off[c + 1])));
+        }
+        if (!any) break;
     }
-    CK(cudaMemcpyAsync(flow.csrBegin, begin.data(), sizeof(int32_t) * begin.size(),
-                       cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(flow.csr, csr.data(), sizeof(int32_t) * csr.size(),
-                       cudaMemcpyHostToDevice, stream));
-    return UploadFlowChunks(ctx);
+    return UploadFlowChunks(ctx, groupChunks);
 }
 
-bepugpu_status Scene::UploadFlowChunks(Context* ctx) {
-    const int n = groupPlan.globalCount;
-    const std::vector<int2> chunks = FlowChunks(manifoldOffsets);
+bepugpu_status Scene::UploadFlowChunks(Context* ctx, const std::vector<int2>& groupChunks) {
+    std::vector<int2> chunks = FlowChunks(manifoldOffsets);
     flow.chunkCount = (int)chunks.size();
-    if (n == 0) return BEPUGPU_OK;
+    flow.groupChunkCount = (int)groupChunks.size();
+    chunks.insert(chunks.end(), groupChunks.begin(), groupChunks.end());
+    if (chunks.empty()) return BEPUGPU_OK;
     if (!ctx->flowError) {  // once a context, outside any stream capture
         CK(cudaHostAlloc((void**)&ctx->flowError, sizeof(int), cudaHostAllocMapped));
         *ctx->flowError = 0;
@@ -322,9 +353,8 @@ bepugpu_status Scene::UploadFlowChunks(Context* ctx) {
     }
     CK(cudaHostGetDevicePointer((void**)&flow.error, ctx->flowError, 0));
     // the ends without a dynamic body keep visit -1
-    CK(cudaMemsetAsync(flow.visit, 0xff, sizeof(int2) * n, stream));
-    CK(cudaMemcpyAsync(flow.chunks, chunks.data(), sizeof(int2) * chunks.size(),
-                       cudaMemcpyHostToDevice, stream));
+    CK(cudaMemsetAsync(flow.visit, 0xff, sizeof(int2) * groupPlan.slotOf.size(), stream));
+    CK(cudaMemcpyAsync(flow.chunks, chunks.data(), sizeof(int2) * chunks.size(), cudaMemcpyHostToDevice, stream));
     CK(cudaStreamSynchronize(stream));
     return BEPUGPU_OK;
 }
@@ -333,14 +363,23 @@ bepugpu_status Scene::BuildFlowOnDevice(Context* ctx, const unsigned long long* 
                                         const int* slots) {
     k_flow_csr<<<(count + 1 + 255) / 256, 256, 0, stream>>>(entries, count, b.count, ends, slots, flow);
     CK(cudaGetLastError());
-    return UploadFlowChunks(ctx);
+    return UploadFlowChunks(ctx, {});
 }
 
-bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool warm, int* launches) {
-    const FlowTables& f = s->flow;
-    const int nb = s->b.count;
+bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool groups, bool warm, int* launches) {
+    FlowTables f = s->flow;
+    const int32_t* list = nullptr;
+    int nb = s->b.count;
+    if (groups) {
+        const GroupPlan& plan = s->groupPlan;
+        const GroupDesc &first = plan.groups[plan.global.begin], &last = plan.groups[plan.global.end - 1];
+        list = s->groupBodiesDev + first.bBegin;
+        nb = last.bEnd - first.bBegin;
+        f.chunks += f.chunkCount;
+        f.chunkCount = f.groupChunkCount;
+    }
     const unsigned sweeps = (unsigned)p.iterationLimit + 1;
-    k_flow_order<<<(nb + 127) / 128, 128, 0, s->stream>>>(s->m, s->b, f, warm ? 0u : 1u, sweeps);
+    k_flow_order<<<(nb + 127) / 128, 128, 0, s->stream>>>(s->m, s->b, f, list, nb, warm ? 0u : 1u, sweeps);
     if (launches) (*launches)++;
     cudaLaunchConfig_t cfg = {};
     // a warp per chunk on its own CTA while the CTAs last

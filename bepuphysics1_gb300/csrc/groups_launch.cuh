@@ -75,7 +75,10 @@ bepugpu_status LaunchClasses(Context* ctx, Scene* s, const StepParams& p, uint32
                              int* launches) {
     const GroupPlan& g = s->groupPlan;
     bepugpu_status st = LaunchClass<true, 0, kPrestepped>(ctx, s, g.shared, p, flags, count, t, launches);
-    if (st == BEPUGPU_OK) st = LaunchClass<false, 0, kPrestepped>(ctx, s, g.global, p, flags, count, t, launches);
+    // (the census of an instrumented step counts the visits of the group kernel)
+    if (st == BEPUGPU_OK)
+        st = !count && FlowGroups(g) ? LaunchFlowGroups(ctx, s, p, flags, t, kPrestepped, launches)
+                                     : LaunchClass<false, 0, kPrestepped>(ctx, s, g.global, p, flags, count, t, launches);
     if (s->addedJointTypes) {
         if (st == BEPUGPU_OK)
             st = LaunchClass<true, 2, kPrestepped>(ctx, s, g.sharedJoints, p, flags, count, t, launches);

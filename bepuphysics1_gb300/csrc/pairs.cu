@@ -608,7 +608,7 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
         CK(cudaMemcpyAsync(plan.slotOf.data(), col.slotOf, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
     }
     s->manifoldOffsets = col.offsets;
-    s->flow.chunkCount = 0;
+    s->flow.chunkCount = s->flow.groupChunkCount = 0;
     if (n) {
         bepugpu_status fs = s->BuildFlowOnDevice(ctx, col.entries, 2 * n, rec.ends, col.slotOf);
         if (fs != BEPUGPU_OK) return fs;

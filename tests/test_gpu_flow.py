@@ -63,3 +63,36 @@ def test_manifolds_without_work(gpu_context):
     s = default_settings()
     s["minimum_impulse"] = 0.05
     _run(gpu_context, b, m, s, steps=5)
+
+
+def _together(*parts):
+    """Scenes side by side: bodies and manifolds concatenated."""
+    bodies, manifolds, at, x = [], [], 0, 0.0
+    for b, m in parts:
+        b, m = b.copy(), m.copy()
+        b["position"][:, 0] += x
+        m["contacts"]["position"][..., 0] += x
+        x += 300.0
+        for end in ("body_a", "body_b"):
+            m[end] += np.where(m[end] >= 0, at, 0).astype(np.int32)
+        at += len(b)
+        bodies.append(b)
+        manifolds.append(m)
+    return np.concatenate(bodies), np.concatenate(manifolds)
+
+
+@pytest.mark.parametrize("policy", [None, (1, 400, 4096, 64, 0)], ids=["groups", "groups_and_sweeps"])
+@pytest.mark.parametrize("flags", [N.STEP_ALL, N.STEP_FORCES | N.STEP_SOLVE, N.STEP_POSITIONS])
+def test_large_islands_beside_small_ones(gpu_context, policy, flags):
+    """Islands past a CTA's shared memory (stepped by grid-wide launches), small
+    islands in group CTAs and, with 400 bodies a group, sweep islands at once."""
+    b, m = _together(_pile(7, 7, 7), scenes.make_tower(150, seed=2)[:2], _pile(8, 6, 9, seed=8))
+    b["linear_velocity"][1:40, 1] = -0.5
+    s = default_settings()
+    p = Pair(gpu_context, b, m, settings=s, group_policy=policy)
+    for _ in range(4):
+        p.step(flags=flags)
+        errs, exact = p.compare()
+        assert exact, errs
+        assert errs["position"] == 0 and errs["orientation"] == 0
+    p.close()
