@@ -710,6 +710,9 @@ Scene::~Scene() {
         if (e) cudaEventDestroy(e);
     for (auto e : evGroup)
         if (e) cudaEventDestroy(e);
+    for (auto e : evSide)
+        if (e) cudaEventDestroy(e);
+    if (sideStream) cudaStreamDestroy(sideStream);
     ReleaseBroadPhase(this);
     ReleaseIslands(this);
     ReleasePairs(this);

@@ -186,13 +186,13 @@ bepugpu_status LaunchFlowGroups(Context* ctx, Scene* s, const StepParams& p, uin
                                 bool started, int* launches);
 // The split prologue's default: scenes whose groups hold joints and at least
 // this many constraints.  Measured on GB300, in-kernel against split: chains
-// of 16 capsules step in 98 and 82 us at 417 constraints, 112 and 100 us at
-// 1,671, 121 and 106 us at 8,347; with the added joint types 217 and 186 us at
-// 1,671.  Smaller scenes gain too, but keep the step at one launch per kind of
-// group.  Contact-only groups (the 65,536-box pile, towers) are 7-13 % slower
-// split, the group CTA's own pass over its bodies and manifolds being cheaper
-// there than two more launches and the copy of the solve lanes.
-constexpr int32_t kSplitPrologueConstraints = 1024;
+// of 16 capsules step in 70 and 80 us at 4,169 constraints, 85 and 85 us at
+// 8,347, 89 and 86 us at 16,663; with the added joint types 111 and 115 us at
+// 8,347, 139 and 132 us at 10,200, 132 and 120 us at 16,663.  Below the line every group is resident with
+// several warps, whose own prestep is cheaper than two launches and the copy
+// of the lanes.  Contact-only groups (the 65,536-box pile, towers) are 7-13 %
+// slower split at any size.
+constexpr int32_t kSplitPrologueConstraints = 8192;
 // The barrier-free sweeps' tables (flow.cu), for the manifold slots outside
 // island groups.
 struct FlowTables {
@@ -344,6 +344,10 @@ struct Scene {
     bool planStale = false;          // dynamic flags changed since the constraints were planned
     uint64_t batchStamp = 0;         // last batched call listing the scene (duplicate check)
     cudaEvent_t evGroup[2] = {nullptr, nullptr};
+    // Groups with joints run beside the others (LaunchClasses): created at the
+    // upload of constraints that make both kinds.
+    cudaStream_t sideStream = nullptr;
+    cudaEvent_t evSide[2] = {nullptr, nullptr};
     bepugpu_status UploadGroups(Context* ctx);
     bepugpu_status RebuildSweepBodies(Context* ctx);
     // The colour-sweep part of the manifold list: slots [0, globalCount).

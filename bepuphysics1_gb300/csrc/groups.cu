@@ -304,7 +304,15 @@ bepugpu_status Scene::UploadGroups(Context* ctx) {
     const GroupPlan& g = groupPlan;
     size_t G = g.groups.size();
     if (G == 0) return BEPUGPU_OK;
-    cudaError_t e;
+    cudaError_t e = cudaSuccess;
+    const bool contacts = g.shared.end > g.shared.begin || g.global.end > g.global.begin;
+    if (g.groupJoints && contacts && !sideStream &&
+        ((e = cudaStreamCreateWithFlags(&sideStream, cudaStreamNonBlocking)) ||
+         (e = cudaEventCreateWithFlags(&evSide[0], cudaEventDisableTiming)) ||
+         (e = cudaEventCreateWithFlags(&evSide[1], cudaEventDisableTiming)))) {
+        ctx->SetError("group side stream: %s", cudaGetErrorString(e));
+        return BEPUGPU_CUDA_ERROR;
+    }
     if ((e = cudaMemcpyAsync(groupDescDev, g.groups.data(), sizeof(GroupDesc) * G, cudaMemcpyHostToDevice, stream)) ||
         (e = cudaMemcpyAsync(groupBodiesDev, g.groupBodies.data(), sizeof(int32_t) * g.groupBodies.size(),
                              cudaMemcpyHostToDevice, stream)) ||

@@ -313,9 +313,15 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
     if (flags & BEPUGPU_STEP_SOLVE) {
         const int* co = t.colourOffsets + g.cBegin;
         const int* jco = kJoints ? t.jointColourOffsets + g.jcBegin : nullptr;
+        // A colour's joints in one contiguous part per warp: they are sorted by
+        // type, so the warps run different types side by side.
+        const int warps = T >> 5, warp = tid >> 5;
+        auto jointPart = [&](int c) { return (jco[c + 1] - jco[c] + warps - 1) / warps; };
+        auto jointFirst = [&](int c) { return jco[c] + warp * jointPart(c) + (tid & 31); };
+        auto jointEnd = [&](int c) { return min(jco[c + 1], jco[c] + (warp + 1) * jointPart(c)); };
         for (int c = 0; c < g.cCount; c++) {
             if (kJoints)
-                for (int q = jco[c] + tid; q < jco[c + 1]; q += T) {
+                for (int q = jointFirst(c), end = jointEnd(c); q < end; q += 32) {
                     const uint2 st = jl.state[q];
                     if (!(st.x & kGroupActive)) continue;
                     const int2 r = jRefs[q];
@@ -341,7 +347,7 @@ __device__ __forceinline__ void GroupStep(const ManifoldSoA& m, const BodySoA& b
         for (int it = 0; it < p.iterationLimit; it++)
             for (int c = 0; c < g.cCount; c++) {
                 if (kJoints)
-                    for (int q = jco[c] + tid; q < jco[c + 1]; q += T) {
+                    for (int q = jointFirst(c), end = jointEnd(c); q < end; q += 32) {
                         uint2 st = jl.state[q];
                         if (!(st.x & kGroupActive)) continue;
                         const int2 r = jRefs[q];

@@ -642,7 +642,7 @@ bepugpu_status bepugpu_set_group_smem_budget(bepugpu_context* ctx, int32_t scene
  * and joints' prestep): 0 inside the group kernel, each CTA over its own group; 1 as two
  * grid-wide launches before it, one thread per manifold, joint or body, the group
  * kernel then copying the solve lanes into shared memory; -1 (default) the
- * grid-wide launches when the groups hold joints and at least 1,024
+ * grid-wide launches when the groups hold joints and at least 8,192
  * constraints.  The results are the same bit for bit.  Takes effect at the
  * next step.  No reference counterpart: it only chooses how the GPU runs the
  * stages of Space.cs:496-513. */
