@@ -196,7 +196,7 @@ constexpr int32_t kSplitPrologueConstraints = 8192;
 // The barrier-free sweeps' tables (flow.cu), for the manifold slots outside
 // island groups.
 struct FlowTables {
-    int2* chunks;             // slots [x, y) of one colour, at most 32, colour-major
+    int2* chunks;             // slots [x, y) of one colour, at most 16, colour-major
     int2* visit;              // per slot: its place among its bodies A's and B's visits of a sweep, -1 none
     int32_t* degree;          // per body: visits of a sweep
     int32_t* csrBegin;        // per body: its entries of csr, bodies + 1
@@ -210,13 +210,15 @@ struct FlowTables {
 // groups that FlowGroups names, after their prestep and, with `warm`, their
 // warm start: two launches.
 bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool groups, bool warm, int* launches);
-// Scenes of more chunks than this (four for each of the 8 warps a GB300 SM
-// holds of k_flow) warm-start in a launch per colour, whose smaller kernel
-// keeps more loads in flight.  Measured in a step, in the flow launch against
-// per colour: 82,000 manifolds 7.8 and 8.0 ms (four frames of a settling heap
-// of 16 colours), 188,667 manifolds 325 and 332 us, 425,999 754 and 744 us,
-// 757,861 1,388 and 1,354 us.
-constexpr int kFlowWarmChunks = 4864;
+// Scenes of more chunks than this (four for each of the 16 warps a GB300 SM
+// holds of k_flow) warm-start in a launch per colour.  Such a step has more
+// launches than colours, as callers of bepugpu_last_step_launches know the
+// sweep path (a test of the packed 65,536-box pile holds it to that).  A step
+// with the warm start in the flow launch against per colour: 188,667 manifolds
+// 285 and 305 us, 425,999 650 and 657 us, 757,861 1,190 and 1,178 us; in
+// smaller scenes the colours' launches cost more (82,000 manifolds of 16
+// colours: 45 us a step).
+constexpr int kFlowWarmChunks = 9728;
 // TIMEOUT when a wait of a finished flow launch ran out (and clears it).
 bepugpu_status FlowStatus(Context* ctx);
 // Joints (joints.cu): record checks, upload into the scene's joint slots, and

@@ -24,7 +24,7 @@
 // and no fence is needed.  Everything else a visit writes (impulses, state) is
 // read again only by the same thread, or after the launch.
 //
-// Progress: a warp takes its 32-slot chunks of one colour in sweep-major,
+// Progress: a warp takes its 16-slot chunks of one colour in sweep-major,
 // colour-major order, and the launch is cooperative, so every warp is
 // resident; the earliest unfinished chunk never waits for a later one.  A
 // wait that sees no tag change for kFlowSpinLimit polls reports a timeout
@@ -44,6 +44,7 @@ namespace bepugpu {
 namespace {
 
 constexpr int kFlowThreads = 128;
+constexpr int kFlowChunk = 16;  // manifolds a warp visits at once, two lanes each
 constexpr int kFlowSpinLimit = 1 << 21;
 
 // A body's word: its velocity and its tag.
@@ -132,82 +133,285 @@ __global__ void k_flow_order(ManifoldSoA m, BodySoA b, FlowTables f, const int32
     f.ang[i] = make_float4(w.x, w.y, w.z, __uint_as_float(tag));
 }
 
+// One end's share of a manifold's visit.  Lanes 2 i and 2 i + 1 of a warp run
+// one visit: the even lane holds body A, the odd one body B.  Each computes
+// its body's half of every relative velocity and applies its body's half of
+// every impulse; the halves meet in one shuffle, and both lanes then run the
+// same child arithmetic on the same values (the sums commute, and a sign
+// multiplies exactly, so every bit is SolveManifold's).  A visit is one chain
+// of dependent operations, so half the instructions in it is what shortens a
+// turn; the lanes' loads halve with them.
+struct HalfLanes {
+    float4 j0[4];       // linear jacobian of this end (B: A's negated), w = bias
+    float4 j[4];        // angular jacobian, w = softness
+    float v2i[4];
+    float4 r, l1, l2;   // sliding: signed arm, w = friction; rows of linear A, w = M12, M21
+    float4 row1, row2;  // angular rows, w = M22, twist velocityToImpulse
+    float4 n, lev;      // twist: axis, w = friction; lever arms
+    float m11;
+    float4 acc, f;      // accumulated impulses
+};
+__device__ __forceinline__ float OfA(float own, bool second) {  // lane A's value, in both lanes
+    const float other = __shfl_xor_sync(0xffffffffu, own, 1);
+    return second ? other : own;
+}
+__device__ __forceinline__ float OfB(float own, bool second) {
+    const float other = __shfl_xor_sync(0xffffffffu, own, 1);
+    return second ? own : other;
+}
+__device__ __forceinline__ float4 Signed(float4 v, float sign) {
+    return make_float4(sign * v.x, sign * v.y, sign * v.z, v.w);
+}
+// Every lane of the warp calls it (shuffles); a manifold's two lanes pass the
+// same st and children.
+__device__ __forceinline__ void LoadHalf(const ManifoldSoA& m, int s, uint32_t st, uint32_t children, bool second,
+                                         HalfLanes& H) {
+    const int cap = m.capacity;
+    const float sign = second ? -1.f : 1.f;
+    const bool friction = !(st & kContactFriction);
+    const bool sliding = friction && ChildOn(children, kSlidingChild), twist = friction && ChildOn(children, kTwistChild);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (children != ~0u) {
+        H.acc = m.penacc[s];
+        H.f = m.fricacc[s];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const bool on = ChildOn(children, k);
+        H.j0[k] = H.j[k] = zero;
+        if (on || (k == 0 && twist)) H.j0[k] = m.pj0[k * cap + s];
+        if (on) H.j[k] = (second ? m.pj2 : m.pj1)[k * cap + s];
+    }
+    H.r = H.row1 = H.row2 = zero;
+    if (sliding) {
+        H.r = (second ? m.s1 : m.s0)[s];
+        H.l1 = m.saxis[s];
+        H.l2 = m.s3[s];
+    }
+    if (sliding || twist) {
+        H.row1 = (second ? m.s6 : m.s4)[s];
+        H.row2 = (second ? m.s7 : m.s5)[s];
+    }
+    if (twist) H.lev = m.lever[s];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float w = H.j[k].w;  // A: softness, B: velocityToImpulse
+        H.v2i[k] = OfB(w, second);
+        H.j[k].w = OfA(w, second);
+    }
+    H.n = make_float4(-H.j0[0].x, -H.j0[0].y, -H.j0[0].z, OfB(H.row1.w, second));
+    H.row1.w = OfA(H.row1.w, second);
+    H.row2.w = OfA(H.row2.w, second);
+    H.m11 = OfB(H.r.w, second);
+    H.r.w = OfA(H.r.w, second);
+    H.r = Signed(H.r, sign);
+#pragma unroll
+    for (int k = 0; k < 4; k++) H.j0[k] = Signed(H.j0[k], sign);
+}
+__device__ __forceinline__ void ApplyHalf(BodyState& b, float impulse, float4 linear, float4 angular) {
+    ApplyLinear(b, impulse * linear.x, impulse * linear.y, impulse * linear.z);
+    ApplyAngular(b, impulse * angular.x, impulse * angular.y, impulse * angular.z);
+}
+__device__ __forceinline__ float VelocityHalf(const BodyState& b, float4 linear, float4 angular) {
+    return b.vx * linear.x + b.vy * linear.y + b.vz * linear.z + b.wx * angular.x + b.wy * angular.y + b.wz * angular.z;
+}
+// WarmStartManifold for one end.
+__device__ __forceinline__ void WarmHalf(const ManifoldSoA& m, int s, BodyState& b, uint2 state, bool second,
+                                         const HalfLanes& H) {
+    const int cap = m.capacity;
+    const float sign = second ? -1.f : 1.f;
+    const float accs[4] = {H.acc.x, H.acc.y, H.acc.z, H.acc.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (ChildOn(state.y, k)) ApplyHalf(b, accs[k], H.j0[k], H.j[k]);
+    if (state.x & kContactFriction) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (!ChildOn(state.y, 4 + k)) continue;
+            const float4 fr = m.cfr[k * cap + s];
+            ApplyHalf(b, fr.w, Signed(fr, sign), (second ? m.cfb : m.cfa)[k * cap + s]);
+        }
+        return;
+    }
+    if (!ChildOn(state.y, kSlidingChild)) return;  // no contacts
+    const float ax = H.f.x, ay = H.f.y;
+    ApplyLinear(b, sign * (ax * H.l1.x + ay * H.l2.x), sign * (ax * H.l1.y + ay * H.l2.y),
+                sign * (ax * H.l1.z + ay * H.l2.z));
+    ApplyAngular(b, ax * H.row1.x + ay * H.row2.x, ax * H.row1.y + ay * H.row2.y, ax * H.row1.z + ay * H.row2.z);
+    ApplyAngular(b, sign * (H.f.z * H.n.x), sign * (H.f.z * H.n.y), sign * (H.f.z * H.n.z));
+}
+// The warp's lanes whose visit solves a child (both lanes of a visit), for the
+// shuffles inside SolveHalf: penetration 0..3, contact friction 0..3, sliding
+// and twist apart, since a warp may hold NONCONVEX manifolds beside convex ones.
+struct ChildLanes {
+    unsigned penetration[4], friction[4], sliding, twist;
+};
+__device__ __forceinline__ ChildLanes LanesOf(uint32_t st, uint32_t children) {
+    ChildLanes c;
+    const bool nonConvex = st & kContactFriction;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        c.penetration[k] = __ballot_sync(0xffffffffu, ChildOn(children, k));
+        c.friction[k] = __ballot_sync(0xffffffffu, nonConvex && ChildOn(children, 4 + k));
+    }
+    c.sliding = __ballot_sync(0xffffffffu, !nonConvex && ChildOn(children, kSlidingChild));
+    c.twist = __ballot_sync(0xffffffffu, !nonConvex && ChildOn(children, kTwistChild));
+    return c;
+}
+// SolveManifold for one end.
+__device__ __forceinline__ void SolveHalf(const ManifoldSoA& m, int s, BodyState& b, uint2& state, bool second,
+                                          const StepParams& p, const HalfLanes& H, const ChildLanes& lanes) {
+    const int cap = m.capacity;
+    const float sign = second ? -1.f : 1.f;
+    uint32_t st = state.x, children = state.y;
+    const uint32_t iter = (st >> kIterShift) + 1;
+    st = (st & 0xffffu) | (iter << kIterShift);
+    const uint32_t on = children;
+    uint32_t still = 0;
+    auto account = [&](int c, float r) { still |= r < p.minimumImpulse ? 1u << (4 * c) : 0u; };
+    auto both = [](unsigned lanesOn, float own) { return own + __shfl_xor_sync(lanesOn, own, 1); };
+    float accs[4] = {H.acc.x, H.acc.y, H.acc.z, H.acc.w};
+    float4 f = H.f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (!ChildOn(on, k)) continue;
+        const float rv = both(lanes.penetration[k], VelocityHalf(b, H.j0[k], H.j[k]));
+        float lambda = (rv - H.j0[k].w + H.j[k].w * accs[k]) * H.v2i[k];
+        const float prev = accs[k];
+        accs[k] = Maxf(0, accs[k] + lambda);
+        lambda = accs[k] - prev;
+        ApplyHalf(b, lambda, H.j0[k], H.j[k]);
+        account(k, fabsf(lambda));
+    }
+    if (st & kContactFriction) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (!ChildOn(on, 4 + k)) continue;
+            float4 fr = m.cfr[k * cap + s];
+            const float4 fa = m.cfa[k * cap + s], fb = m.cfb[k * cap + s];
+            const float4 own = second ? fb : fa, linear = Signed(fr, sign);
+            float lambda = both(lanes.friction[k], VelocityHalf(b, linear, own)) * fa.w;
+            const float prev = fr.w, maxForce = fb.w * accs[k];
+            fr.w = Clampf(fr.w + lambda, -maxForce, maxForce);
+            lambda = fr.w - prev;
+            ApplyHalf(b, lambda, linear, own);
+            account(4 + k, fabsf(lambda));
+            m.cfr[k * cap + s] = fr;  // by both lanes, the same value
+        }
+    } else {
+        if (ChildOn(on, kSlidingChild)) {
+            const float dvx = both(lanes.sliding, sign * b.vx + (b.wy * H.r.z) - (b.wz * H.r.y));
+            const float dvy = both(lanes.sliding, sign * b.vy + (b.wz * H.r.x) - (b.wx * H.r.z));
+            const float dvz = both(lanes.sliding, sign * b.vz + (b.wx * H.r.y) - (b.wy * H.r.x));
+            float lxv = dvx * H.l1.x + dvy * H.l1.y + dvz * H.l1.z;
+            float lyv = dvx * H.l2.x + dvy * H.l2.y + dvz * H.l2.z;
+            const float x = lxv;
+            lxv = x * H.m11 + lyv * H.l2.w;       // M11, M21
+            lyv = x * H.l1.w + lyv * H.row1.w;    // M12, M22
+            const float px = f.x, py = f.y;
+            f.x += lxv;
+            f.y += lyv;
+            float length = f.x * f.x + f.y * f.y;
+            float maximumFrictionForce = accs[0] + accs[1] + accs[2] + accs[3];
+            maximumFrictionForce *= H.r.w;
+            if (length > maximumFrictionForce * maximumFrictionForce) {
+                length = maximumFrictionForce / SqrtOfFloat(length);
+                f.x *= length;
+                f.y *= length;
+            }
+            lxv = f.x - px;
+            lyv = f.y - py;
+            ApplyLinear(b, sign * (lxv * H.l1.x + lyv * H.l2.x), sign * (lxv * H.l1.y + lyv * H.l2.y),
+                        sign * (lxv * H.l1.z + lyv * H.l2.z));
+            ApplyAngular(b, lxv * H.row1.x + lyv * H.row2.x, lxv * H.row1.y + lyv * H.row2.y,
+                         lxv * H.row1.z + lyv * H.row2.z);
+            account(kSlidingChild, fabsf(lxv) + fabsf(lyv));
+        }
+        if (ChildOn(on, kTwistChild)) {
+            // A's part minus B's, in both lanes
+            const float own = b.wx * H.n.x + b.wy * H.n.y + b.wz * H.n.z;
+            const float other = __shfl_xor_sync(lanes.twist, own, 1);
+            float lambda = ((second ? other : own) - (second ? own : other)) * H.row2.w;
+            const float prev = f.z;
+            float maximumFrictionForce =
+                H.lev.x * accs[0] + H.lev.y * accs[1] + H.lev.z * accs[2] + H.lev.w * accs[3];
+            maximumFrictionForce *= H.n.w;
+            f.z = Clampf(f.z + lambda, -maximumFrictionForce, maximumFrictionForce);
+            lambda = f.z - prev;
+            ApplyAngular(b, sign * (lambda * H.n.x), sign * (lambda * H.n.y), sign * (lambda * H.n.z));
+            account(kTwistChild, fabsf(lambda));
+        }
+    }
+    st = AccountChildren(st, children, still, p);
+    // both lanes write the same values, and read their own back in the next sweep
+    m.penacc[s] = make_float4(accs[0], accs[1], accs[2], accs[3]);
+    m.fricacc[s] = f;
+    state = make_uint2(st, children);
+}
+
 // Sweeps [first, sweeps); sweep 0 is the warm start.
-// Bound by the turns' latency in small scenes (a turn is a visit of about 1 us
-// plus one trip through L2) and by the lanes' trips through L2 in large ones
-// (76 MB a sweep at 188,667 manifolds).  180 registers, 8 warps an SM; held to
-// 168 for 12 warps it measured 11 % slower, at 32- or 64-thread CTAs the same.
-// A step of the packed piles, launches per colour against this kernel: 15,789
-// manifolds 228 -> 93 us, 188,667 manifolds 590 -> 332 us (without the sets of
-// active manifolds 175 and 390 us).
-__global__ void __launch_bounds__(kFlowThreads) k_flow(ManifoldSoA m, BodySoA b, StepParams p, FlowTables f,
+// Bound by the turns' latency in small and deep scenes (a visit and one trip
+// through L2 per turn) and by the lanes' trips through L2 in large ones (76 MB
+// a sweep at 188,667 manifolds).  128 registers, 16 warps an SM; 20 warps spill
+// and measured 11 % slower.  Against launches per colour and sweep: the frame
+// of a 5,750-box pile 307 -> 151 us, of a 1,000-box one (in one CTA before)
+// 225 -> 104 us, four frames of the settling 65,536-box heap 4.35 -> 3.98 ms
+// against one lane per manifold (8 warps an SM), the packed 65,536-box pile
+// four steps 2,890 -> 1,860 us (1,973 with one lane).
+__global__ void __launch_bounds__(kFlowThreads, 4) k_flow(ManifoldSoA m, BodySoA b, StepParams p, FlowTables f,
                                                        unsigned first, unsigned sweeps) {
     const int lane = threadIdx.x & 31;
+    const bool second = lane & 1;  // this lane's end: A, or B
     // consecutive chunks on different CTAs: a scene of few chunks spreads over the SMs
     const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, warps = gridDim.x * (kFlowThreads / 32);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     for (unsigned t = first; t < sweeps; t++)
         for (int c = warp; c < f.chunkCount; c += warps) {
             const int2 range = f.chunks[c];
-            const int s = range.x + lane;
+            const int s = range.x + (lane >> 1);
             const int2 visit = s < range.y ? f.visit[s] : make_int2(-1, -1);
-            uint2 state = make_uint2(0u, 0u);
-            if (visit.x >= 0 || visit.y >= 0) state = m.state[s];
+            const bool listed = visit.x >= 0 || visit.y >= 0;
+            uint2 state = listed ? m.state[s] : make_uint2(0u, ~0u);
             const bool active = state.x & kGroupActive;
-            int4 h = make_int4(-1, -1, 0, 0);
-            FlowEnd A, B;
-            A.v = A.w = B.v = B.w = zero;
-            A.degree = B.degree = 0;
-            if (visit.x >= 0 || visit.y >= 0) {
-                h = m.head[s];
-                if (visit.x >= 0) A.degree = (unsigned)f.degree[h.x];
-                if (visit.y >= 0) B.degree = (unsigned)f.degree[h.y];
-            }
-            A.masked = Masked(A.degree, sweeps);
-            B.masked = Masked(B.degree, sweeps);
+            // the visit's iteration past a limit only ends the manifold (Solver.cs:285-314)
+            const int iter = (int)(state.x >> kIterShift) + 1;
+            const bool runs = active && (t == 0 || (iter <= p.iterationLimit && iter <= p.maximumIterationCount));
+            const int4 h = listed ? m.head[s] : make_int4(-1, -1, 0, 0);
+            const int body = second ? h.y : h.x;
+            const bool dynamic = state.x & (second ? kDynB : kDynA);
+            FlowEnd E;
+            E.v = E.w = zero;
+            E.place = (unsigned)(second ? visit.y : visit.x);
+            const bool turns = listed && (int)E.place >= 0;
+            E.degree = turns ? (unsigned)f.degree[body] : 0u;
+            E.masked = Masked(E.degree, sweeps);
+            E.turn = t * E.degree + E.place;
             // a stopped manifold only takes its turn at bodies without a set
-            const bool atA = visit.x >= 0 && (active || !A.masked), atB = visit.y >= 0 && (active || !B.masked);
-            if (!__any_sync(0xffffffffu, atA || atB)) continue;
-            A.place = (unsigned)visit.x;
-            B.place = (unsigned)visit.y;
-            A.turn = t * A.degree + A.place;
-            B.turn = t * B.degree + B.place;
-            A.ready = !atA;
-            B.ready = !atB;
-            SolveLanes L;
-            float4 aa = zero, ca = zero, ab = zero, cb = zero;
-            float massA = 0.f, massB = 0.f, lastA = 0.f, lastB = 0.f;  // inverse mass, inertia M33
-            if (active) {
-                // everything that no other thread writes during the sweeps, before the wait
-                LoadSolveLanes(m, s, state.x, state.y, L);
-                if (visit.x < 0 && h.x >= 0) {
-                    A.v = b.vlin[h.x];
-                    A.w = b.vang[h.x];
-                }
-                if (visit.y < 0 && h.y >= 0) {
-                    B.v = b.vlin[h.y];
-                    B.w = b.vang[h.y];
-                }
-                if (state.x & kDynA) {
-                    aa = b.inv0[h.x];
-                    ca = b.inv1[h.x];
-                    massA = b.vlin[h.x].w;
-                    lastA = b.vang[h.x].w;
-                }
-                if (state.x & kDynB) {
-                    ab = b.inv0[h.y];
-                    cb = b.inv1[h.y];
-                    massB = b.vlin[h.y].w;
-                    lastB = b.vang[h.y].w;
-                }
+            const bool at = turns && (active || !E.masked);
+            if (!__any_sync(0xffffffffu, at)) continue;
+            E.ready = !at;
+            // everything that no other visit writes during the sweeps, before the wait
+            HalfLanes H;
+            const uint32_t children = runs ? state.y : ~0u;
+            LoadHalf(m, s, state.x, children, second, H);
+            const ChildLanes lanes = LanesOf(state.x, children);
+            float4 ia = zero, ic = zero;
+            float mass = 0.f, last = 0.f;  // inverse mass, inertia M33
+            if (runs && !turns && body >= 0) {
+                E.v = b.vlin[body];
+                E.w = b.vang[body];
+            }
+            if (runs && dynamic) {
+                ia = b.inv0[body];
+                ic = b.inv1[body];
+                mass = b.vlin[body].w;
+                last = b.vang[body].w;
             }
             unsigned seen = 0;
             for (int spins = 0;; spins++) {
-                if (!A.ready) A.Poll(f, h.x);
-                if (!B.ready) B.Poll(f, h.y);
-                if (__all_sync(0xffffffffu, A.ready && B.ready)) break;
-                const unsigned now = __float_as_uint(A.v.w) + __float_as_uint(A.w.w) + __float_as_uint(B.v.w) +
-                                     __float_as_uint(B.w.w);
+                if (!E.ready) E.Poll(f, body);
+                if (__all_sync(0xffffffffu, E.ready)) break;
+                const unsigned now = __float_as_uint(E.v.w) + __float_as_uint(E.w.w);
                 if (__any_sync(0xffffffffu, now != seen)) spins = 0;
                 seen = now;
                 if (spins > kFlowSpinLimit) {
@@ -215,35 +419,24 @@ __global__ void __launch_bounds__(kFlowThreads) k_flow(ManifoldSoA m, BodySoA b,
                     return;
                 }
             }
-            if (active) {
-                BodyState bodyA, bodyB;
-                MakeBody(make_float4(A.v.x, A.v.y, A.v.z, massA), make_float4(A.w.x, A.w.y, A.w.z, lastA), aa, ca, bodyA);
-                MakeBody(make_float4(B.v.x, B.v.y, B.v.z, massB), make_float4(B.w.x, B.w.y, B.w.z, lastB), ab, cb, bodyB);
-                if (t == 0) {
-                    WarmStartManifold(m, s, bodyA, bodyB, state, L);
-                } else {
-                    SolveManifold(m, s, bodyA, bodyB, state, p, &L);
-                    m.state[s] = state;
+            if (runs) {
+                BodyState own;
+                MakeBody(make_float4(E.v.x, E.v.y, E.v.z, mass), make_float4(E.w.x, E.w.y, E.w.z, last), ia, ic, own);
+                if (t == 0) WarmHalf(m, s, own, state, second, H);
+                else SolveHalf(m, s, own, state, second, p, H, lanes);
+                if (dynamic) {
+                    E.v.x = own.vx; E.v.y = own.vy; E.v.z = own.vz;
+                    E.w.x = own.wx; E.w.y = own.wy; E.w.z = own.wz;
                 }
-                if (state.x & kDynA) {
-                    A.v.x = bodyA.vx; A.v.y = bodyA.vy; A.v.z = bodyA.vz;
-                    A.w.x = bodyA.wx; A.w.y = bodyA.wy; A.w.z = bodyA.wz;
-                }
-                if (state.x & kDynB) {
-                    B.v.x = bodyB.vx; B.v.y = bodyB.vy; B.v.z = bodyB.vz;
-                    B.w.x = bodyB.wx; B.w.y = bodyB.wy; B.w.z = bodyB.wz;
-                }
+            } else if (active) {
+                state.x = ((state.x & 0xffffu) | ((uint32_t)iter << kIterShift)) & ~kGroupActive;
             }
-            const bool still = state.x & kGroupActive;  // active in the next sweep
             // the body's last visit leaves the velocity in the scene's lanes
-            if (atA && A.Pass(f, h.x, still, t, sweeps) && (state.x & kDynA)) {
-                b.vlin[h.x] = make_float4(A.v.x, A.v.y, A.v.z, b.vlin[h.x].w);
-                b.vang[h.x] = make_float4(A.w.x, A.w.y, A.w.z, b.vang[h.x].w);
+            if (at && E.Pass(f, body, state.x & kGroupActive, t, sweeps) && dynamic) {
+                b.vlin[body] = make_float4(E.v.x, E.v.y, E.v.z, b.vlin[body].w);
+                b.vang[body] = make_float4(E.w.x, E.w.y, E.w.z, b.vang[body].w);
             }
-            if (atB && B.Pass(f, h.y, still, t, sweeps) && (state.x & kDynB)) {
-                b.vlin[h.y] = make_float4(B.v.x, B.v.y, B.v.z, b.vlin[h.y].w);
-                b.vang[h.y] = make_float4(B.w.x, B.w.y, B.w.z, b.vang[h.y].w);
-            }
+            if (active && t > 0) m.state[s] = state;
         }
 }
 
@@ -274,8 +467,8 @@ __global__ void k_flow_csr(const unsigned long long* __restrict__ entries, int c
 std::vector<int2> FlowChunks(const std::vector<int32_t>& colourOffsets) {
     std::vector<int2> chunks;
     for (size_t c = 0; c + 1 < colourOffsets.size(); c++)
-        for (int32_t s = colourOffsets[c]; s < colourOffsets[c + 1]; s += 32)
-            chunks.push_back(make_int2(s, std::min(s + 32, colourOffsets[c + 1])));
+        for (int32_t s = colourOffsets[c]; s < colourOffsets[c + 1]; s += kFlowChunk)
+            chunks.push_back(make_int2(s, std::min(s + kFlowChunk, colourOffsets[c + 1])));
     return chunks;
 }
 
@@ -332,8 +525,8 @@ bepugpu_status Scene::UploadFlow(Context* ctx, const int32_t* a, const int32_t* 
             if (c >= g.cCount) continue;
             any = true;
             const int32_t* off = groupPlan.colourOffsets.data() + g.cBegin;
-            for (int32_t s = off[c]; s < off[c + 1]; s += 32)
-                groupChunks.push_back(make_int2(g.mBegin + s, g.mBegin + std::min(s + 32, off[c + 1])));
+            for (int32_t s = off[c]; s < off[c + 1]; s += kFlowChunk)
+                groupChunks.push_back(make_int2(g.mBegin + s, g.mBegin + std::min(s + kFlowChunk, off[c + 1])));
         }
         if (!any) break;
     }

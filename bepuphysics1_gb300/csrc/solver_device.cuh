@@ -1058,6 +1058,22 @@ __device__ __forceinline__ void WarmStartManifold(const ManifoldSoA& m, int s, B
     ApplyAngular(B, -gx, -gy, -gz);
 }
 
+// SolveUpdateable's bookkeeping (SolverGroup.cs:117-150) of a visit's children:
+// still marks those whose |impulse| was below the minimum by a one in their
+// nibble.  A still child's count goes up, a moving one's starts again, a
+// stopped one keeps its 15; a count that passes minimumIterationCount -- one
+// more than it, since the child was active -- becomes 15.  Returns the state's
+// word x.
+__device__ __forceinline__ uint32_t AccountChildren(uint32_t st, uint32_t& children, uint32_t still,
+                                                    const StepParams& p) {
+    const uint32_t off = children & (children >> 1) & (children >> 2) & (children >> 3) & 0x11111111u;
+    children = (children & (off * 15u)) | ((children & (still * 15u)) + still);
+    const uint32_t x = children ^ (still * ((uint32_t)p.minimumIterationCount + 1u));
+    const uint32_t stop = still & ~(x | (x >> 1) | (x >> 2) | (x >> 3));
+    children |= stop * 15u;
+    return children == ~0u ? st & ~kGroupActive : st;
+}
+
 // One solver visit of a manifold: Solver.UnsafeSolveIteration (Solver.cs:285-314)
 // -> ConvexContactManifoldConstraint.SolveIteration (:199-212) ->
 // SolverGroup.SolveUpdateable (SolverGroup.cs:117-150) on each child.
@@ -1091,10 +1107,7 @@ __device__ __forceinline__ void SolveManifold(const ManifoldSoA& m, int s, BodyS
     else LoadSolveLanes(m, s, st, children, Lv);
     float4 f = m.fricacc[s];
     const uint32_t on = children;  // the children this visit solves
-    // SolveUpdateable's bookkeeping (SolverGroup.cs:117-150): a child whose
-    // |impulse| is below the minimum is marked by a one in its nibble here;
-    // all children's counts follow at the end.
-    uint32_t still = 0;
+    uint32_t still = 0;  // AccountChildren
     auto account = [&](int c, float r) { still |= r < p.minimumImpulse ? 1u << (4 * c) : 0u; };
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -1181,15 +1194,7 @@ __device__ __forceinline__ void SolveManifold(const ManifoldSoA& m, int s, BodyS
             account(kTwistChild, fabsf(lambda));
         }
     }
-    // A still child's count goes up, a moving one's starts again, a stopped
-    // one keeps its 15; a count that passes minimumIterationCount -- one more
-    // than it, since the child was active -- becomes 15.
-    const uint32_t off = children & (children >> 1) & (children >> 2) & (children >> 3) & 0x11111111u;
-    children = (children & (off * 15u)) | ((children & (still * 15u)) + still);
-    const uint32_t x = children ^ (still * ((uint32_t)p.minimumIterationCount + 1u));
-    const uint32_t stop = still & ~(x | (x >> 1) | (x >> 2) | (x >> 3));
-    children |= stop * 15u;
-    if (children == ~0u) st &= ~kGroupActive;
+    st = AccountChildren(st, children, still, p);
     m.penacc[s] = make_float4(accs[0], accs[1], accs[2], accs[3]);
     m.fricacc[s] = f;
     state = make_uint2(st, children);
