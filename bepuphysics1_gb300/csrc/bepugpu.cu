@@ -1506,6 +1506,7 @@ bepugpu_status bepugpu_upload_bodies(bepugpu_context* c, int32_t id, const bepug
         if (s->asyncPending) CK(cudaStreamSynchronize(s->stream));
         s->asyncPending = false;
         ReleaseIslands(s);
+        CK(s->FetchColouring());
         ReleasePairs(s);
         s->version++;
     }
@@ -1612,6 +1613,7 @@ bepugpu_status bepugpu_upload_constraints(bepugpu_context* c, int32_t id, const 
         ctx->SetError("a constraint references a body outside [0, %d)", nb);
         return BEPUGPU_INVALID_ARGUMENT;
     }
+    s->colouringOnDevice = false;
     // Manifold and joint slots: the colour-sweep part in colour-major order,
     // then the island groups (groups.cu); the persistent mode keeps everything
     // on the sweep path.
@@ -2053,8 +2055,10 @@ bepugpu_status bepugpu_get_colouring(bepugpu_context* c, int32_t id, int32_t* co
     CTX_CHECK(ctx);
     Scene* s = FindScene(ctx, id);
     if (!s) return SceneMissing(ctx, id);
-    if (n != s->colouring.colour.size()) {
-        ctx->SetError("colouring has %zu entries", s->colouring.colour.size());
+    if (s->colouringOnDevice && n == (uint32_t)s->colouringEntries) CK(s->FetchColouring());
+    if (s->colouringOnDevice || n != s->colouring.colour.size()) {
+        ctx->SetError("colouring has %zu entries",
+                      s->colouringOnDevice ? (size_t)s->colouringEntries : s->colouring.colour.size());
         return BEPUGPU_INVALID_ARGUMENT;
     }
     if (colour && n) std::memcpy(colour, s->colouring.colour.data(), 4 * n);

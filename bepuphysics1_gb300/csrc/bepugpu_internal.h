@@ -362,7 +362,7 @@ struct Scene {
     // flow.cu: the tables from the constraint upload's records (bodies a, b
     // per manifold record), or from update_pairs' sorted (body, entry) keys.
     bepugpu_status UploadFlow(Context* ctx, const int32_t* a, const int32_t* b);
-    bepugpu_status UploadFlowChunks(Context* ctx, const std::vector<int2>& groupChunks);
+    bepugpu_status UploadFlowChunks(Context* ctx, const std::vector<int2>& groupChunks, size_t slots);
     bepugpu_status BuildFlowOnDevice(Context* ctx, const unsigned long long* entries, int count, const int2* ends,
                                      const int* slots);
     int SweepColours() const { return manifoldOffsets.empty() ? 0 : (int)manifoldOffsets.size() - 1; }
@@ -406,6 +406,11 @@ struct Scene {
     bepugpu_body* bodyRecords = nullptr;  // device copy of the last uploaded body records (downloads patch it)
     std::vector<float4> hostJointAcc;     // download scratch: [2][joints]
     Colouring colouring;
+    // update_pairs leaves the per-entry arrays on the device (pairs.cu) until a
+    // caller asks for them.
+    bool colouringOnDevice = false;
+    int32_t colouringEntries = 0;
+    cudaError_t FetchColouring();
     std::vector<int32_t> manifoldOffsets;
     std::vector<int32_t> hostSlotOf;
     std::vector<float> hostLinDamp, hostAngDamp, hostLocalM33;

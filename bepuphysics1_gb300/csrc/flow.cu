@@ -530,10 +530,10 @@ bepugpu_status Scene::UploadFlow(Context* ctx, const int32_t* a, const int32_t* 
         }
         if (!any) break;
     }
-    return UploadFlowChunks(ctx, groupChunks);
+    return UploadFlowChunks(ctx, groupChunks, groupPlan.slotOf.size());
 }
 
-bepugpu_status Scene::UploadFlowChunks(Context* ctx, const std::vector<int2>& groupChunks) {
+bepugpu_status Scene::UploadFlowChunks(Context* ctx, const std::vector<int2>& groupChunks, size_t slots) {
     std::vector<int2> chunks = FlowChunks(manifoldOffsets);
     flow.chunkCount = (int)chunks.size();
     flow.groupChunkCount = (int)groupChunks.size();
@@ -546,7 +546,7 @@ bepugpu_status Scene::UploadFlowChunks(Context* ctx, const std::vector<int2>& gr
     }
     CK(cudaHostGetDevicePointer((void**)&flow.error, ctx->flowError, 0));
     // the ends without a dynamic body keep visit -1
-    CK(cudaMemsetAsync(flow.visit, 0xff, sizeof(int2) * groupPlan.slotOf.size(), stream));
+    CK(cudaMemsetAsync(flow.visit, 0xff, sizeof(int2) * slots, stream));
     CK(cudaMemcpyAsync(flow.chunks, chunks.data(), sizeof(int2) * chunks.size(), cudaMemcpyHostToDevice, stream));
     CK(cudaStreamSynchronize(stream));
     return BEPUGPU_OK;
@@ -556,7 +556,7 @@ bepugpu_status Scene::BuildFlowOnDevice(Context* ctx, const unsigned long long* 
                                         const int* slots) {
     k_flow_csr<<<(count + 1 + 255) / 256, 256, 0, stream>>>(entries, count, b.count, ends, slots, flow);
     CK(cudaGetLastError());
-    return UploadFlowChunks(ctx, {});
+    return UploadFlowChunks(ctx, {}, count / 2);
 }
 
 bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool groups, bool warm, int* launches) {

@@ -38,11 +38,32 @@ struct PairBuffers {
     int32_t materialCount = 0;
     void* block = nullptr;
     size_t blockBytes = 0;
+    int* colouring = nullptr;  // the last call's colours, then their order; the scene's capacity of each
     ~PairBuffers() {
+        cudaFree(colouring);
         cudaFree(material);
         cudaFree(block);
     }
 };
+
+// The entries' colours and their order that the last update_pairs kept.  They
+// are read by bepugpu_get_colouring alone, so the call itself does not wait for
+// them: copying them and the slots into host vectors on each call was 70 of
+// the 1,000 us a settling heap's frame of 82,000 pairs takes.
+cudaError_t Scene::FetchColouring() {
+    if (!colouringOnDevice) return cudaSuccess;
+    const size_t n = colouringEntries, bytes = sizeof(int32_t) * n;
+    std::vector<int32_t> colour(n), order(n);
+    cudaError_t e = cudaSuccess;
+    if (n && ((e = cudaMemcpyAsync(colour.data(), pairs->colouring, bytes, cudaMemcpyDeviceToHost, stream)) ||
+              (e = cudaMemcpyAsync(order.data(), pairs->colouring + n, bytes, cudaMemcpyDeviceToHost, stream)) ||
+              (e = cudaStreamSynchronize(stream))))
+        return e;
+    colouring.colour.swap(colour);
+    colouring.order.swap(order);
+    colouringOnDevice = false;
+    return cudaSuccess;
+}
 
 void ReleasePairs(Scene* s) {
     delete s->pairs;
@@ -539,6 +560,14 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
         }
         P.blockBytes = bytes;
     }
+    if (!P.colouring) {
+        const size_t bytes = 2 * sizeof(int) * std::max<size_t>(s->maxManifolds, 1);
+        cudaError_t e = cudaMalloc(&P.colouring, bytes);
+        if (e != cudaSuccess) {
+            ctx->SetError("update_pairs: %zu bytes for the colouring: %s", bytes, cudaGetErrorString(e));
+            return e == cudaErrorMemoryAllocation ? BEPUGPU_OUT_OF_MEMORY : BEPUGPU_CUDA_ERROR;
+        }
+    }
     Carve cv{(char*)P.block};
     const int T = 256;
     auto* table = cv.take<unsigned long long>(tableSlots);
@@ -586,6 +615,8 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
         k_move_lanes<<<(n + T - 1) / T, T, 0, st>>>(s->m, rec, col.slotOf, n, P.material, scratch);
         k_lanes_back<<<(n + T - 1) / T, T, 0, st>>>(s->m, scratch, n, s->genSlotsDev);
         CK(cudaMemcpyAsync(s->slotOf, col.slotOf, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(P.colouring, col.colour, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(P.colouring + n, col.order, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
     }
     CK(cudaGetLastError());
     // the scene's bookkeeping: every manifold on the colour-sweep path
@@ -596,17 +627,11 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
     plan.globalOffsets = col.offsets;
     plan.globalCount = n;
     plan.jointGlobalOffsets.assign(col.colours + 1, 0);
-    plan.slotOf.resize(n);
     plan.jointSlotOf.clear();
     s->colouring.colours = col.colours;
-    s->colouring.colour.resize(n);
-    s->colouring.order.resize(n);
     s->colouring.offsets = col.offsets;
-    if (n) {
-        CK(cudaMemcpyAsync(s->colouring.colour.data(), col.colour, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(s->colouring.order.data(), col.order, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(plan.slotOf.data(), col.slotOf, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
-    }
+    s->colouringOnDevice = true;
+    s->colouringEntries = n;
     s->manifoldOffsets = col.offsets;
     s->flow.chunkCount = s->flow.groupChunkCount = 0;
     if (n) {
@@ -614,7 +639,6 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
         if (fs != BEPUGPU_OK) return fs;
     }
     s->jointOffsets.assign(col.colours + 1, 0);
-    s->hostSlotOf = plan.slotOf;
     s->m.count = n;
     s->generatedCount = n;
     s->hostGenPairs.clear();  // the shapes' pair check of bepugpu_upload_shapes applies to uploaded records only

@@ -3,6 +3,8 @@ the sizes where they can go wrong: few keys, keys on either side of a block's
 tile, more pairs than the first buffer holds, and colours past one 64-bit mask."""
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -75,4 +77,40 @@ def test_pairs_that_come_and_go(gpu_context):
         got = got[np.lexsort((got[:, 1], got[:, 0]))]
         np.testing.assert_array_equal(got, obp.overlapping_pairs(state, sh, DT))
         np.testing.assert_array_equal(sp.colouring()[0], colour_list(state, m)[0])
+    sp.close()
+
+
+def test_colouring_is_kept_until_asked_for(gpu_context):
+    """The colouring of the last pair update, or of the upload after it: read
+    late, twice, past a refused count, and after the scene's buffers went."""
+    gpu_context.set_settings(default_settings())
+    b, _, sh = _jumble(seed=12, n=300, sphere_every=4)
+    sp = GpuSpace(gpu_context, b, None, capacity=(len(b), 16 * len(b), 0), shapes=sh)
+    sp.set_materials(np.full((len(b), 3), 0.5, np.float32))
+    away = b.copy()
+    away["position"][np.flatnonzero(b["is_dynamic"] != 0)[::3], 1] += 500
+    sp.update_pairs(DT)
+    sp.update_bodies(away)
+    n = sp.update_pairs(DT)  # fewer records, the colours of the update before never read
+    m, _ = sp.download_constraints()
+    want = colour_list(away, m)
+    out = np.zeros(n + 1, np.int32)
+    k = ctypes.c_uint32()
+
+    def status(count):
+        return sp.ctx.lib.bepugpu_get_colouring(sp.ctx.handle, sp.id, N.ptr(out), None, count, ctypes.byref(k))
+
+    for again in range(2):
+        assert status(n + 1) == status(0) == N.INVALID_ARGUMENT
+        for got, w in zip(sp.colouring(), want):
+            np.testing.assert_array_equal(got, w)
+    sp.update_pairs(DT)
+    sp.upload_bodies(away)  # materials and their buffers are given up
+    for got, w in zip(sp.colouring(), want):
+        np.testing.assert_array_equal(got, w)
+    sp.set_materials(np.full((len(b), 3), 0.5, np.float32))
+    sp.update_pairs(DT)
+    sp.upload_constraints(m[: n // 2])
+    for got, w in zip(sp.colouring(), colour_list(away, m[: n // 2])):
+        np.testing.assert_array_equal(got, w)
     sp.close()
