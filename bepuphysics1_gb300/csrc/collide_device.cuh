@@ -14,7 +14,13 @@
 //   Box/SphereContactManifold.Update (:55-83) and the constraint's
 //   AddContact / RemoveContact (ConvexContactManifoldConstraint.cs:117-155).
 // One thread owns one manifold; candidate lists live in local arrays of eight
-// (TinyStructList's capacity).  Built with -fmad=false like the rest of the
+// (TinyStructList's capacity).  Bound by the length of a thread's own chain
+// and its lanes' divergence, not by memory: all warps of 65,536 pairs are
+// resident at once.  So the contacts that stay are indices in registers, their
+// lanes untouched in memory (they were local arrays read and written whole,
+// most of an 816-byte stack frame that is now 336), and the clip's crossings
+// are listed by bits before they are computed.  Eight steps of 65,536 box
+// pairs: 1,210 -> 1,018 us; a settling heap's four frames 3,723 -> 3,578.  Built with -fmad=false like the rest of the
 // library; (float)Math.Sqrt of a float is the IEEE float square root, and
 // Vector3.Normalize's 1/Math.Sqrt stays in double.
 #pragma once
@@ -80,10 +86,6 @@ struct Cands {
     int n;
     __device__ __forceinline__ void add(V3 pos, float depth, int i) {
         if (n < 8) { p[n] = pos; d[n] = depth; id[n] = i; n++; }
-    }
-    __device__ __forceinline__ void removeAt(int i) {
-        for (int k = i; k + 1 < n; k++) { p[k] = p[k + 1]; d[k] = d[k + 1]; id[k] = id[k + 1]; }
-        n--;
     }
 };
 
@@ -188,49 +190,35 @@ struct Face {
 };
 
 // GetNearestFace: the face whose normal is most aligned with `m` (none when
-// no component strictly dominates, as in the reference).
+// no component strictly dominates, as in the reference).  The corners V1..V4
+// (:6076-6170) run + - - + along the first of the face's two axes and + + - -
+// along the second; a sign taken out of a product is exact, so each axis'
+// products are formed once.
 __device__ __forceinline__ void NearestFace(V3 pos, const V3 o[3], V3 m, V3 h, Face& f) {
-    float dd[3] = {dot(o[0], m), dot(o[1], m), dot(o[2], m)};
-    float ad[3] = {fabsf(dd[0]), fabsf(dd[1]), fabsf(dd[2])};
-    int k = -1;
-    if (ad[0] > ad[1] && ad[0] > ad[2]) k = 0;
-    else if (ad[1] > ad[0] && ad[1] > ad[2]) k = 1;
-    else if (ad[2] > ad[0] && ad[2] > ad[1]) k = 2;
-    for (int i = 0; i < 4; i++) { f.v[i] = mk(0, 0, 0); f.id[i] = 0; }
-    f.normal = mk(0, 0, 0);
-    f.width = f.height = 0;
-    if (k < 0) return;
-    const bool neg = dd[k] < 0;
-    float hw = h.x, hh = h.y, hl = h.z;
-    int bit;
-    // corner signs (x, y, z) of V1..V4 on each face family, from :6076-6170
-    int sx[4], sy[4], sz[4];
-    if (k == 0) {
-        if (neg) { hw = -hw; bit = 0; } else bit = 1;
-        const int X[4] = {1, 1, 1, 1}, Y[4] = {1, -1, -1, 1}, Z[4] = {1, 1, -1, -1};
-        for (int i = 0; i < 4; i++) { sx[i] = X[i]; sy[i] = Y[i]; sz[i] = Z[i]; }
-        f.width = hh * 2; f.height = hl * 2;
-        f.id[0] = bit + 2 + 4; f.id[1] = bit + 4; f.id[2] = bit + 2; f.id[3] = bit;
-    } else if (k == 1) {
-        if (neg) { hh = -hh; bit = 0; } else bit = 2;
-        const int X[4] = {1, -1, -1, 1}, Y[4] = {1, 1, 1, 1}, Z[4] = {1, 1, -1, -1};
-        for (int i = 0; i < 4; i++) { sx[i] = X[i]; sy[i] = Y[i]; sz[i] = Z[i]; }
-        f.width = hw * 2; f.height = hl * 2;
-        f.id[0] = 1 + bit + 4; f.id[1] = bit + 4; f.id[2] = 1 + bit; f.id[3] = bit;
-    } else {
-        if (neg) { hl = -hl; bit = 0; } else bit = 4;
-        const int X[4] = {1, -1, -1, 1}, Y[4] = {1, 1, -1, -1}, Z[4] = {1, 1, 1, 1};
-        for (int i = 0; i < 4; i++) { sx[i] = X[i]; sy[i] = Y[i]; sz[i] = Z[i]; }
-        f.width = hw * 2; f.height = hh * 2;
-        f.id[0] = 1 + 2 + bit; f.id[1] = 2 + bit; f.id[2] = 1 + bit; f.id[3] = bit;
+    const float d0 = dot(o[0], m), d1 = dot(o[1], m), d2 = dot(o[2], m);
+    const float a0 = fabsf(d0), a1 = fabsf(d1), a2 = fabsf(d2);
+    const bool k0 = a0 > a1 && a0 > a2, k1 = a1 > a0 && a1 > a2, k2 = a2 > a0 && a2 > a1;
+    if (!k0 && !k1 && !k2) {
+        for (int i = 0; i < 4; i++) { f.v[i] = mk(0, 0, 0); f.id[i] = 0; }
+        f.normal = mk(0, 0, 0);
+        f.width = f.height = 0;
+        return;
     }
+    const bool neg = (k0 ? d0 : k1 ? d1 : d2) < 0;
+    const V3 n = k0 ? o[0] : k1 ? o[1] : o[2];
+    f.normal = neg ? -n : n;
+    f.width = (k0 ? h.y : h.x) * 2;
+    f.height = (k2 ? h.y : h.z) * 2;
+    const int bit = neg ? 0 : (k0 ? 1 : k1 ? 2 : 4), u = k0 ? 2 : 1, w = k2 ? 2 : 4;
+    f.id[0] = bit + u + w; f.id[1] = bit + w; f.id[2] = bit + u; f.id[3] = bit;
+    const V3 x = scale(o[0], h.x), y = scale(o[1], h.y), z = scale(o[2], h.z);
+#pragma unroll
     for (int i = 0; i < 4; i++) {
-        float x = sx[i] > 0 ? hw : -hw, y = sy[i] > 0 ? hh : -hh, z = sz[i] > 0 ? hl : -hl;
+        const bool n1 = i == 1 || i == 2, n2 = i >= 2;  // the corner's signs on the face's axes
+        const bool nx = k0 ? neg : n1, ny = k0 ? n1 : k1 ? neg : n2, nz = k2 ? neg : n2;
         // Matrix.Transform by the orientation rows and the position (Matrix.cs:717-725)
-        f.v[i] = mk(x * o[0].x + y * o[1].x + z * o[2].x + pos.x, x * o[0].y + y * o[1].y + z * o[2].y + pos.y,
-                    x * o[0].z + y * o[1].z + z * o[2].z + pos.z);
+        f.v[i] = (nx ? -x : x) + (ny ? -y : y) + (nz ? -z : z) + pos;
     }
-    f.normal = neg ? -o[k] : o[k];
 }
 
 struct ClipEdge {
@@ -324,27 +312,35 @@ __device__ __forceinline__ void ClipFaces(const Face& clip, const Face& face, V3
     // neighbour then its higher one (v1: v2, v4) -- on edge v3v4, v4 tries v3
     // before v1.  Candidates past eight are dropped; depths are taken once at
     // the end.
-    const int flagOf[4] = {4, 2, 8, 1};
+    // Every lane lists its crossings first, one bit each in that order (edge,
+    // vertex, neighbour), and the lanes then walk their own lists together: a
+    // quad crosses a clip line twice at most, against 32 turns of the loops.
     const int first = out.n;
+    unsigned crossings = 0;
+#pragma unroll
     for (int e = 0; e < 4; e++) {
-        const ClipEdge ce = EdgeOf(clip, e);
-        const int fl = flagOf[e];
+        const int fl = e == 0 ? 4 : e == 1 ? 2 : e == 2 ? 8 : 1;
+#pragma unroll
         for (int v = 0; v < 4; v++) {
-            if (fv[v] & fl) continue;
-            int n0 = (v + 1) & 3, n1 = (v + 3) & 3;
-            int lo = n0 < n1 ? n0 : n1, hi = n0 < n1 ? n1 : n0;
-            if (e == 2 && v == 3) { int t = lo; lo = hi; hi = t; }
-            for (int w = 0; w < 2; w++) {
-                const int n = w == 0 ? lo : hi;
-                if (!(fv[n] & fl)) continue;
-                // the face edge between v and n, in the reference's argument order
-                const bool wrap = (v == 0 && n == 3) || (v == 3 && n == 0);
-                const int p = wrap ? 3 : (v < n ? v : n), q = (p + 1) & 3;
-                V3 at;
-                if (out.n < 8 && Intersect(face.v[p], face.v[q], ce, at))
-                    out.add(at, 0.f, EdgeId(face.id[p], face.id[q]) * 2549 + ce.id * 2857);
-            }
+            const int a = (v + 1) & 3, b = (v + 3) & 3;
+            const bool swap = (e == 2 && v == 3) != (a > b);  // whether the higher neighbour comes first
+            const int n0 = swap ? b : a, n1 = swap ? a : b;
+            const unsigned at = 8 * e + 2 * v;
+            if (!(fv[v] & fl)) crossings |= ((fv[n0] & fl) ? 1u << at : 0u) | ((fv[n1] & fl) ? 2u << at : 0u);
         }
+    }
+    while (crossings && out.n < 8) {
+        const int at = __ffs((int)crossings) - 1, e = at >> 3, v = (at >> 1) & 3;
+        crossings &= crossings - 1;
+        const int a = (v + 1) & 3, b = (v + 3) & 3;
+        const bool swap = (e == 2 && v == 3) != (a > b);
+        const int n = swap != (bool)(at & 1) ? b : a;
+        const ClipEdge ce = EdgeOf(clip, e);
+        // the face edge between v and n, in the reference's argument order
+        const int p = ((v + 1) & 3) == n ? v : n, q = (p + 1) & 3;
+        V3 hit;
+        if (Intersect(face.v[p], face.v[q], ce, hit))
+            out.add(hit, 0.f, EdgeId(face.id[p], face.id[q]) * 2549 + ce.id * 2857);
     }
     // depths of the edge candidates; positive ones dropped, order kept
     int kept = first;
@@ -511,41 +507,43 @@ __device__ __forceinline__ bool BoxSphere(V3 h, float r, V3 pa, float4 qa, V3 pb
 }
 
 // The manifold's contacts in solver order (the constraint's penetration
-// list) plus the manifold's own list order.
+// list) plus the manifold's own list order.  A contact is the slot index its
+// lanes lie at so far and the candidate it takes its position from, four bits
+// each (15: none); the lanes themselves stay in memory.
 struct Kept {
-    float4 cp[4], cn[4], oa[4], ob[4];
-    float4 cf[4];  // NONCONVEX: each contact's friction direction and impulse
-    float acc[4];
+    uint32_t from, cand;  // by solver index
+    uint32_t list;        // list position -> solver index, two bits each
     int n;
-    int list[4];  // list position -> solver index
 };
+__device__ __forceinline__ int Nibble(uint32_t w, int i) { return (int)(w >> (4 * i)) & 15; }
+__device__ __forceinline__ uint32_t SetNibble(uint32_t w, int i, int v) {
+    return (w & ~(15u << (4 * i))) | ((uint32_t)v << (4 * i));
+}
+__device__ __forceinline__ int ListAt(uint32_t w, int i) { return (int)(w >> (2 * i)) & 3; }
+__device__ __forceinline__ uint32_t SetList(uint32_t w, int i, int v) {
+    return (w & ~(3u << (2 * i))) | ((uint32_t)v << (2 * i));
+}
 
 // ContactManifold.Remove of list entry i: the list moves its last entry into
 // the gap (RawList.FastRemoveAt); the constraint removes its penetration child
 // (and, NONCONVEX, the contact's friction child) keeping order (RawList.RemoveAt).
 __device__ __forceinline__ void RemoveListAt(Kept& k, int i) {
-    const int p = k.list[i];
-    k.list[i] = k.list[k.n - 1];
-    for (int q = p; q + 1 < k.n; q++) {
-        k.cp[q] = k.cp[q + 1]; k.cn[q] = k.cn[q + 1]; k.oa[q] = k.oa[q + 1]; k.ob[q] = k.ob[q + 1];
-        k.cf[q] = k.cf[q + 1];
-        k.acc[q] = k.acc[q + 1];
-    }
+    const int p = ListAt(k.list, i);
+    k.list = SetList(k.list, i, ListAt(k.list, k.n - 1));
+    const uint32_t below = (1u << (4 * p)) - 1u;
+    k.from = (k.from & below) | ((k.from >> 4) & ~below);
+    k.cand = (k.cand & below) | ((k.cand >> 4) & ~below);
     k.n--;
-    for (int q = 0; q < k.n; q++)
-        if (k.list[q] > p) k.list[q]--;
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+        if (q < k.n && ListAt(k.list, q) > p) k.list -= 1u << (2 * q);
 }
 
 // ContactManifold.Add: appended to both lists with a fresh (zero) impulse.
-__device__ __forceinline__ void AddContact(Kept& k, V3 p, V3 n, float depth, int id) {
-    const int s = k.n;
-    k.cp[s] = make_float4(p.x, p.y, p.z, depth);
-    k.cn[s] = make_float4(n.x, n.y, n.z, __int_as_float(id));
-    k.oa[s] = make_float4(0, 0, 0, 0);
-    k.ob[s] = make_float4(0, 0, 0, 0);
-    k.cf[s] = make_float4(0, 0, 0, 0);  // ContactFrictionConstraint.Setup: linearA = 0, impulse 0
-    k.acc[s] = 0.f;
-    k.list[s] = s;
+__device__ __forceinline__ void AddContact(Kept& k, int candidate) {
+    k.from = SetNibble(k.from, k.n, 15);
+    k.cand = SetNibble(k.cand, k.n, candidate);
+    k.list = SetList(k.list, k.n, k.n);
     k.n++;
 }
 
@@ -561,92 +559,107 @@ __device__ __forceinline__ void CollideManifold(const ManifoldSoA& m, const Body
     const int ta = __float_as_int(sa.w), tb = __float_as_int(sb.w);
     Kept k;
     k.n = h.z & 0xff;
+    k.from = 0x3210u;
+    k.cand = 0xffffu;
     float4 fr = m.fricacc[s];
-    const uint32_t code = (uint32_t)__float_as_int(fr.w) ^ 0xE4u;
+    k.list = ((uint32_t)__float_as_int(fr.w) ^ 0xE4u) & 0xffu;
     const float4 pen = m.penacc[s];
-    const float accs[4] = {pen.x, pen.y, pen.z, pen.w};
+    int ids[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) ids[q] = q < k.n ? __float_as_int(m.cnrm[q * cap + s].w) : 0;
     const bool nonConvex = ((uint32_t)h.z >> 8) & kManifoldNonConvex;
-    for (int q = 0; q < 4; q++) {
-        if (q < k.n) {
-            k.cp[q] = m.cpos[q * cap + s];
-            k.cn[q] = m.cnrm[q * cap + s];
-            k.oa[q] = m.offA[q * cap + s];
-            k.ob[q] = m.offB[q * cap + s];
-            k.cf[q] = nonConvex ? m.cfr[q * cap + s] : make_float4(0, 0, 0, 0);
-            k.acc[q] = accs[q];
-            k.list[q] = (int)((code >> (2 * q)) & 3u);
-        }
-    }
     const int before = k.n;
     bool setup = false;  // the first contact after none: friction is set up again
+    V3 axis = mk(0, 0, 0);
+    Cands c;
+    c.n = 0;
     if (ta == 1 && tb == 1) {
-        V3 axis;
-        Cands c;
-        c.n = 0;
         if (BoxBox(mk(sa.x, sa.y, sa.z), mk(sb.x, sb.y, sb.z), pa, qa, pb, qb, axis, c)) {
             axis = -axis;
-            int toRemove[4], nr = 0;
-            for (int i = 0; i < k.n; i++) {
-                const int pi = k.list[i];
-                const int id = __float_as_int(k.cn[pi].w);
-                bool found = false;
-                for (int j = c.n - 1; j >= 0; j--) {
-                    if (c.id[j] == id) {
-                        found = true;
-                        k.cp[pi] = make_float4(c.p[j].x, c.p[j].y, c.p[j].z, -c.d[j]);
-                        k.cn[pi] = make_float4(axis.x, axis.y, axis.z, k.cn[pi].w);
-                        c.removeAt(j);
-                        break;
-                    }
+            // a contact takes the last candidate left that has its id
+            unsigned left = (1u << c.n) - 1u, gone = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                if (i >= k.n) continue;
+                const int pi = ListAt(k.list, i);
+                const int id = pi == 0 ? ids[0] : pi == 1 ? ids[1] : pi == 2 ? ids[2] : ids[3];
+                int j = c.n - 1;
+                while (j >= 0 && !((left >> j & 1u) && c.id[j] == id)) j--;
+                if (j >= 0) {
+                    left &= ~(1u << j);
+                    k.cand = SetNibble(k.cand, pi, j);
+                } else {
+                    gone |= 1u << i;
                 }
-                if (!found) toRemove[nr++] = i;
             }
-            for (int r = nr - 1; r >= 0; r--) RemoveListAt(k, toRemove[r]);
+            for (int r = 3; r >= 0; r--)
+                if (gone >> r & 1u) RemoveListAt(k, r);
             const bool emptied = before > 0 && k.n == 0;
-            for (int j = 0; j < c.n; j++) {
+            for (; left; left &= left - 1) {
                 if (k.n == 0) setup = true;
-                AddContact(k, c.p[j], axis, -c.d[j], c.id[j]);
+                AddContact(k, __ffs((int)left) - 1);
             }
             if (emptied) fr = make_float4(0.f, 0.f, 0.f, fr.w);
         } else {
-            for (int i = k.n - 1; i >= 0; i--) RemoveListAt(k, i);
+            k.n = 0;
             if (before > 0) fr = make_float4(0.f, 0.f, 0.f, fr.w);
         }
     } else {
-        One c;
-        const bool hit = ta == 2 ? SphereSphere(sa.x, sb.x, pa, pb, prm.maximumContactDistance, c)
-                                 : BoxSphere(mk(sa.x, sa.y, sa.z), sb.x, pa, qa, pb, prm.maximumContactDistance, c);
+        One one;
+        const bool hit = ta == 2 ? SphereSphere(sa.x, sb.x, pa, pb, prm.maximumContactDistance, one)
+                                 : BoxSphere(mk(sa.x, sa.y, sa.z), sb.x, pa, qa, pb, prm.maximumContactDistance, one);
         const bool previously = k.n > 0;
         if (hit) {
-            if (!previously && c.depth >= 0) {
+            axis = one.n;
+            c.p[0] = one.p;
+            c.d[0] = -one.depth;
+            c.id[0] = ids[0];
+            if (!previously && one.depth >= 0) {
                 setup = true;
-                AddContact(k, c.p, c.n, c.depth, 0);
+                AddContact(k, 0);
             } else if (previously) {
-                const int p = 0;
-                k.cp[p] = make_float4(c.p.x, c.p.y, c.p.z, c.depth);
-                k.cn[p] = make_float4(c.n.x, c.n.y, c.n.z, k.cn[p].w);
+                k.cand = SetNibble(k.cand, 0, 0);
             }
         } else if (previously) {
             RemoveListAt(k, 0);
             fr = make_float4(0.f, 0.f, 0.f, fr.w);
         }
     }
-    // write back: contacts in solver order, the list order, impulses
+    // Write back: contacts in solver order, the list order, impulses.  A kept
+    // contact's lanes only ever move down, so in ascending order they move in
+    // place; those that stay where they were are not touched.
     uint32_t out = 0;
-    for (int q = 0; q < 4; q++) out |= (uint32_t)(q < k.n ? k.list[q] : q) << (2 * q);
-    fr.w = __int_as_float((int)(out ^ 0xE4u));
+    float acc[4];
+#pragma unroll
     for (int q = 0; q < 4; q++) {
+        out |= (uint32_t)(q < k.n ? ListAt(k.list, q) : q) << (2 * q);
+        acc[q] = 0.f;
         if (q < k.n) {
-            m.cpos[q * cap + s] = k.cp[q];
-            m.cnrm[q * cap + s] = k.cn[q];
-            m.offA[q * cap + s] = k.oa[q];
-            m.offB[q * cap + s] = k.ob[q];
+            const int from = Nibble(k.from, q), j = Nibble(k.cand, q);
+            acc[q] = from == 0 ? pen.x : from == 1 ? pen.y : from == 2 ? pen.z : from == 3 ? pen.w : 0.f;
+            const bool fresh = from == 15;
+            const int at = q * cap + s, was = fresh ? at : from * cap + s;
+            const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (from != q) {
+                m.offA[at] = fresh ? none : m.offA[was];
+                m.offB[at] = fresh ? none : m.offB[was];
+                // ContactFrictionConstraint.Setup: linearA = 0, impulse 0
+                if (nonConvex) m.cfr[at] = fresh ? none : m.cfr[was];
+                if (j == 15) {
+                    m.cpos[at] = m.cpos[was];
+                    m.cnrm[at] = m.cnrm[was];
+                }
+            }
+            if (j != 15) {
+                m.cpos[at] = make_float4(c.p[j].x, c.p[j].y, c.p[j].z, -c.d[j]);
+                m.cnrm[at] = make_float4(axis.x, axis.y, axis.z, __int_as_float(c.id[j]));
+            }
+        } else if (nonConvex && q < before) {
+            m.cfr[q * cap + s] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        if (nonConvex && q < (k.n > before ? k.n : before))
-            m.cfr[q * cap + s] = q < k.n ? k.cf[q] : make_float4(0, 0, 0, 0);
     }
-    m.penacc[s] = make_float4(k.n > 0 ? k.acc[0] : 0.f, k.n > 1 ? k.acc[1] : 0.f, k.n > 2 ? k.acc[2] : 0.f,
-                              k.n > 3 ? k.acc[3] : 0.f);
+    fr.w = __int_as_float((int)(out ^ 0xE4u));
+    m.penacc[s] = make_float4(acc[0], acc[1], acc[2], acc[3]);
     m.fricacc[s] = fr;
     if (setup) {
         float4 ax = m.saxis[s];
