@@ -41,4 +41,32 @@ __device__ __forceinline__ bool GridBarrier(unsigned int* counter, volatile unsi
     return *err == 0;
 }
 
+// The same for a kernel that knows its number of barriers: `counter` only
+// counts up while it runs, so a block that has arrived waits for the counter
+// itself, with no reset and no generation behind the last arrival.  `arrived`
+// is the blocks' total before this barrier.  FinishGridBarriers, on every
+// block's way out, lets the last one put the counter back to zero.
+__device__ __forceinline__ bool CountBarrier(unsigned int* counter, unsigned int& arrived, volatile int* err) {
+    arrived += gridDim.x;
+    bool ok = true;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(counter, 1u);
+        for (long long spins = 1; *(volatile unsigned int*)counter < arrived; spins++) {
+            if (spins > kBarrierSpinLimit) *err = BEPUGPU_TIMEOUT;
+            // another block's error is looked for now and then: a load a poll is a trip through L2
+            if ((spins & 63) == 0 && *err) {
+                ok = false;
+                break;
+            }
+        }
+        __threadfence();
+    }
+    return __syncthreads_and(ok);
+}
+__device__ __forceinline__ void FinishGridBarriers(unsigned int* counter, unsigned int arrived) {
+    if (threadIdx.x == 0 && atomicAdd(counter, 1u) == arrived + gridDim.x - 1) atomicExch(counter, 0u);
+}
+
 }  // namespace bepugpu

@@ -6,13 +6,14 @@
 // stable: a block counts its tile's digits, a grid barrier, every block adds
 // up the blocks' counts to its own digit offsets, and moves its tile in order
 // (ranks from __match_any_sync inside a warp, a prefix over the warps).  Four
-// passes are eight barriers in one launch.
-// Bound by the barriers and the passes' trips through L2, not by bandwidth:
-// about 16 us a pass.  The broad phase of 65,536 boxes sorts some 230,000 cell
-// entries by 18 bits and 150,000 pairs by 34 in 97 us, where the bitonic
-// network that this replaces took 57 launches and 224 us.  64 blocks: with 32
-// the tiles' serial ranking, with 128 the blocks' adding up of each other's
-// counts cost more (235 and 237 us a broad phase against 222).
+// passes are seven barriers in one launch.
+// Bound by the barriers and the passes' trips through L2, not by bandwidth: a
+// barrier that counts up and is polled for itself, in place of one that resets
+// and then releases, took the broad phase of 65,536 boxes (some 230,000 cell
+// entries by 18 bits and 150,000 pairs by 34) from 219 to 206 us; the bitonic
+// network before it took 57 launches and 451.  64 blocks: with 32 the tiles'
+// serial ranking, with 128 the barriers cost more (235 and 237 us a broad phase
+// against 222, before the change of barrier; 100 blocks 218 against 206 after).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,11 +32,11 @@ constexpr int kSortDigitBits = 9, kSortBins = 1 << kSortDigitBits;
 __global__ void __launch_bounds__(kSortThreads) k_radix_sort(unsigned long long* keys, unsigned long long* other,
                                                              const unsigned* __restrict__ count, unsigned capacity,
                                                              SortDigits digits, unsigned* hist, unsigned* counter,
-                                                             unsigned* generation, int* err) {
+                                                             int* err) {
     __shared__ unsigned base[kSortBins];
     __shared__ __align__(16) unsigned short warpCount[kSortWarps][kSortBins];
     __shared__ int warpSums[32];
-    unsigned localGen = *(volatile unsigned*)generation;
+    unsigned arrived = 0;
     const unsigned n = count ? min(*count, capacity) : capacity;
     const unsigned tile = (n + gridDim.x - 1) / gridDim.x;
     const unsigned begin = min(n, blockIdx.x * tile), end = min(n, begin + tile);
@@ -52,7 +53,7 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_sort(unsigned long long*
             atomicAdd(base + ((unsigned)(__ldcg(src + i) >> shift) & mask), 1u);
         __syncthreads();
         if (bin) hist[blockIdx.x * kSortBins + tid] = base[tid];
-        if (!GridBarrier(counter, generation, localGen, err)) return;
+        if (!CountBarrier(counter, arrived, err)) return;
         unsigned total = 0, before = 0;
         if (bin) {
 #pragma unroll 16
@@ -87,15 +88,17 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_sort(unsigned long long*
                 }
             }
             __syncthreads();
-            if (i < end) dst[base[digit] + warpCount[warp][digit] + rank] = key;
+            const unsigned to = i < end ? base[digit] + warpCount[warp][digit] + rank : n;
+            if (to < n) dst[to] = key;
             __syncthreads();
             if (bin) base[tid] += sum;
         }
-        if (!GridBarrier(counter, generation, localGen, err)) return;
+        if (pass + 1 < digits.passes && !CountBarrier(counter, arrived, err)) return;
         unsigned long long* t = src;
         src = dst;
         dst = t;
     }
+    FinishGridBarriers(counter, arrived);
 }
 
 }  // namespace
@@ -135,7 +138,7 @@ cudaError_t RadixSort(const Scene* s, unsigned long long* keys, unsigned long lo
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_radix_sort, keys, other, count, (unsigned)capacity, digits, hist,
-                              s->BarrierCounter(), s->BarrierGeneration(), err);
+                              s->BarrierCounter(), err);
 }
 
 }  // namespace bepugpu
