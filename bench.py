@@ -19,10 +19,10 @@ One step = ContactRefresher -> ForceUpdater -> Solver (prestep, warm start,
   roofline    the dominant kernel: k_groups when island groups run the step
               (algorithmic bytes of the units one launch processes: executed
               solve visits counted by a census, warm start, prestep, bodies),
-              else k_solve (76 d + 136 + 48 c per executed manifold visit);
+              else k_flow (76 d + 136 + 48 c per executed manifold visit);
               divided by the kernel's device time from events captured in the
               step graph; peak = measured HBM copy bandwidth.  `sweep` adds
-              the colour-sweep path's k_solve on the same pile, groups off.
+              the sweep path's k_flow on the same pile, groups off.
   cpu_baseline the oracle port of Solver.UpdateMultithreaded (per-body spin
               locks, chunked parallel loop) on all host cores, on a bounded
               sample of steps of the same pile.
@@ -243,23 +243,25 @@ def timed_steps(space, steps, flush, flags):
 
 
 def solve_roofline(prof, solve_ms, peak, peak_kind):
-    """k_solve: the executed manifold visits' algorithmic bytes (census) over
-    the solve phase's device time, one launch per colour sweep."""
+    """k_flow: the executed manifold visits' algorithmic bytes (census) over the
+    device time of the launch that holds every sweep and the short one before
+    it that sets the turns (and, of scenes that are not too large for it, the
+    warm start, whose bytes are not counted)."""
     bytes_per_step = float(prof["solve_algorithmic_bytes"])
-    launches = int(prof["solve_launches"])
+    launches = 1
     mean_s = statistics.mean(solve_ms) / 1000.0
     achieved = bytes_per_step / mean_s / 1e9 if mean_s > 0 else 0.0
-    return {"bound": "hbm", "kernel": "k_solve", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    return {"bound": "hbm", "kernel": "k_flow", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_kind": peak_kind,
-            "algorithmic_bytes_per_launch": bytes_per_step / max(launches, 1),
+            "algorithmic_bytes_per_launch": bytes_per_step / launches,
             "algorithmic": "76 d + 136 + 48 c per executed manifold visit",
-            "launch_ms_avg": 1000.0 * mean_s / max(launches, 1), "solve_launches_per_step": launches,
+            "launch_ms_avg": 1000.0 * mean_s / launches, "solve_launches_per_step": launches,
             "solve_ms_per_step": 1000.0 * mean_s,
             "manifold_visits_per_step": float(prof["solve_manifold_visits"])}
 
 
 def sweep_section(args, ctx, local, pg, peak, peak_kind):
-    """The colour-sweep path (one launch per colour, one thread per manifold):
+    """The sweep path (every sweep in one launch, ordered visit by visit):
     the 65,536-box pile with island groups off, and the pile packed as config
     1 packs its 1,000 boxes (unit boxes at 1.05 m, +-0.05 m jitter) scaled to
     64 x 16 x 64, whose touching columns make one island too large for a
@@ -1292,14 +1294,14 @@ def main():
                     "kernel_only_ms_per_step": kernel_only}
     else:
         bytes_per_step = float(prof["solve_algorithmic_bytes"])
-        solve_launches = int(prof["solve_launches"])
+        solve_launches = 1
         mean_solve_s = statistics.mean(solve_ms) / 1000.0 if solve_ms else float(prof["solve_ms"]) / 1000.0
         achieved = bytes_per_step / mean_solve_s / 1e9 if mean_solve_s > 0 else 0.0
-        roofline = {"bound": "hbm", "kernel": "k_solve", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                    "frac": achieved / peak, "peak_kind": peak_kind, "traffic": ncu_traffic_per_launch("k_solve"),
-                    "algorithmic_bytes_per_launch": bytes_per_step / max(solve_launches, 1),
+        roofline = {"bound": "hbm", "kernel": "k_flow", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                    "frac": achieved / peak, "peak_kind": peak_kind, "traffic": ncu_traffic_per_launch("k_flow"),
+                    "algorithmic_bytes_per_launch": bytes_per_step / solve_launches,
                     "algorithmic": "76 d + 136 + 48 c per executed manifold visit",
-                    "launch_ms_avg": 1000.0 * mean_solve_s / max(solve_launches, 1),
+                    "launch_ms_avg": 1000.0 * mean_solve_s / solve_launches,
                     "solve_launches_per_step": solve_launches,
                     "manifold_visits_per_step": float(prof["solve_manifold_visits"]),
                     "kernel_only_ms_per_step": kernel_only}
@@ -1377,7 +1379,7 @@ def main():
         space.close()
         sweep = sweep_section(args, ctx, local, pg, peak, peak_kind)
         off = sweep["pile_64k_groups_off"]
-        roofline["sweep"] = {"kernel": "k_solve", "workload": "pile_64k, island groups off",
+        roofline["sweep"] = {"kernel": "k_flow", "workload": "pile_64k, island groups off",
                              "frac": off["roofline"]["frac"], "achieved": off["roofline"]["achieved"],
                              "ms_per_step": off["ms_per_step"],
                              "solve_ms_per_step": off["roofline"]["solve_ms_per_step"],

@@ -357,7 +357,8 @@ typedef struct bepugpu_shape {
 } bepugpu_shape;
 
 /* Solve strategies for the one-scene path. */
-#define BEPUGPU_MODE_GRAPH      0  /* one launch per colour sweep, captured in a CUDA graph */
+#define BEPUGPU_MODE_GRAPH      0  /* launches captured in a CUDA graph: all sweeps of manifolds in one,
+                                      ordered visit by visit; with swept joints one per colour */
 #define BEPUGPU_MODE_PERSISTENT 1  /* one cooperative launch, bounded grid barrier per colour */
 
 int32_t bepugpu_abi_version(void);
@@ -659,7 +660,8 @@ bepugpu_status bepugpu_last_step_ms(bepugpu_context* ctx, int32_t scene, float* 
  * the island-group kernel, which runs first.  Graph mode: the colour-sweep
  * path's phases from events captured into the graph, [0] refresh +
  * ForceUpdater, [1] prestep, [2] warm start, [3] solve iterations, [4]
- * PositionUpdater.  Persistent mode: [3] only, from globaltimer stamps around
+ * PositionUpdater; where one launch does the warm start with the iterations,
+ * [2] is 0 and [3] has both.  Persistent mode: [3] only, from globaltimer stamps around
  * the solve iterations; [0], [1], [2], [4] are 0. */
 bepugpu_status bepugpu_last_step_phase_ms(bepugpu_context* ctx, int32_t scene, float* phase_ms);
 
