@@ -500,6 +500,7 @@ struct Context {
     int batchThreads = 0;  // threads per CTA of batched launches, 0 = from the groups' colour sizes
     uint64_t batchEpoch = 0;  // batched calls so far (Scene::batchStamp)
     int* flowError = nullptr;   // page-locked: a flow launch's wait ran out (flow.cu)
+    int* checkHost = nullptr;   // page-locked: the verdict of an update call's record checks
     int flowBlocksPerSm = 0;
     int colourBlocksPerSm = 0;  // pairs.cu
     std::vector<bepugpu_server*> servers;  // live servers: shut down before the scenes go
