@@ -208,47 +208,101 @@ __global__ void k_colour_positions(const unsigned long long* __restrict__ entrie
 // thread takes its entries in list order and every thread is resident
 // (cooperative launch), so the first uncoloured entry is never waiting; only
 // the colours themselves pass between threads, each read past L1, and a stale
-// one reads as uncoloured.  A wait of kColourSpinLimit polls ends with *err.
-// Bound by the polls' trips through L2 along the longest chain: 82,000 entries
-// of a settling heap in 80 us, where rounds of a launch each took 32 launches
-// and 270 us.
+// one reads as uncoloured.  An entry keeps its place in its walk over the
+// entries before it, so a poll is one trip and each of them is read once, four
+// at a time; only an entry that finds 64 colours taken walks again, 256 colours
+// a walk.  A warp that polls kColourSpinLimit times while no entry anywhere is
+// coloured (*progress) ends with *err.
+// Bound by the polls' trips through L2 along the longest chain.  82,000 entries
+// of a settling heap took 80 us with a walk from the start in every poll (270
+// with a launch for each of 32 rounds); four frames of it 3,450 -> 3,275 us
+// with this walk and the slots' single sort pass.  With a walk from the start
+// 560 bodies that all overlap ran into the limit; they take 0.1 s.
 constexpr int kColourSpinLimit = 1 << 22;
 __device__ __forceinline__ int PeekColour(const int* colour, int i) { return *(volatile const int*)(colour + i); }
+// Up to four entries of `body` from q down: q moves past the coloured ones,
+// their colours go to `take`; false at one that is not coloured.  q is -1 at
+// the body's first entry.
+template <class Take>
+__device__ __forceinline__ bool WalkEntries(const unsigned long long* __restrict__ entries, const int* colour,
+                                            unsigned body, int& q, Take take) {
+    bool mine[4];
+    int c[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const unsigned long long entry = q - u >= 0 ? entries[q - u] : ~0ull;
+        mine[u] = (unsigned)(entry >> 32) == body;
+        c[u] = mine[u] ? PeekColour(colour, (int)(entry & 0xffffffffu)) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        if (!mine[u]) {
+            q = -1;
+            return true;
+        }
+        if (c[u] < 0) return false;
+        take(c[u]);
+        q--;
+    }
+    return true;
+}
 __global__ void k_colour_entries_in_order(const unsigned long long* __restrict__ entries, const int2* __restrict__ at,
-                                          int n, int* colour, int* err) {
+                                          int n, int* colour, int* progress, int* err) {
     const int stride = gridDim.x * blockDim.x;
-    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 - (int)(threadIdx.x & 31) < n; i0 += stride) {
-        const int i = i0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i - (int)(threadIdx.x & 31) < n; i += stride) {
         bool done = i >= n;
         const int2 pos = done ? make_int2(-1, -1) : at[i];
         const int ks[2] = {pos.x, pos.y};
+        unsigned body[2];
+        int q[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            body[e] = ks[e] >= 0 ? (unsigned)(entries[ks[e]] >> 32) : 0u;
+            q[e] = ks[e] - 1;  // below zero: nothing to wait for
+        }
+        unsigned long long used = 0;
+        int seen = -1;
         for (int spins = 0; !__all_sync(0xffffffffu, done); spins++) {
             if (spins > kColourSpinLimit) {
-                *(volatile int*)err = BEPUGPU_TIMEOUT;
-                return;
-            }
-            if (done) continue;
-            int chosen = -1;
-            for (int base = 0; chosen < 0; base += 64) {
-                unsigned long long used = 0;
-                bool ready = true;
-                for (int e = 0; e < 2; e++) {
-                    const int k = ks[e];
-                    if (k < 0) continue;
-                    const unsigned long long body = entries[k] >> 32;
-                    for (int q = k - 1; ready && q >= 0 && (entries[q] >> 32) == body; q--) {
-                        const int c = PeekColour(colour, (int)(entries[q] & 0xffffffffu));
-                        ready = c >= 0;
-                        if (c >= base && c < base + 64) used |= 1ull << (c - base);
-                    }
+                const int now = __shfl_sync(0xffffffffu, *(volatile int*)progress, 0);
+                if (now == seen) {
+                    *(volatile int*)err = BEPUGPU_TIMEOUT;
+                    return;
                 }
-                if (!ready) break;
-                if (used != ~0ull) chosen = base + __ffsll((long long)~used) - 1;
+                seen = now;
+                spins = 0;
             }
-            if (chosen >= 0) {
-                *(volatile int*)(colour + i) = chosen;
-                done = true;
+            int chosen = -1;
+            if (!done) {
+                bool ready = true;
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+                    while (ready && q[e] >= 0)
+                        ready = WalkEntries(entries, colour, body[e], q[e], [&](int c) {
+                            if (c < 64) used |= 1ull << c;
+                        });
+                if (ready && ~used) chosen = __ffsll((long long)~used) - 1;
+                for (int from = 64; ready && chosen < 0; from += 256) {
+                    unsigned long long more[4] = {0, 0, 0, 0};
+#pragma unroll
+                    for (int e = 0; e < 2; e++)
+                        for (int w = ks[e] - 1; w >= 0;)
+                            WalkEntries(entries, colour, body[e], w, [&](int c) {
+                                const unsigned k = (unsigned)(c - from);
+#pragma unroll
+                                for (unsigned g = 0; g < 4; g++)
+                                    if (k >> 6 == g) more[g] |= 1ull << (k & 63);
+                            });
+#pragma unroll
+                    for (int g = 3; g >= 0; g--)
+                        if (~more[g]) chosen = from + 64 * g + __ffsll((long long)~more[g]) - 1;
+                }
+                if (chosen >= 0) {
+                    *(volatile int*)(colour + i) = chosen;
+                    done = true;
+                }
             }
+            if (__any_sync(0xffffffffu, chosen >= 0) && (threadIdx.x & 31) == 0) atomicAdd(progress, 1);
         }
     }
 }
@@ -422,7 +476,7 @@ static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, i
     auto* keys = c.take<unsigned long long>(n);
     auto* at = c.take<int2>(n);
     unsigned* hist = c.take<unsigned>(kSortHistWords);
-    // counts[0, n]: entries per colour; then the highest colour, and the status words
+    // counts[0, n]: entries per colour; then the highest colour, the status and the colouring's progress
     int* counts = c.take<int>((size_t)n + 4);
     int *maxColour = counts + n + 1, *err = counts + n + 2;
     CK(cudaMemsetAsync(counts, 0, sizeof(int) * ((size_t)n + 4), st));
@@ -448,7 +502,7 @@ static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, i
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         CK(cudaLaunchKernelEx(&cfg, k_colour_entries_in_order, (const unsigned long long*)entries, (const int2*)at, n,
-                              out.colour, err));
+                              out.colour, err + 1, err));
     }
     k_colour_count<<<std::min((n + T - 1) / T, ctx->smCount), T, 0, st>>>(out.colour, n, counts, maxColour);
     CK(cudaGetLastError());

@@ -114,3 +114,22 @@ def test_colouring_is_kept_until_asked_for(gpu_context):
     for got, w in zip(sp.colouring(), colour_list(away, m[: n // 2])):
         np.testing.assert_array_equal(got, w)
     sp.close()
+
+
+@pytest.mark.parametrize("n", [34, 560])
+def test_slots_of_one_and_two_digits_of_colours(gpu_context, n):
+    """A cluster's colours number its bodies: one digit up to 512, two beyond."""
+    gpu_context.set_settings(default_settings())
+    b, sh = _cluster(200, n)
+    b, sh = np.resize(b[1:], n), np.resize(sh[1:], n)  # without the ground
+    sp = GpuSpace(gpu_context, b, None, capacity=(n, n * n // 2, 0), shapes=sh)
+    sp.set_materials(np.full((n, 3), 0.5, np.float32))
+    for _ in range(2):
+        assert sp.update_pairs(DT) == n * (n - 1) // 2
+    m, _ = sp.download_constraints()
+    colour, order, k = sp.colouring()
+    c2, o2, k2 = colour_list(b, m)
+    assert k == k2 and (k > 512) == (n > 512)
+    np.testing.assert_array_equal(colour, c2)
+    np.testing.assert_array_equal(order, o2)
+    sp.close()
