@@ -40,7 +40,8 @@ struct SortDigits {
     int shift[10], bits[10];
 };
 constexpr int kSortBlocks = 64, kSortHistWords = kSortBlocks * 512;
-SortDigits SortPlan(int lowFrom, int lowBits, int highBits);
+// The sorted keys end in `keys`; `odd` allows a number of passes that ends in `other`.
+SortDigits SortPlan(int lowFrom, int lowBits, int highBits, bool odd = false);
 int BitsFor(size_t values);  // bits that tell `values` values apart
 cudaError_t RadixSort(const Scene* s, unsigned long long* keys, unsigned long long* other, const unsigned* count,
                       size_t capacity, const SortDigits& digits, unsigned* hist, int* err, cudaStream_t st);

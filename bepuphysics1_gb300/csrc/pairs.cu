@@ -525,8 +525,10 @@ static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, i
     }
     // slots: entries sorted by colour, in list order inside one
     k_slot_keys<<<(n + T - 1) / T, T, 0, st>>>(out.colour, n, keys);
-    CK(RadixSort(s, keys, other, nullptr, (size_t)n, SortPlan(0, 0, BitsFor((size_t)out.colours)), hist, err, st));
-    k_slots<<<(n + T - 1) / T, T, 0, st>>>(keys, n, out.slotOf, out.order);
+    // up to 512 colours are one digit: one pass of about 12 us, which ends in `other`, where an even number took 24
+    const SortDigits byColour = SortPlan(0, 0, BitsFor((size_t)out.colours), true);
+    CK(RadixSort(s, keys, other, nullptr, (size_t)n, byColour, hist, err, st));
+    k_slots<<<(n + T - 1) / T, T, 0, st>>>(byColour.passes & 1 ? other : keys, n, out.slotOf, out.order);
     CK(cudaGetLastError());
     out.offsets.assign(out.colours + 1, 0);
     for (int k = 0; k < out.colours; k++) out.offsets[k + 1] = out.offsets[k] + hc[k];

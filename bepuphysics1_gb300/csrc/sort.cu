@@ -103,11 +103,11 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_sort(unsigned long long*
 
 }  // namespace
 
-SortDigits SortPlan(int lowFrom, int lowBits, int highBits) {
+SortDigits SortPlan(int lowFrom, int lowBits, int highBits, bool odd) {
     SortDigits d{};
     const auto parts = [](int bits) { return (bits + kSortDigitBits - 1) / kSortDigitBits; };
     int low = parts(lowBits), high = parts(highBits);
-    if ((low + high) & 1) (highBits > lowBits ? high : low)++;  // an even number of passes ends in `keys`
+    if (!odd && ((low + high) & 1)) (highBits > lowBits ? high : low)++;  // an even number of passes ends in `keys`
     const auto add = [&](int from, int bits, int n) {
         for (int k = 0; k < n; k++) {
             const int at = bits * k / n, to = bits * (k + 1) / n;
