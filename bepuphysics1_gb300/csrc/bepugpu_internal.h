@@ -360,6 +360,9 @@ struct Scene {
         return g;
     }
     FlowTables flow{};
+    // CTAs of k_flow an SM holds: with the scene, since a server's worker steps
+    // it through a context of its own.
+    int flowBlocksPerSm = 0;
     // flow.cu: the tables from the constraint upload's records (bodies a, b
     // per manifold record), or from update_pairs' sorted (body, entry) keys.
     bepugpu_status UploadFlow(Context* ctx, const int32_t* a, const int32_t* b);
@@ -502,7 +505,6 @@ struct Context {
     uint64_t batchEpoch = 0;  // batched calls so far (Scene::batchStamp)
     int* flowError = nullptr;   // page-locked: a flow launch's wait ran out (flow.cu)
     int* checkHost = nullptr;   // page-locked: the verdict of an update call's record checks
-    int flowBlocksPerSm = 0;
     int colourBlocksPerSm = 0;  // pairs.cu
     std::vector<bepugpu_server*> servers;  // live servers: shut down before the scenes go
     void SetError(const char* fmt, ...);

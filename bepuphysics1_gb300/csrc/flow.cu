@@ -542,8 +542,8 @@ bepugpu_status Scene::UploadFlowChunks(Context* ctx, const std::vector<int2>& gr
     if (!ctx->flowError) {  // once a context, outside any stream capture
         CK(cudaHostAlloc((void**)&ctx->flowError, sizeof(int), cudaHostAllocMapped));
         *ctx->flowError = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->flowBlocksPerSm, k_flow, kFlowThreads, 0));
     }
+    if (!flowBlocksPerSm) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&flowBlocksPerSm, k_flow, kFlowThreads, 0));
     CK(cudaHostGetDevicePointer((void**)&flow.error, ctx->flowError, 0));
     // the ends without a dynamic body keep visit -1
     CK(cudaMemsetAsync(flow.visit, 0xff, sizeof(int2) * slots, stream));
@@ -571,12 +571,17 @@ bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool grou
         f.chunks += f.chunkCount;
         f.chunkCount = f.groupChunkCount;
     }
+    const int resident = s->flowBlocksPerSm * ctx->smCount;
+    if (resident < 1) {
+        ctx->SetError("solve sweeps: no resident CTA (%d an SM of %d)", s->flowBlocksPerSm, ctx->smCount);
+        return BEPUGPU_CUDA_ERROR;
+    }
     const unsigned sweeps = (unsigned)p.iterationLimit + 1;
     k_flow_order<<<(nb + 127) / 128, 128, 0, s->stream>>>(s->m, s->b, f, list, nb, warm ? 0u : 1u, sweeps);
     if (launches) (*launches)++;
     cudaLaunchConfig_t cfg = {};
     // a warp per chunk on its own CTA while the CTAs last
-    cfg.gridDim = dim3((unsigned)std::max(1, std::min(ctx->flowBlocksPerSm * ctx->smCount, f.chunkCount)));
+    cfg.gridDim = dim3((unsigned)std::max(1, std::min(resident, f.chunkCount)));
     cfg.blockDim = dim3(kFlowThreads);
     cfg.stream = s->stream;
     cudaLaunchAttribute attr[1];
