@@ -2019,6 +2019,19 @@ bepugpu_status bepugpu_probe_bounded_wait(bepugpu_context* c, uint32_t limit) {
     return (bepugpu_status)status;
 }
 
+bepugpu_status bepugpu_probe_expired_wait(bepugpu_context* c, int32_t id, uint32_t where) {
+    auto* ctx = reinterpret_cast<Context*>(c);
+    CTX_CHECK(ctx);
+    Scene* s = FindScene(ctx, id);
+    if (!s) return SceneMissing(ctx, id);
+    if (where & ~(uint32_t)BEPUGPU_WAIT_ALL) {
+        ctx->SetError("probe_expired_wait: unknown wait");
+        return BEPUGPU_INVALID_ARGUMENT;
+    }
+    s->expiredWaits |= where;
+    return BEPUGPU_OK;
+}
+
 bepugpu_status bepugpu_download_bodies(bepugpu_context* c, int32_t id, bepugpu_body* bodies, uint32_t n) {
     NvtxRange range("bepugpu_download_bodies");
     auto* ctx = reinterpret_cast<Context*>(c);

@@ -415,6 +415,14 @@ struct Scene {
     bool colouringOnDevice = false;
     int32_t colouringEntries = 0;
     cudaError_t FetchColouring();
+    // bepugpu_probe_expired_wait: the named waits' next status words start as
+    // a wait that ran out leaves them.
+    uint32_t expiredWaits = 0;
+    cudaError_t MarkExpired(int* status, uint32_t where) {
+        if (!(expiredWaits & where)) return cudaSuccess;
+        expiredWaits &= ~where;
+        return cudaMemsetAsync(status, BEPUGPU_TIMEOUT, sizeof(int), stream);
+    }
     std::vector<int32_t> manifoldOffsets;
     std::vector<int32_t> hostSlotOf;
     std::vector<float> hostLinDamp, hostAngDamp, hostLocalM33;

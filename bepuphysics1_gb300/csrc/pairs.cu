@@ -193,13 +193,16 @@ __global__ void k_colour_entries(const int2* __restrict__ ends, int n, BodySoA b
     entries[2 * i + 1] = db ? ((unsigned long long)(unsigned)e.y << 32) | (unsigned)i : ~0ull;
     colour[i] = -1;
 }
+// (entries that a sort left half moved when its wait ran out may name none of
+// the n entries; the colouring then returns at once.)
 __global__ void k_colour_positions(const unsigned long long* __restrict__ entries, int count, const int2* __restrict__ ends,
-                                   int2* at) {
+                                   int n, int2* at) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const unsigned long long key = entries[k];
     if (key == ~0ull) return;
     const int body = (int)(key >> 32), i = (int)(key & 0xffffffffu);
+    if ((unsigned)i >= (unsigned)n) return;
     if (ends[i].x == body) at[i].x = k;
     else at[i].y = k;
 }
@@ -212,7 +215,8 @@ __global__ void k_colour_positions(const unsigned long long* __restrict__ entrie
 // entries before it, so a poll is one trip and each of them is read once, four
 // at a time; only an entry that finds 64 colours taken walks again, 256 colours
 // a walk.  A warp that polls kColourSpinLimit times while no entry anywhere is
-// coloured (*progress) ends with *err.
+// coloured (*progress) ends with *err, and its entries keep colour -1; nothing
+// reads a colour once *err is set.
 // Bound by the polls' trips through L2 along the longest chain.  82,000 entries
 // of a settling heap took 80 us with a walk from the start in every poll (270
 // with a launch for each of 32 rounds); four frames of it 3,450 -> 3,275 us
@@ -248,6 +252,7 @@ __device__ __forceinline__ bool WalkEntries(const unsigned long long* __restrict
 }
 __global__ void k_colour_entries_in_order(const unsigned long long* __restrict__ entries, const int2* __restrict__ at,
                                           int n, int* colour, int* progress, int* err) {
+    if (*(volatile int*)err) return;  // the entries are not sorted
     const int stride = gridDim.x * blockDim.x;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i - (int)(threadIdx.x & 31) < n; i += stride) {
         bool done = i >= n;
@@ -307,10 +312,13 @@ __global__ void k_colour_entries_in_order(const unsigned long long* __restrict__
     }
 }
 // Entries per colour; the colours up to kColourBins through shared memory.
+// Nothing when a wait ran out: some entries then have no colour.
 constexpr int kColourBins = 1024;
-__global__ void k_colour_count(const int* __restrict__ colour, int n, int* counts, int* maxColour) {
+__global__ void k_colour_count(const int* __restrict__ colour, int n, int* counts, int* maxColour,
+                               const int* __restrict__ err) {
     __shared__ int bins[kColourBins];
     __shared__ int top;
+    if (*err) return;
     for (int k = threadIdx.x; k < kColourBins; k += blockDim.x) bins[k] = 0;
     if (threadIdx.x == 0) top = 0;
     __syncthreads();
@@ -480,6 +488,7 @@ static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, i
     int* counts = c.take<int>((size_t)n + 4);
     int *maxColour = counts + n + 1, *err = counts + n + 2;
     CK(cudaMemsetAsync(counts, 0, sizeof(int) * ((size_t)n + 4), st));
+    CK(s->MarkExpired(err, BEPUGPU_WAIT_COLOURING));
     k_colour_entries<<<(n + T - 1) / T, T, 0, st>>>(ends, n, s->b, entries, out.colour);
     // by body alone: the entries start in list order and the sort is stable
     // (entries of no dynamic body have every bit set: one value more than the bodies)
@@ -487,7 +496,7 @@ static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, i
                  st));
     out.entries = entries;
     CK(cudaMemsetAsync(at, 0xff, sizeof(int2) * n, st));
-    k_colour_positions<<<(int)((2 * (size_t)n + T - 1) / T), T, 0, st>>>(entries, 2 * n, ends, at);
+    k_colour_positions<<<(int)((2 * (size_t)n + T - 1) / T), T, 0, st>>>(entries, 2 * n, ends, n, at);
     CK(cudaGetLastError());
     if (!ctx->colourBlocksPerSm)
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->colourBlocksPerSm, k_colour_entries_in_order, T, 0));
@@ -504,7 +513,7 @@ static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, i
         CK(cudaLaunchKernelEx(&cfg, k_colour_entries_in_order, (const unsigned long long*)entries, (const int2*)at, n,
                               out.colour, err + 1, err));
     }
-    k_colour_count<<<std::min((n + T - 1) / T, ctx->smCount), T, 0, st>>>(out.colour, n, counts, maxColour);
+    k_colour_count<<<std::min((n + T - 1) / T, ctx->smCount), T, 0, st>>>(out.colour, n, counts, maxColour, err);
     CK(cudaGetLastError());
     int tail[2];  // the highest colour, the status
     const int listed = std::min(n, kColourBins);

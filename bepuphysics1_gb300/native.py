@@ -162,6 +162,7 @@ GPU_EXPORTS = {
     "bepugpu_update_bodies": (_I, [_P, _I, _P, _U]),
     "bepugpu_check_finite": (_I, [_P, _I, ctypes.POINTER(_I)]),
     "bepugpu_probe_bounded_wait": (_I, [_P, _U]),
+    "bepugpu_probe_expired_wait": (_I, [_P, _I, _U]),
     "bepugpu_download_bodies": (_I, [_P, _I, _P, _U]),
     "bepugpu_download_constraints": (_I, [_P, _I, _P, _U, _P, _U]),
     "bepugpu_get_colouring": (_I, [_P, _I, _P, _P, _U, ctypes.POINTER(_U)]),

@@ -576,6 +576,13 @@ bepugpu_status bepugpu_check_finite(bepugpu_context* ctx, int32_t scene, int32_t
  * host reads.  Returns that status (TIMEOUT when the wait ran out); the
  * context stays usable.  No reference counterpart. */
 bepugpu_status bepugpu_probe_bounded_wait(bepugpu_context* ctx, uint32_t spin_limit);
+/* Tests what follows a device-side wait that ran out, without one: the status
+ * words of the named waits start as such a wait leaves them, once each, the
+ * next time the scene's calls come to them.  Those calls return TIMEOUT and
+ * leave the scene as it was. */
+#define BEPUGPU_WAIT_COLOURING 1u /* bepugpu_update_pairs: the entries' sort and the colouring */
+#define BEPUGPU_WAIT_ALL 1u
+bepugpu_status bepugpu_probe_expired_wait(bepugpu_context* ctx, int32_t scene, uint32_t where);
 
 /* Self-test of the device's float results of the reference's double-precision
  * expressions, which the step computes in double-float FP32 arithmetic and
