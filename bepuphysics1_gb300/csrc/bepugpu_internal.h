@@ -207,6 +207,8 @@ struct FlowTables {
     int chunkCount;
     int groupChunkCount;      // chunks after those: the slots of FlowGroups
 };
+// The chunks of slots that lie colour by colour.
+std::vector<int2> FlowChunks(const std::vector<int32_t>& colourOffsets);
 // The solve sweeps of the slots outside groups, or (groups) of the island
 // groups that FlowGroups names, after their prestep and, with `warm`, their
 // warm start: two launches.
@@ -366,9 +368,9 @@ struct Scene {
     // flow.cu: the tables from the constraint upload's records (bodies a, b
     // per manifold record), or from update_pairs' sorted (body, entry) keys.
     bepugpu_status UploadFlow(Context* ctx, const int32_t* a, const int32_t* b);
-    bepugpu_status UploadFlowChunks(Context* ctx, const std::vector<int2>& groupChunks, size_t slots);
+    bepugpu_status UploadFlowChunks(Context* ctx, const std::vector<int2>& chunks, size_t slots);
     bepugpu_status BuildFlowOnDevice(Context* ctx, const unsigned long long* entries, int count, const int2* ends,
-                                     const int* slots);
+                                     const int* slots, const int* status);
     int SweepColours() const { return manifoldOffsets.empty() ? 0 : (int)manifoldOffsets.size() - 1; }
     uint32_t maxBodies = 0, maxManifolds = 0, maxJoints = 0;
     DeviceHeap* heap = nullptr;     // the owning context's heap: arena and staging blocks

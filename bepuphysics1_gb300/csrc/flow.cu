@@ -442,14 +442,15 @@ __global__ void __launch_bounds__(kFlowThreads, 4) k_flow(ManifoldSoA m, BodySoA
 
 // update_pairs' side of the tables, from its (dynamic body, entry) keys
 // sorted by body: where each body's entries start, and the entries as
-// slot << 1 | end in slot order.
+// slot << 1 | end in slot order.  Nothing when the slots' sort gave up (*err).
 __device__ __forceinline__ int BodyOfEntry(const unsigned long long* __restrict__ entries, int count, int bodies, int k) {
     return k < 0 ? -1 : (k < count && entries[k] != ~0ull ? (int)(entries[k] >> 32) : bodies);
 }
 __global__ void k_flow_csr(const unsigned long long* __restrict__ entries, int count, int bodies,
-                           const int2* __restrict__ ends, const int* __restrict__ slotOf, FlowTables f) {
+                           const int2* __restrict__ ends, const int* __restrict__ slotOf, FlowTables f,
+                           const int* __restrict__ err) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k > count) return;
+    if (k > count || *err) return;
     // the bodies after the previous entry's, up to this one's, start here
     const int body = BodyOfEntry(entries, count, bodies, k);
     for (int i = BodyOfEntry(entries, count, bodies, k - 1) + 1; i <= body; i++) f.csrBegin[i] = k;
@@ -530,14 +531,17 @@ bepugpu_status Scene::UploadFlow(Context* ctx, const int32_t* a, const int32_t* 
         }
         if (!any) break;
     }
-    return UploadFlowChunks(ctx, groupChunks, groupPlan.slotOf.size());
-}
-
-bepugpu_status Scene::UploadFlowChunks(Context* ctx, const std::vector<int2>& groupChunks, size_t slots) {
     std::vector<int2> chunks = FlowChunks(manifoldOffsets);
     flow.chunkCount = (int)chunks.size();
     flow.groupChunkCount = (int)groupChunks.size();
     chunks.insert(chunks.end(), groupChunks.begin(), groupChunks.end());
+    bepugpu_status st = UploadFlowChunks(ctx, chunks, groupPlan.slotOf.size());
+    CK(cudaStreamSynchronize(stream));
+    return st;
+}
+
+// The caller keeps the chunks until the stream has passed the copy.
+bepugpu_status Scene::UploadFlowChunks(Context* ctx, const std::vector<int2>& chunks, size_t slots) {
     if (chunks.empty()) return BEPUGPU_OK;
     if (!ctx->flowError) {  // once a context, outside any stream capture
         CK(cudaHostAlloc((void**)&ctx->flowError, sizeof(int), cudaHostAllocMapped));
@@ -548,15 +552,14 @@ bepugpu_status Scene::UploadFlowChunks(Context* ctx, const std::vector<int2>& gr
     // the ends without a dynamic body keep visit -1
     CK(cudaMemsetAsync(flow.visit, 0xff, sizeof(int2) * slots, stream));
     CK(cudaMemcpyAsync(flow.chunks, chunks.data(), sizeof(int2) * chunks.size(), cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
     return BEPUGPU_OK;
 }
 
 bepugpu_status Scene::BuildFlowOnDevice(Context* ctx, const unsigned long long* entries, int count, const int2* ends,
-                                        const int* slots) {
-    k_flow_csr<<<(count + 1 + 255) / 256, 256, 0, stream>>>(entries, count, b.count, ends, slots, flow);
+                                        const int* slots, const int* status) {
+    k_flow_csr<<<(count + 1 + 255) / 256, 256, 0, stream>>>(entries, count, b.count, ends, slots, flow, status);
     CK(cudaGetLastError());
-    return UploadFlowChunks(ctx, {}, count / 2);
+    return BEPUGPU_OK;
 }
 
 bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool groups, bool warm, int* launches) {

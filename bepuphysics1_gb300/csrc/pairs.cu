@@ -337,10 +337,12 @@ __global__ void k_slot_keys(const int* __restrict__ colour, int n, unsigned long
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) keys[i] = ((unsigned long long)(unsigned)colour[i] << 32) | (unsigned)i;
 }
+// (keys of a sort whose wait ran out may name none of the n entries)
 __global__ void k_slots(const unsigned long long* __restrict__ keys, int n, int* slotOf, int* order) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int i = (int)(keys[k] & 0xffffffffu);
+    if ((unsigned)i >= (unsigned)n) return;
     slotOf[i] = k;
     order[k] = i;
 }
@@ -348,10 +350,11 @@ __global__ void k_slots(const unsigned long long* __restrict__ keys, int n, int*
 // A record's input lanes at its new slot of the scratch copy (capacity n):
 // a kept record's lanes as a download and upload would carry them, a new
 // record's empty with the blended material (MaterialManager.cs:77-85).
+// Nothing when the slots' sort gave up: not every entry has a slot then.
 __global__ void k_move_lanes(ManifoldSoA m, NewRecords rec, const int* __restrict__ newSlot, int n,
-                             const float4* __restrict__ material, float4* scratch) {
+                             const float4* __restrict__ material, float4* scratch, const int* __restrict__ err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n || *err) return;
     const int ns = newSlot[i], os = rec.oldSlot[i], cap = m.capacity;
     const int2 e = rec.ends[i];
     const uint32_t flags = rec.flags[i];
@@ -386,10 +389,19 @@ __global__ void k_move_lanes(ManifoldSoA m, NewRecords rec, const int* __restric
     at(19) = make_float4(count > 0 ? f.x : 0.f, count > 0 ? f.y : 0.f, count > 0 ? f.z : 0.f, f.w);
     at(20) = make_float4(ax.x, ax.y, ax.z, 0.f);
 }
-// The scratch copy back into the scene's lanes, slots [0, n).
-__global__ void k_lanes_back(ManifoldSoA m, const float4* __restrict__ scratch, int n, int32_t* genSlots) {
+// The scratch copy back into the scene's lanes, slots [0, n), and the entries'
+// slots, colours and order beside them; nothing when the slots' sort gave up.
+struct KeptColouring {
+    const int *slotOf, *colour, *order;  // scratch
+    int *sceneSlotOf, *colouring;        // the scene's: slots; colours, then order
+};
+__global__ void k_lanes_back(ManifoldSoA m, const float4* __restrict__ scratch, int n, int32_t* genSlots,
+                             KeptColouring keep, const int* __restrict__ err) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
+    if (s >= n || *err) return;
+    keep.sceneSlotOf[s] = keep.slotOf[s];
+    keep.colouring[s] = keep.colour[s];
+    keep.colouring[n + s] = keep.order[s];
     const int cap = m.capacity;
     auto L = [&](int lane) { return scratch[(size_t)lane * n + s]; };
     const float4 h = L(0);
@@ -466,9 +478,18 @@ struct DeviceColouring {
     int* order;
     int* slotOf;
     const unsigned long long* entries = nullptr;  // (dynamic body << 32 | entry), sorted, 2 n of them (~0: none)
+    const int* status = nullptr;  // device: set when the slots' sort gave up (its end is not waited for)
     int colours = 0;
     std::vector<int32_t> offsets;
 };
+
+// A sort's or the colouring's wait ran out: blocks that gave up leave the
+// barrier counter where it was, so it starts again from zero.
+static bepugpu_status GaveUp(Context* ctx, Scene* s, const char* what) {
+    CK(cudaMemsetAsync(s->BarrierCounter(), 0, sizeof(unsigned), s->stream));
+    ctx->SetError("update_pairs: %s did not finish", what);
+    return BEPUGPU_TIMEOUT;
+}
 
 static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, int n, Carve& c, DeviceColouring& out) {
     const cudaStream_t st = s->stream;
@@ -521,11 +542,7 @@ static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, i
     CK(cudaMemcpyAsync(tail, maxColour, sizeof(tail), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(hc.data(), counts, sizeof(int) * listed, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (tail[1]) {
-        cudaMemsetAsync(s->BarrierCounter(), 0, sizeof(unsigned), st);
-        ctx->SetError("update_pairs: the colouring did not finish");
-        return BEPUGPU_TIMEOUT;
-    }
+    if (tail[1]) return GaveUp(ctx, s, "the colouring");
     out.colours = tail[0] + 1;
     if (out.colours > listed) {
         hc.resize(out.colours);
@@ -536,6 +553,8 @@ static bepugpu_status ColourOnDevice(Context* ctx, Scene* s, const int2* ends, i
     k_slot_keys<<<(n + T - 1) / T, T, 0, st>>>(out.colour, n, keys);
     // up to 512 colours are one digit: one pass of about 12 us, which ends in `other`, where an even number took 24
     const SortDigits byColour = SortPlan(0, 0, BitsFor((size_t)out.colours), true);
+    out.status = err;
+    CK(s->MarkExpired(err, BEPUGPU_WAIT_SLOTS));
     CK(RadixSort(s, keys, other, nullptr, (size_t)n, byColour, hist, err, st));
     k_slots<<<(n + T - 1) / T, T, 0, st>>>(byColour.passes & 1 ? other : keys, n, out.slotOf, out.order);
     CK(cudaGetLastError());
@@ -676,14 +695,22 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
         ctx->SetError("update_pairs: scratch overrun (%zu of %zu bytes)", cv.used, P.blockBytes);
         return BEPUGPU_CUDA_ERROR;
     }
+    // Everything so far went to scratch.  The scene changes from here on: in
+    // kernels that look at the status themselves, and on the host and in the
+    // tables it uploads once the status has been read.
+    const std::vector<int2> chunks = FlowChunks(col.offsets);
     if (n) {
-        k_move_lanes<<<(n + T - 1) / T, T, 0, st>>>(s->m, rec, col.slotOf, n, P.material, scratch);
-        k_lanes_back<<<(n + T - 1) / T, T, 0, st>>>(s->m, scratch, n, s->genSlotsDev);
-        CK(cudaMemcpyAsync(s->slotOf, col.slotOf, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemcpyAsync(P.colouring, col.colour, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemcpyAsync(P.colouring + n, col.order, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
+        k_move_lanes<<<(n + T - 1) / T, T, 0, st>>>(s->m, rec, col.slotOf, n, P.material, scratch, col.status);
+        const KeptColouring keep{col.slotOf, col.colour, col.order, s->slotOf, P.colouring};
+        k_lanes_back<<<(n + T - 1) / T, T, 0, st>>>(s->m, scratch, n, s->genSlotsDev, keep, col.status);
+        CK(cudaGetLastError());
+        bepugpu_status fs = s->BuildFlowOnDevice(ctx, col.entries, 2 * n, rec.ends, col.slotOf, col.status);
+        if (fs != BEPUGPU_OK) return fs;
+        int status = 0;
+        CK(cudaMemcpyAsync(&status, col.status, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        if (status) return GaveUp(ctx, s, "the slots' sort");
     }
-    CK(cudaGetLastError());
     // the scene's bookkeeping: every manifold on the colour-sweep path
     if (s->islands) ReleaseIslands(s);
     const bool hadGroups = !s->groupPlan.groups.empty();
@@ -698,11 +725,10 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
     s->colouringOnDevice = true;
     s->colouringEntries = n;
     s->manifoldOffsets = col.offsets;
-    s->flow.chunkCount = s->flow.groupChunkCount = 0;
-    if (n) {
-        bepugpu_status fs = s->BuildFlowOnDevice(ctx, col.entries, 2 * n, rec.ends, col.slotOf);
-        if (fs != BEPUGPU_OK) return fs;
-    }
+    s->flow.chunkCount = (int)chunks.size();
+    s->flow.groupChunkCount = 0;
+    bepugpu_status fs = s->UploadFlowChunks(ctx, chunks, (size_t)n);
+    if (fs != BEPUGPU_OK) return fs;
     s->jointOffsets.assign(col.colours + 1, 0);
     s->m.count = n;
     s->generatedCount = n;

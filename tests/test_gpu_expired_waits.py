@@ -14,7 +14,7 @@ from parity import DT
 
 pytestmark = pytest.mark.gpu
 FLAGS = N.STEP_ALL | N.STEP_COLLIDE
-COLOURING = 1
+COLOURING, SLOTS = 1, 2
 
 
 def _expire(sp, where):
@@ -55,7 +55,7 @@ def _frames(sp, n):
         sp.step(DT, FLAGS)
 
 
-@pytest.mark.parametrize("where", [COLOURING])
+@pytest.mark.parametrize("where", [COLOURING, SLOTS])
 def test_pair_update_that_gave_up(gpu_context, where):
     gpu_context.set_settings(default_settings())
     sp, twin = _heap(gpu_context, 21), _heap(gpu_context, 21)
