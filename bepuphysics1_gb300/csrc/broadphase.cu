@@ -174,10 +174,12 @@ __device__ __forceinline__ void Report(int a, int b, unsigned long long* __restr
 
 // Threads over the sorted cell entries: each tests the later entries of its
 // cell.  A run of entries that agree in the upper `sortedBits` code bits may
-// hold several cells.
+// hold several cells.  Nothing when the entries' sort gave up: a key that it
+// left half moved may name no body.
 __global__ void k_bp_cell_pairs(const unsigned long long* __restrict__ keys, const float4* __restrict__ lo,
                                 const float4* __restrict__ hi, unsigned* __restrict__ words, int sortedBits,
                                 unsigned long long* __restrict__ pairs, unsigned capacity) {
+    if (words[kWError]) return;
     const unsigned entries = words[kWEntries];
     const float inv = 1.f / CellSize(words);
     const int drop = kCellCodeBits - sortedBits;
@@ -319,6 +321,7 @@ bepugpu_status RunBroadPhase(Context* ctx, Scene* s, float dt, unsigned& found) 
     const int cellBits = std::min(kCellCodeBits, std::max(12, BitsFor((size_t)4 * n)));
     const int bodyBits = BitsFor((size_t)n);
     CK(cudaMemsetAsync(bp.words, 0, sizeof(unsigned) * kWords, st));
+    CK(s->MarkExpired(err, BEPUGPU_WAIT_BROAD_PHASE));
     k_bp_boxes<<<(n + 255) / 256, 256, 0, st>>>(s->b, s->shape, dt, bp.lo, bp.hi, bp.words);
     k_bp_cells<<<(n + 255) / 256, 256, 0, st>>>(bp.lo, bp.hi, n, bp.words, bp.keys, (unsigned)bp.keyCap, bp.wide,
                                                (unsigned)wideCap);
@@ -341,7 +344,7 @@ bepugpu_status RunBroadPhase(Context* ctx, Scene* s, float dt, unsigned& found) 
         CK(cudaMemcpyAsync(w, bp.words, sizeof(w), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         if (w[kWError]) {
-            cudaMemsetAsync(s->BarrierCounter(), 0, sizeof(unsigned), st);
+            CK(cudaMemsetAsync(s->BarrierCounter(), 0, sizeof(unsigned), st));
             ctx->SetError("broad phase: a sort's grid barrier wait ran out");
             return BEPUGPU_TIMEOUT;
         }

@@ -14,7 +14,7 @@ from parity import DT
 
 pytestmark = pytest.mark.gpu
 FLAGS = N.STEP_ALL | N.STEP_COLLIDE
-COLOURING, SLOTS = 1, 2
+COLOURING, SLOTS, BROAD_PHASE = 1, 2, 4
 
 
 def _expire(sp, where):
@@ -29,11 +29,12 @@ def _timeout(call, *args):
 
 
 def _heap(ctx, seed):
-    """A dropped pile after a few frames, its pairs kept on the device."""
-    b, sh, fr = scenes.dropped_pile(nx=12, ny=6, nz=12, seed=seed)
+    """Overlapping layers of boxes after a few frames: pairs for several blocks
+    of a sort, kept on the device."""
+    b, sh, fr = scenes.dropped_pile(nx=12, ny=8, nz=12, drop_spacing=0.7, seed=seed)
     sp = GpuSpace(ctx, b, None, capacity=(len(b), 16 * len(b), 0), shapes=sh)
     sp.set_materials(np.stack([fr, fr, np.zeros_like(fr)], 1))
-    for _ in range(30):
+    for _ in range(10):
         sp.update_pairs(float(DT))
         sp.step(DT, FLAGS)
     return sp
@@ -55,14 +56,14 @@ def _frames(sp, n):
         sp.step(DT, FLAGS)
 
 
-@pytest.mark.parametrize("where", [COLOURING, SLOTS])
+@pytest.mark.parametrize("where", [COLOURING, SLOTS, BROAD_PHASE])
 def test_pair_update_that_gave_up(gpu_context, where):
     gpu_context.set_settings(default_settings())
     sp, twin = _heap(gpu_context, 21), _heap(gpu_context, 21)
     before = _state(sp)
     for _ in range(2):
         _expire(sp, where)
-        assert "update_pairs" in _timeout(sp.update_pairs, float(DT))
+        assert ("broad phase" if where == BROAD_PHASE else "update_pairs") in _timeout(sp.update_pairs, float(DT))
         _same(_state(sp), before)
     # the scene steps on with the list it has, and the next update is whole
     sp.step(DT, FLAGS)
@@ -73,6 +74,18 @@ def test_pair_update_that_gave_up(gpu_context, where):
     _same(_state(sp), _state(twin))
     sp.close()
     twin.close()
+
+
+def test_broad_phase_that_gave_up(gpu_context):
+    gpu_context.set_settings(default_settings())
+    sp = _heap(gpu_context, 22)
+    want = sp.broad_phase(float(DT))
+    assert len(want) > 0
+    for _ in range(2):
+        _expire(sp, BROAD_PHASE)
+        _timeout(sp.broad_phase, float(DT))
+        np.testing.assert_array_equal(sp.broad_phase(float(DT)), want)
+    sp.close()
 
 
 def test_unknown_waits_are_refused(gpu_context):
