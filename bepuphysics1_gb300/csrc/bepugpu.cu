@@ -2028,7 +2028,11 @@ bepugpu_status bepugpu_probe_expired_wait(bepugpu_context* c, int32_t id, uint32
         ctx->SetError("probe_expired_wait: unknown wait");
         return BEPUGPU_INVALID_ARGUMENT;
     }
-    s->expiredWaits |= where;
+    if (where & BEPUGPU_WAIT_PERSISTENT) {
+        CK(cudaMemsetAsync(s->BarrierCounter(), 1, sizeof(unsigned int), s->stream));
+        CK(cudaMemsetAsync(s->ErrorWord(), BEPUGPU_TIMEOUT, sizeof(int), s->stream));
+    }
+    s->expiredWaits |= where & ~(uint32_t)BEPUGPU_WAIT_PERSISTENT;
     return BEPUGPU_OK;
 }
 

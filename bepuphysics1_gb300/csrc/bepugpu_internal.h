@@ -34,7 +34,8 @@ const unsigned long long* BroadPhasePairs(const Scene* s);
 // lowBits from bit lowFrom on, then highBits from bit 32 on -- in one
 // cooperative launch.  `count` (device, null: capacity) keys, at most
 // `capacity`; `other` as large as `keys`; hist kSortHistWords words; *err is
-// set to TIMEOUT when a barrier's wait ran out.  Uses the scene's barrier words.
+// set to TIMEOUT when a barrier's wait ran out.  Uses the scene's SortCounter,
+// which whoever reads that status puts back to zero.
 struct SortDigits {
     int passes;
     int shift[10], bits[10];
@@ -274,10 +275,13 @@ struct KinematicState {
 
 // Layout of a scene's device scratch block (kScratchBytes): grid barrier
 // arrival counter, barrier generation, error word, record-check words, census
-// accumulators, timer stamps -- each on its own 128-byte line.
+// accumulators, timer stamps, the sorts' barrier counter -- each on its own
+// 128-byte line.  The sorts rely on a counter that starts at zero, so they
+// share none with the persistent step, which may leave its own anywhere when
+// its wait runs out.
 constexpr size_t kScratchBytes = 1024;
 constexpr size_t kBarrierCounterAt = 0, kBarrierGenerationAt = 128, kErrorAt = 256, kCheckAt = 384, kCensusAt = 512,
-                 kStampsAt = 640;
+                 kStampsAt = 640, kSortCounterAt = 768;
 
 // Byte offsets of a scene's device arrays inside its arena.
 struct ArenaLayout {
@@ -299,6 +303,7 @@ struct Scene {
     Server* server = nullptr;     // a server owns the scene's residency and steps (serve.cu)
     unsigned int* BarrierCounter() const { return (unsigned int*)((char*)counter + kBarrierCounterAt); }
     unsigned int* BarrierGeneration() const { return (unsigned int*)((char*)counter + kBarrierGenerationAt); }
+    unsigned int* SortCounter() const { return (unsigned int*)((char*)counter + kSortCounterAt); }
     int* ErrorWord() const { return (int*)((char*)counter + kErrorAt); }
     unsigned long long* Census() const { return (unsigned long long*)((char*)counter + kCensusAt); }
     int* CheckWords() const { return (int*)((char*)counter + kCheckAt); }  // record checks of update calls

@@ -344,7 +344,7 @@ bepugpu_status RunBroadPhase(Context* ctx, Scene* s, float dt, unsigned& found) 
         CK(cudaMemcpyAsync(w, bp.words, sizeof(w), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
         if (w[kWError]) {
-            CK(cudaMemsetAsync(s->BarrierCounter(), 0, sizeof(unsigned), st));
+            CK(cudaMemsetAsync(s->SortCounter(), 0, sizeof(unsigned), st));
             ctx->SetError("broad phase: a sort's grid barrier wait ran out");
             return BEPUGPU_TIMEOUT;
         }

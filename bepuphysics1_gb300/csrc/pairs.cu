@@ -486,7 +486,7 @@ struct DeviceColouring {
 // A sort's or the colouring's wait ran out: blocks that gave up leave the
 // barrier counter where it was, so it starts again from zero.
 static bepugpu_status GaveUp(Context* ctx, Scene* s, const char* what) {
-    CK(cudaMemsetAsync(s->BarrierCounter(), 0, sizeof(unsigned), s->stream));
+    CK(cudaMemsetAsync(s->SortCounter(), 0, sizeof(unsigned), s->stream));
     ctx->SetError("update_pairs: %s did not finish", what);
     return BEPUGPU_TIMEOUT;
 }

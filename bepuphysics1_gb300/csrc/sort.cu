@@ -138,7 +138,7 @@ cudaError_t RadixSort(const Scene* s, unsigned long long* keys, unsigned long lo
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_radix_sort, keys, other, count, (unsigned)capacity, digits, hist,
-                              s->BarrierCounter(), err);
+                              s->SortCounter(), err);
 }
 
 }  // namespace bepugpu

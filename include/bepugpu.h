@@ -583,7 +583,9 @@ bepugpu_status bepugpu_probe_bounded_wait(bepugpu_context* ctx, uint32_t spin_li
 #define BEPUGPU_WAIT_COLOURING 1u /* bepugpu_update_pairs: the entries' sort and the colouring */
 #define BEPUGPU_WAIT_SLOTS 2u     /* bepugpu_update_pairs: the sort of the entries into slots */
 #define BEPUGPU_WAIT_BROAD_PHASE 4u /* the broad phase's sorts (bepugpu_broad_phase, bepugpu_update_pairs) */
-#define BEPUGPU_WAIT_ALL 7u
+#define BEPUGPU_WAIT_PERSISTENT 8u /* a persistent step before this call: its barrier and status words at once,
+                                      for bepugpu_synchronize to report */
+#define BEPUGPU_WAIT_ALL 15u
 bepugpu_status bepugpu_probe_expired_wait(bepugpu_context* ctx, int32_t scene, uint32_t where);
 
 /* Self-test of the device's float results of the reference's double-precision

@@ -14,7 +14,7 @@ from parity import DT
 
 pytestmark = pytest.mark.gpu
 FLAGS = N.STEP_ALL | N.STEP_COLLIDE
-COLOURING, SLOTS, BROAD_PHASE = 1, 2, 4
+COLOURING, SLOTS, BROAD_PHASE, PERSISTENT = 1, 2, 4, 8
 
 
 def _expire(sp, where):
@@ -86,6 +86,23 @@ def test_broad_phase_that_gave_up(gpu_context):
         _timeout(sp.broad_phase, float(DT))
         np.testing.assert_array_equal(sp.broad_phase(float(DT)), want)
     sp.close()
+
+
+def test_sorts_after_a_persistent_step_that_gave_up(gpu_context):
+    gpu_context.set_settings(default_settings())
+    sp, twin = _heap(gpu_context, 23), _heap(gpu_context, 23)
+    sp.ctx.check(sp.ctx.lib.bepugpu_set_solve_mode(sp.ctx.handle, sp.id, N.MODE_PERSISTENT))
+    _expire(sp, PERSISTENT)
+    _same(_state(sp), _state(twin))
+    assert sp.update_pairs(float(DT)) == twin.update_pairs(float(DT))
+    _same(_state(sp), _state(twin))
+    _timeout(sp.ctx.synchronize)
+    _frames(sp, 3)
+    _frames(twin, 3)
+    sp.ctx.synchronize()
+    _same(_state(sp), _state(twin))
+    sp.close()
+    twin.close()
 
 
 def test_unknown_waits_are_refused(gpu_context):
