@@ -368,7 +368,9 @@ static bepugpu_status BatchStep(bepugpu_context* c, const int32_t* scenes, const
         return BEPUGPU_CUDA_ERROR;
     }
     uint32_t launches = bt.launches;
-    // Scenes outside the batched launch take their own path, step by step.
+    // Scenes outside the batched launch take their own path, step by step; one
+    // whose sweeps gave up is reported when every scene has advanced.
+    bepugpu_status late = BEPUGPU_OK;
     for (uint32_t i = 0; i < count; i++) {
         Scene* s = list[i];
         if (ready[i]) {
@@ -385,10 +387,11 @@ static bepugpu_status BatchStep(bepugpu_context* c, const int32_t* scenes, const
             return BEPUGPU_CUDA_ERROR;
         }
         s->asyncPending = false;
+        if (FlowStatus(ctx, s) != BEPUGPU_OK) late = BEPUGPU_TIMEOUT;
     }
     ctx->lastLaunches = launches;
     cudaEventElapsedTime(&ctx->lastMs, bt.ev0, bt.ev1);
-    return BEPUGPU_OK;
+    return late;
 }
 
 extern "C" bepugpu_status bepugpu_batch_step(bepugpu_context* c, const int32_t* scenes, uint32_t count, float dt,

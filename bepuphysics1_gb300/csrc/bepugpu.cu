@@ -734,6 +734,7 @@ Scene::~Scene() {
     ReleaseBroadPhase(this);
     ReleaseIslands(this);
     ReleasePairs(this);
+    if (words) words->Give(flowStatus);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -1434,7 +1435,6 @@ void bepugpu_destroy(bepugpu_context* c) {
     ShutdownServers(ctx);  // their workers step these scenes
     ctx->batch.reset();
     ctx->scenes.clear();
-    if (ctx->flowError) cudaFreeHost(ctx->flowError);
     if (ctx->checkHost) cudaFreeHost(ctx->checkHost);
     delete ctx;
 }
@@ -1480,7 +1480,15 @@ bepugpu_status bepugpu_synchronize(bepugpu_context* c) {
             }
         }
     }
-    return FlowStatus(ctx);
+    // every scene's sweeps, the one with the lowest id by name; a server reads its own scenes'
+    Scene* lowest = nullptr;
+    for (auto& kv : ctx->scenes) {
+        Scene* s = kv.second.get();
+        if (!s->server && FlowStatus(ctx, s) != BEPUGPU_OK && (!lowest || s->id < lowest->id)) lowest = s;
+    }
+    if (!lowest) return BEPUGPU_OK;
+    ctx->SetError("solve sweeps of scene %d: a wait for an earlier visit ran out", lowest->id);
+    return BEPUGPU_TIMEOUT;
 }
 
 bepugpu_status bepugpu_scene_create(bepugpu_context* c, uint32_t nb, uint32_t nm, uint32_t nj, int32_t* out) {
@@ -1493,6 +1501,7 @@ bepugpu_status bepugpu_scene_create(bepugpu_context* c, uint32_t nb, uint32_t nm
     }
     auto s = std::make_unique<Scene>();
     s->heap = ctx->heap.get();
+    s->words = &ctx->words;
     bepugpu_status st = s->Allocate(ctx, nb, nm, nj);
     if (st != BEPUGPU_OK) return st;
     int32_t id = ctx->nextScene++;
@@ -1783,7 +1792,7 @@ bepugpu_status bepugpu_step_host(bepugpu_context* c, int32_t id, bepugpu_body* b
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s->stream));
     s->asyncPending = false;
-    return BEPUGPU_OK;
+    return FlowStatus(ctx, s);
 }
 
 namespace {
@@ -1886,7 +1895,7 @@ bepugpu_status bepugpu_step_state(bepugpu_context* c, int32_t id, bepugpu_body_s
     st = QueueStateDownload(ctx, s, bodies, nb, man, nm);
     CK(cudaStreamSynchronize(s->stream));
     s->asyncPending = false;
-    return st == BEPUGPU_OK ? FlowStatus(ctx) : st;
+    return st == BEPUGPU_OK ? FlowStatus(ctx, s) : st;
 }
 
 bepugpu_status bepugpu_download_state(bepugpu_context* c, int32_t id, bepugpu_body_state* bodies, uint32_t nb,
@@ -1904,7 +1913,7 @@ bepugpu_status bepugpu_download_state(bepugpu_context* c, int32_t id, bepugpu_bo
     }
     st = QueueStateDownload(ctx, s, bodies, nb, man, nm);
     CK(cudaStreamSynchronize(s->stream));
-    return st == BEPUGPU_OK ? FlowStatus(ctx) : st;
+    return st == BEPUGPU_OK ? FlowStatus(ctx, s) : st;
 }
 
 bepugpu_status bepugpu_update_bodies(bepugpu_context* c, int32_t id, const bepugpu_body* bodies, uint32_t n) {
@@ -2032,7 +2041,14 @@ bepugpu_status bepugpu_probe_expired_wait(bepugpu_context* c, int32_t id, uint32
         CK(cudaMemsetAsync(s->BarrierCounter(), 1, sizeof(unsigned int), s->stream));
         CK(cudaMemsetAsync(s->ErrorWord(), BEPUGPU_TIMEOUT, sizeof(int), s->stream));
     }
-    s->expiredWaits |= where & ~(uint32_t)BEPUGPU_WAIT_PERSISTENT;
+    if (where & BEPUGPU_WAIT_SWEEPS) {
+        if (!s->flowStatus) {
+            ctx->SetError("probe_expired_wait: the scene has no barrier-free sweeps");
+            return BEPUGPU_INVALID_OPERATION;
+        }
+        *(volatile int*)s->flowStatus = BEPUGPU_TIMEOUT;
+    }
+    s->expiredWaits |= where & ~(uint32_t)(BEPUGPU_WAIT_PERSISTENT | BEPUGPU_WAIT_SWEEPS);
     return BEPUGPU_OK;
 }
 
@@ -2051,7 +2067,7 @@ bepugpu_status bepugpu_download_bodies(bepugpu_context* c, int32_t id, bepugpu_b
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(bodies, s->bodyRecords, sizeof(bepugpu_body) * n, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    return BEPUGPU_OK;
+    return FlowStatus(ctx, s);
 }
 
 bepugpu_status bepugpu_download_constraints(bepugpu_context* c, int32_t id, bepugpu_manifold* man, uint32_t nm,
@@ -2069,7 +2085,7 @@ bepugpu_status bepugpu_download_constraints(bepugpu_context* c, int32_t id, bepu
         bepugpu_status jst = DownloadJoints(ctx, s, joints, nj);
         if (jst != BEPUGPU_OK) return jst;
     }
-    if (!nm) return BEPUGPU_OK;
+    if (!nm) return FlowStatus(ctx, s);
     // Whole records are rebuilt on the device in record order and copied
     // straight into the caller's array (their fields are the uploaded ones,
     // the state fields current; `reserved` comes back 0).
@@ -2078,7 +2094,7 @@ bepugpu_status bepugpu_download_constraints(bepugpu_context* c, int32_t id, bepu
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(man, s->staging, sizeof(bepugpu_manifold) * nm, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    return BEPUGPU_OK;
+    return FlowStatus(ctx, s);
 }
 
 bepugpu_status bepugpu_get_colouring(bepugpu_context* c, int32_t id, int32_t* colour, int32_t* order, uint32_t n,

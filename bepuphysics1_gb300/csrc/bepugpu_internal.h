@@ -108,6 +108,24 @@ class DeviceHeap {
     int holds_ = 0;
 };
 
+// Page-locked words that kernels leave a status in and the host reads without a
+// copy, 1,024 to a page.  Used by the caller's thread alone; a word's scene
+// stays with it.
+class StatusWords {
+  public:
+    StatusWords() = default;
+    StatusWords(const StatusWords&) = delete;
+    StatusWords& operator=(const StatusWords&) = delete;
+    ~StatusWords();
+    cudaError_t Take(int** word);  // zero
+    void Give(int* word) {
+        if (word) free_.push_back(word);
+    }
+
+  private:
+    std::vector<int*> pages_, free_;
+};
+
 StepParams MakeParams(const bepugpu_settings& s, float dt);
 
 // An NVTX range for the duration of a scope: the host-side phases (steps,
@@ -204,7 +222,7 @@ struct FlowTables {
     int32_t* csrBegin;        // per body: its entries of csr, bodies + 1
     int32_t* csr;             // slot << 1 | end (0 A, 1 B), ascending
     float4 *lin, *ang;        // per body: velocity, w = visits so far (bits)
-    int* error;
+    int* error;               // Scene::flowStatus, as the device sees it
     int chunkCount;
     int groupChunkCount;      // chunks after those: the slots of FlowGroups
 };
@@ -223,8 +241,9 @@ bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool grou
 // smaller scenes the colours' launches cost more (82,000 manifolds of 16
 // colours: 45 us a step).
 constexpr int kFlowWarmChunks = 9728;
-// TIMEOUT when a wait of a finished flow launch ran out (and clears it).
-bepugpu_status FlowStatus(Context* ctx);
+// TIMEOUT when a wait of one of the scene's finished flow launches ran out (and
+// clears it).  For each call that hands the scene's results out.
+bepugpu_status FlowStatus(Context* ctx, Scene* s);
 // Joints (joints.cu): record checks, upload into the scene's joint slots, and
 // the accumulated impulses back into records.
 bepugpu_status CheckJointRecords(Context* ctx, const bepugpu_joint* joints, uint32_t nj, int32_t bodies);
@@ -370,6 +389,8 @@ struct Scene {
     // CTAs of k_flow an SM holds: with the scene, since a server's worker steps
     // it through a context of its own.
     int flowBlocksPerSm = 0;
+    StatusWords* words = nullptr;  // the owning context's
+    int* flowStatus = nullptr;     // page-locked: a wait of the scene's sweeps ran out (FlowStatus)
     // flow.cu: the tables from the constraint upload's records (bodies a, b
     // per manifold record), or from update_pairs' sorted (body, entry) keys.
     bepugpu_status UploadFlow(Context* ctx, const int32_t* a, const int32_t* b);
@@ -510,7 +531,8 @@ struct Context {
     int smCount = 0;
     bepugpu_settings settings{};
     std::string lastError;
-    std::unique_ptr<DeviceHeap> heap;  // declared before the scenes: it outlives them
+    std::unique_ptr<DeviceHeap> heap;  // declared before the scenes: they outlive them
+    StatusWords words;
     std::unordered_map<int32_t, std::unique_ptr<Scene>> scenes;
     int32_t nextScene = 1;
     std::unique_ptr<BatchEngine> batch;
@@ -518,7 +540,6 @@ struct Context {
     float lastMs = 0.f;
     int batchThreads = 0;  // threads per CTA of batched launches, 0 = from the groups' colour sizes
     uint64_t batchEpoch = 0;  // batched calls so far (Scene::batchStamp)
-    int* flowError = nullptr;   // page-locked: a flow launch's wait ran out (flow.cu)
     int* checkHost = nullptr;   // page-locked: the verdict of an update call's record checks
     int colourBlocksPerSm = 0;  // pairs.cu
     std::vector<bepugpu_server*> servers;  // live servers: shut down before the scenes go

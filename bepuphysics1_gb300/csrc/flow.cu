@@ -543,12 +543,9 @@ bepugpu_status Scene::UploadFlow(Context* ctx, const int32_t* a, const int32_t* 
 // The caller keeps the chunks until the stream has passed the copy.
 bepugpu_status Scene::UploadFlowChunks(Context* ctx, const std::vector<int2>& chunks, size_t slots) {
     if (chunks.empty()) return BEPUGPU_OK;
-    if (!ctx->flowError) {  // once a context, outside any stream capture
-        CK(cudaHostAlloc((void**)&ctx->flowError, sizeof(int), cudaHostAllocMapped));
-        *ctx->flowError = 0;
-    }
+    if (!flowStatus) CK(words->Take(&flowStatus));  // outside any stream capture
     if (!flowBlocksPerSm) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&flowBlocksPerSm, k_flow, kFlowThreads, 0));
-    CK(cudaHostGetDevicePointer((void**)&flow.error, ctx->flowError, 0));
+    CK(cudaHostGetDevicePointer((void**)&flow.error, flowStatus, 0));
     // the ends without a dynamic body keep visit -1
     CK(cudaMemsetAsync(flow.visit, 0xff, sizeof(int2) * slots, stream));
     CK(cudaMemcpyAsync(flow.chunks, chunks.data(), sizeof(int2) * chunks.size(), cudaMemcpyHostToDevice, stream));
@@ -598,11 +595,29 @@ bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool grou
     return BEPUGPU_OK;
 }
 
-bepugpu_status FlowStatus(Context* ctx) {
-    if (!ctx->flowError || !*(volatile int*)ctx->flowError) return BEPUGPU_OK;
-    *ctx->flowError = 0;
-    ctx->SetError("solve sweeps: a wait for an earlier visit ran out");
+bepugpu_status FlowStatus(Context* ctx, Scene* s) {
+    if (!s->flowStatus || !*(volatile int*)s->flowStatus) return BEPUGPU_OK;
+    *(volatile int*)s->flowStatus = 0;
+    ctx->SetError("solve sweeps of scene %d: a wait for an earlier visit ran out", s->id);
     return BEPUGPU_TIMEOUT;
+}
+
+StatusWords::~StatusWords() {
+    for (int* p : pages_) cudaFreeHost(p);
+}
+cudaError_t StatusWords::Take(int** word) {
+    if (free_.empty()) {
+        constexpr int kWords = 1024;
+        int* page = nullptr;
+        const cudaError_t e = cudaHostAlloc((void**)&page, sizeof(int) * kWords, cudaHostAllocMapped);
+        if (e != cudaSuccess) return e;
+        pages_.push_back(page);
+        for (int k = kWords - 1; k >= 0; k--) free_.push_back(page + k);
+    }
+    *word = free_.back();
+    free_.pop_back();
+    **word = 0;
+    return cudaSuccess;
 }
 
 }  // namespace bepugpu

@@ -427,5 +427,5 @@ extern "C" bepugpu_status bepugpu_get_islands(bepugpu_context* c, int32_t id, ui
     CK(cudaStreamSynchronize(s->stream));
     s->asyncPending = false;
     if (deactivation_index) *deactivation_index = idx;
-    return BEPUGPU_OK;
+    return FlowStatus(ctx, s);
 }

@@ -280,7 +280,12 @@ struct Server {
                     sl.queued = true;
                     ready.push_back(w.slotIds[k]);
                 }
-                Complete(w.reqs[k], status, w.id, w.startUs);
+                int32_t own = status;  // the scene's sweeps may have given up
+                if (own == BEPUGPU_OK && FlowStatus(&sink, sl.s) != BEPUGPU_OK) {
+                    own = BEPUGPU_TIMEOUT;
+                    SetError("wave: " + sink.lastError);
+                }
+                Complete(w.reqs[k], own, w.id, w.startUs);
             }
             w.busy = false;
             any = true;

@@ -577,15 +577,17 @@ bepugpu_status bepugpu_check_finite(bepugpu_context* ctx, int32_t scene, int32_t
  * context stays usable.  No reference counterpart. */
 bepugpu_status bepugpu_probe_bounded_wait(bepugpu_context* ctx, uint32_t spin_limit);
 /* Tests what follows a device-side wait that ran out, without one: the status
- * words of the named waits start as such a wait leaves them, once each, the
- * next time the scene's calls come to them.  Those calls return TIMEOUT and
- * leave the scene as it was. */
+ * words of the named waits read as such a wait leaves them, once each.  The
+ * first three when the scene's calls next come to them: those calls return
+ * TIMEOUT and leave the scene as it was.  The last two at once. */
 #define BEPUGPU_WAIT_COLOURING 1u /* bepugpu_update_pairs: the entries' sort and the colouring */
 #define BEPUGPU_WAIT_SLOTS 2u     /* bepugpu_update_pairs: the sort of the entries into slots */
 #define BEPUGPU_WAIT_BROAD_PHASE 4u /* the broad phase's sorts (bepugpu_broad_phase, bepugpu_update_pairs) */
 #define BEPUGPU_WAIT_PERSISTENT 8u /* a persistent step before this call: its barrier and status words at once,
                                       for bepugpu_synchronize to report */
-#define BEPUGPU_WAIT_ALL 15u
+#define BEPUGPU_WAIT_SWEEPS 16u /* a step before this call whose sweeps wait visit by visit; INVALID_OPERATION
+                                   for a scene without them */
+#define BEPUGPU_WAIT_ALL 31u
 bepugpu_status bepugpu_probe_expired_wait(bepugpu_context* ctx, int32_t scene, uint32_t where);
 
 /* Self-test of the device's float results of the reference's double-precision
@@ -628,7 +630,12 @@ bepugpu_status bepugpu_colour_list(const int32_t* body_a, const int32_t* body_b,
 
 /* Stages.  bepugpu_step runs the flagged stages as one device sequence:
  * refresh -> ForceUpdater -> Solver (prestep, warm start, iterations) ->
- * PositionUpdater.  dt = TimeStepSettings.TimeStepDuration. */
+ * PositionUpdater.  dt = TimeStepSettings.TimeStepDuration.
+ * The call does not wait for the device.  If a wait inside the sweeps ran out,
+ * the first of the scene's calls that hand out results returns TIMEOUT, with
+ * the state as the step left it (bepugpu_step_state, bepugpu_step_host, the
+ * download calls, bepugpu_get_islands, bepugpu_batch_step; bepugpu_synchronize
+ * for all scenes; the completion of a served request). */
 bepugpu_status bepugpu_step(bepugpu_context* ctx, int32_t scene, float dt, uint32_t flags);
 bepugpu_status bepugpu_set_solve_mode(bepugpu_context* ctx, int32_t scene, int32_t mode);
 /* Island groups.  An island (dynamic bodies connected through constraints)
@@ -803,7 +810,7 @@ typedef struct bepugpu_server_config {
 typedef struct bepugpu_completion {
     uint64_t tag;                  /* as submitted */
     int32_t scene;
-    int32_t status;                /* BEPUGPU_OK, NOT_FOUND, ADMISSION_REFUSED, CUDA_ERROR */
+    int32_t status;                /* BEPUGPU_OK, NOT_FOUND, ADMISSION_REFUSED, CUDA_ERROR, TIMEOUT (bepugpu_step) */
     uint32_t steps;
     uint32_t wave;                 /* wave number that ran it */
     double submit_us, start_us, done_us;  /* bepugpu_clock_us() at submit, wave launch, completion seen */

@@ -8,13 +8,14 @@ import pytest
 
 from bepuphysics1_gb300 import native as N
 from bepuphysics1_gb300 import scenes
-from bepuphysics1_gb300.solver import GpuSpace, default_settings
+from bepuphysics1_gb300.serve import Server
+from bepuphysics1_gb300.solver import GpuSpace, batch_step, body_states, default_settings, islands_of
 
 from parity import DT
 
 pytestmark = pytest.mark.gpu
 FLAGS = N.STEP_ALL | N.STEP_COLLIDE
-COLOURING, SLOTS, BROAD_PHASE, PERSISTENT = 1, 2, 4, 8
+COLOURING, SLOTS, BROAD_PHASE, PERSISTENT, SWEEPS = 1, 2, 4, 8, 16
 
 
 def _expire(sp, where):
@@ -105,8 +106,98 @@ def test_sorts_after_a_persistent_step_that_gave_up(gpu_context):
     twin.close()
 
 
+GROUPS_OFF = (0, 1024, 4096, 64, 0)
+
+
+def _flowing(ctx, seed):
+    b, m, _ = scenes.make_pile(nx=4, ny=3, nz=4, seed=seed)
+    sp = GpuSpace(ctx, b, m, group_policy=GROUPS_OFF)
+    sp.step(DT)
+    ctx.synchronize()
+    return sp, b, m
+
+
+# the calls that hand a scene's results out
+READS = {
+    "step_state": lambda sp, b, m: sp.step_state(body_states(b), None, DT),
+    "step_host": lambda sp, b, m: sp.step_host(b, m, DT),
+    "download_state": lambda sp, b, m: sp.download_state(body_states(b)),
+    "download_bodies": lambda sp, b, m: sp.download_bodies(),
+    "download_constraints": lambda sp, b, m: sp.download_constraints(),
+    "get_islands": lambda sp, b, m: (sp.set_islands(islands_of(b, m)), sp.get_islands()),
+    "batch_step": lambda sp, b, m: batch_step(sp.ctx, [sp], DT),
+}
+
+
+@pytest.mark.parametrize("call", sorted(READS))
+def test_a_scenes_own_call_reports_its_sweeps(gpu_context, call):
+    gpu_context.set_settings(default_settings())
+    (a, ab, am), (o, ob, om) = _flowing(gpu_context, 3), _flowing(gpu_context, 4)
+    for sp, b, m in ((a, ab, am), (o, ob, om)):
+        sp.download_bodies(b)
+    _expire(a, SWEEPS)
+    READS[call](o, ob, om)  # another scene's call neither reports nor clears it
+    assert f"scene {a.id}" in _timeout(READS[call], a, ab, am)
+    READS[call](a, ab, am)
+    gpu_context.synchronize()
+    a.close()
+    o.close()
+
+
+def test_synchronize_reports_every_scene(gpu_context):
+    gpu_context.set_settings(default_settings())
+    (a, _, _), (o, _, _) = _flowing(gpu_context, 3), _flowing(gpu_context, 4)
+    _expire(o, SWEEPS)
+    _expire(a, SWEEPS)
+    assert f"scene {a.id}:" in _timeout(gpu_context.synchronize)
+    gpu_context.synchronize()
+    a.download_bodies()
+    o.close()  # a closed scene's word goes to the next one, clear
+    p, _, _ = _flowing(gpu_context, 5)
+    p.download_bodies()
+    a.close()
+    p.close()
+
+
+def test_batch_advances_every_scene_before_it_reports(gpu_context):
+    gpu_context.set_settings(default_settings())
+    (a, _, _), (o, _, _), (t, _, _) = (_flowing(gpu_context, s) for s in (3, 4, 4))
+    _expire(a, SWEEPS)
+    _timeout(batch_step, gpu_context, [a, o], DT, 3)
+    for _ in range(3):
+        t.step(DT)
+    np.testing.assert_array_equal(o.download_bodies(), t.download_bodies())
+    for sp in (a, o, t):
+        sp.close()
+
+
+def test_a_served_requests_completion_reports_its_sweeps(gpu_context):
+    gpu_context.set_settings(default_settings())
+    (a, _, _), (o, _, _) = _flowing(gpu_context, 3), _flowing(gpu_context, 4)
+    _expire(a, SWEEPS)
+    srv = Server(gpu_context, dt=float(DT))
+    srv.add(a)
+    srv.add(o)
+    status = {}
+    for tag, sp in enumerate((o, a, a, o)):
+        srv.submit(sp.id, 2, tag)
+        srv.drain()
+    for c in srv.poll():
+        status[int(c["tag"])] = int(c["status"])
+    assert status == {0: N.OK, 1: N.TIMEOUT, 2: N.OK, 3: N.OK}
+    assert f"scene {a.id}" in srv.last_error()
+    srv.release(a)
+    srv.release(o)
+    srv.close()
+    gpu_context.synchronize()
+    a.close()
+    o.close()
+
+
 def test_unknown_waits_are_refused(gpu_context):
     b, m, _ = scenes.make_pile(nx=2, ny=2, nz=2)
     sp = GpuSpace(gpu_context, b, m)
-    assert sp.ctx.lib.bepugpu_probe_expired_wait(sp.ctx.handle, sp.id, 1 << 31) == N.INVALID_ARGUMENT
+    probe = sp.ctx.lib.bepugpu_probe_expired_wait
+    assert probe(sp.ctx.handle, sp.id, 1 << 31) == N.INVALID_ARGUMENT
+    assert probe(sp.ctx.handle, sp.id, SWEEPS) == N.INVALID_OPERATION  # island groups alone
     sp.close()
