@@ -716,6 +716,7 @@ Scene::~Scene() {
     if ((arena || staging) && stream) cudaStreamSynchronize(stream);  // no work reads the blocks any more
     if (heap) {
         heap->Free(arena);
+        heap->Free(flowBlock);
         heap->Free(staging);
     }
     if (spillHost && !spillHostBorrowed) cudaFreeHost(spillHost);
@@ -820,8 +821,6 @@ bepugpu_status Scene::Allocate(Context* ctx, uint32_t nb, uint32_t nm, uint32_t 
     L.groupJointRefs = take(8 * J); L.groupJointOffsets = take(4 * (2 * (M + J) + 2));
     L.bodyRecords = take(sizeof(bepugpu_body) * B);
     L.shape = take(16 * B); L.genSlots = take(4 * M);
-    L.flowChunks = take(8 * M); L.flowVisit = take(8 * M); L.flowDegree = take(4 * B); L.flowBegin = take(4 * (B + 1));
-    L.flowCsr = take(8 * M); L.flowLin = take(16 * B); L.flowAng = take(16 * B);
     arenaBytes = bytes;
     // The arena and the staging buffer are blocks of the context's heap, like
     // the ones a restore takes after a spill.
@@ -887,36 +886,44 @@ void Scene::Rebase() {
     bodyRecords = (bepugpu_body*)(base + L.bodyRecords);
     shape = (float4*)(base + L.shape);
     genSlotsDev = (int32_t*)(base + L.genSlots);
-    flow.chunks = (int2*)(base + L.flowChunks); flow.visit = (int2*)(base + L.flowVisit);
-    flow.degree = (int32_t*)(base + L.flowDegree); flow.csrBegin = (int32_t*)(base + L.flowBegin);
-    flow.csr = (int32_t*)(base + L.flowCsr); flow.lin = (float4*)(base + L.flowLin);
-    flow.ang = (float4*)(base + L.flowAng);
+    RebaseFlow();
 }
 
-// Moves the arena to pinned host memory and gives the scene's heap blocks
-// back (all of its device memory but the 1 KiB scratch block).  The scene's
-// step graph is dropped: it holds device addresses.
+// Moves the arena, and the sweeps' tables if the scene has them, to pinned host
+// memory and gives the scene's heap blocks back (all of its device memory but
+// the 1 KiB scratch block).  The scene's step graph is dropped: it holds device
+// addresses.
 // Neither call synchronises the device with other scenes' work, and without
 // `wait` neither blocks: the spill's copy is ordered on the scene's stream and
 // marked by evSpill, and its blocks become reusable once that copy is done; a
 // restore takes blocks from the heap, waits for the mark on the stream it is
-// given, copies there, and the scene's stream waits for the copy (evRestore).  `host` (optional) is a pinned buffer of arenaBytes
-// for the first spill, owned by the caller.
+// given, copies there, and the scene's stream waits for the copy (evRestore).
+// `host` (optional) is a pinned buffer of SpillBytes for the first spill, owned
+// by the caller.
 bepugpu_status Scene::Spill(Context* ctx, bool wait, void* host) {
     if (!arena) return BEPUGPU_OK;
+    if (spillHost && !spillHostBorrowed && spillHostBytes < SpillBytes()) {  // from before the scene had its tables
+        CK(cudaStreamSynchronize(stream));
+        cudaFreeHost(spillHost);
+        spillHost = nullptr;
+    }
     if (!spillHost) {
         if (host) {
             spillHost = host;
             spillHostBorrowed = true;
         } else {
-            CK(cudaMallocHost(&spillHost, arenaBytes));
+            CK(cudaMallocHost(&spillHost, SpillBytes()));
+            spillHostBytes = SpillBytes();
             spillHostBorrowed = false;
         }
     }
     if (!evSpill) CK(cudaEventCreateWithFlags(&evSpill, cudaEventDisableTiming));
     CK(cudaMemcpyAsync(spillHost, arena, arenaBytes, cudaMemcpyDeviceToHost, stream));
+    if (flowBlock) CK(cudaMemcpyAsync((char*)spillHost + arenaBytes, flowBlock, flowBytes, cudaMemcpyDeviceToHost, stream));
     CK(heap->FreeAfter(arena, stream));
     arena = nullptr;
+    if (flowBlock) CK(heap->FreeAfter(flowBlock, stream));
+    flowBlock = nullptr;
     if (staging) CK(heap->FreeAfter(staging, stream));
     staging = nullptr;
     CK(cudaEventRecord(evSpill, stream));
@@ -931,23 +938,21 @@ bepugpu_status Scene::Restore(Context* ctx, cudaStream_t q, bool wait) {
     if (arena) return BEPUGPU_OK;
     if (!q) q = stream;
     cudaError_t e = heap->Alloc(arenaBytes, &arena);
-    if (e == cudaSuccess) {
-        e = heap->Alloc(stagingBytes, &staging);
-        if (e != cudaSuccess) {
-            heap->Free(arena);
-            arena = nullptr;
-            staging = nullptr;
-        }
-    } else {
-        arena = nullptr;
-    }
+    if (e != cudaSuccess) arena = nullptr;
+    if (e == cudaSuccess && (e = heap->Alloc(stagingBytes, &staging)) != cudaSuccess) staging = nullptr;
+    if (e == cudaSuccess && flowBytes && (e = heap->Alloc(flowBytes, &flowBlock)) != cudaSuccess) flowBlock = nullptr;
     if (e != cudaSuccess) {
-        ctx->SetError("scene restore of %zu bytes: %s", arenaBytes + stagingBytes, cudaGetErrorString(e));
+        for (void** p : {&arena, &staging, &flowBlock}) {
+            heap->Free(*p);
+            *p = nullptr;
+        }
+        ctx->SetError("scene restore of %zu bytes: %s", DeviceBytes(), cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? BEPUGPU_OUT_OF_MEMORY : BEPUGPU_CUDA_ERROR;
     }
     Rebase();
     if (evSpill) CK(cudaStreamWaitEvent(q, evSpill, 0));
     CK(cudaMemcpyAsync(arena, spillHost, arenaBytes, cudaMemcpyHostToDevice, q));
+    if (flowBlock) CK(cudaMemcpyAsync(flowBlock, (char*)spillHost + arenaBytes, flowBytes, cudaMemcpyHostToDevice, q));
     if (q != stream) {
         if (!evRestore) CK(cudaEventCreateWithFlags(&evRestore, cudaEventDisableTiming));
         CK(cudaEventRecord(evRestore, q));
@@ -973,9 +978,10 @@ bool Scene::OwnSpillBuffer() {
     if (arena || !spillHostBorrowed) return true;
     if (stream) cudaStreamSynchronize(stream);  // the spill copy has landed
     void* own = nullptr;
-    if (cudaMallocHost(&own, arenaBytes) != cudaSuccess) return false;
-    std::memcpy(own, spillHost, arenaBytes);
+    if (cudaMallocHost(&own, SpillBytes()) != cudaSuccess) return false;
+    std::memcpy(own, spillHost, SpillBytes());
     spillHost = own;
+    spillHostBytes = SpillBytes();
     spillHostBorrowed = false;
     return true;
 }

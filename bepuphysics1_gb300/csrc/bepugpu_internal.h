@@ -312,7 +312,6 @@ struct ArenaLayout {
     size_t groupJointRefs, groupJointOffsets;
     size_t bodyRecords;
     size_t shape, genSlots;
-    size_t flowChunks, flowVisit, flowDegree, flowBegin, flowCsr, flowLin, flowAng;
 };
 
 struct Server;
@@ -386,6 +385,13 @@ struct Scene {
         return g;
     }
     FlowTables flow{};
+    // The tables' block, for the scene's capacity: 24 bytes a manifold and 40 a
+    // body, from the first constraints that flow on.  A scene of island groups
+    // that fit a CTA has none.
+    void* flowBlock = nullptr;
+    size_t flowBytes = 0;
+    bepugpu_status NeedFlow(Context* ctx);
+    size_t RebaseFlow();
     // CTAs of k_flow an SM holds: with the scene, since a server's worker steps
     // it through a context of its own.
     int flowBlocksPerSm = 0;
@@ -403,7 +409,7 @@ struct Scene {
     void* arena = nullptr;          // null while spilled
     size_t arenaBytes = 0;
     ArenaLayout layout{};
-    void* spillHost = nullptr;      // pinned copy of the arena while spilled
+    void* spillHost = nullptr;      // pinned copy of the arena (and the sweeps' tables) while spilled
     bool spillHostBorrowed = false; // spillHost belongs to a server's pinned pool
     cudaEvent_t evSpill = nullptr, evRestore = nullptr;
     void Rebase();
@@ -411,7 +417,9 @@ struct Scene {
     bepugpu_status Restore(Context* ctx, cudaStream_t q = nullptr, bool wait = true);
     void DropBorrowedSpillBuffer();
     bool OwnSpillBuffer();
-    // Lends a pinned buffer of arenaBytes for spills (kept until dropped);
+    size_t spillHostBytes = 0;      // of a buffer of its own
+    size_t SpillBytes() const { return arenaBytes + flowBytes; }
+    // Lends a pinned buffer of SpillBytes for spills (kept until dropped);
     // false if the scene already has one.
     bool LendSpillBuffer(void* host) {
         if (spillHost || !host) return false;
@@ -419,7 +427,7 @@ struct Scene {
         spillHostBorrowed = true;
         return true;
     }
-    size_t DeviceBytes() const { return arenaBytes + stagingBytes; }
+    size_t DeviceBytes() const { return arenaBytes + flowBytes + stagingBytes; }
     void* staging = nullptr;
     size_t stagingBytes = 0;
     size_t stagingManifoldsAt = 0;  // manifold records start here in staging (body records first)

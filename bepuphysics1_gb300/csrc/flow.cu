@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/bepugpu.h"
@@ -489,13 +490,46 @@ const GroupClass* FlowGroups(const GroupPlan& plan) {
     return large ? &c : nullptr;
 }
 
+// The tables' places in their block; returns the block's size.
+size_t Scene::RebaseFlow() {
+    const size_t B = maxBodies ? maxBodies : 1, M = maxManifolds ? maxManifolds : 1;
+    size_t bytes = 0;
+    auto take = [&](auto*& p, size_t n) {
+        p = flowBlock ? reinterpret_cast<std::remove_reference_t<decltype(p)>>((char*)flowBlock + bytes) : nullptr;
+        bytes += (n * sizeof(*p) + 255) & ~(size_t)255;
+    };
+    take(flow.chunks, M);
+    take(flow.visit, M);
+    take(flow.csr, 2 * M);
+    take(flow.degree, B);
+    take(flow.csrBegin, B + 1);
+    take(flow.lin, B);
+    take(flow.ang, B);
+    return bytes;
+}
+bepugpu_status Scene::NeedFlow(Context* ctx) {
+    if (flowBlock) return BEPUGPU_OK;
+    const size_t bytes = RebaseFlow();
+    const cudaError_t e = heap->Alloc(bytes, &flowBlock);
+    if (e != cudaSuccess) {
+        flowBlock = nullptr;
+        ctx->SetError("solve sweeps: %zu bytes of tables: %s", bytes, cudaGetErrorString(e));
+        return e == cudaErrorMemoryAllocation ? BEPUGPU_OUT_OF_MEMORY : BEPUGPU_CUDA_ERROR;
+    }
+    flowBytes = bytes;
+    RebaseFlow();
+    return BEPUGPU_OK;
+}
+
 bepugpu_status Scene::UploadFlow(Context* ctx, const int32_t* a, const int32_t* b) {
-    // slots [0, n) and [g0, g1)
-    const int n = groupPlan.globalCount;
+    // slots [0, n) and [g0, g1); beside joints the sweep path runs colour by colour
+    const int n = groupPlan.jointGlobalCount ? 0 : groupPlan.globalCount;
     const GroupClass* large = FlowGroups(groupPlan);
     const int g0 = large ? groupPlan.groups[large->begin].mBegin : n, g1 = large ? groupPlan.groups[large->end - 1].mEnd : n;
     flow.chunkCount = flow.groupChunkCount = 0;
     if (n == 0 && g1 == g0) return BEPUGPU_OK;
+    bepugpu_status st = NeedFlow(ctx);
+    if (st != BEPUGPU_OK) return st;
     std::vector<int32_t> recordOf(groupPlan.slotOf.size(), -1);
     for (size_t i = 0; i < groupPlan.slotOf.size(); i++) recordOf[groupPlan.slotOf[i]] = (int32_t)i;
     const int nb = this->b.count;
@@ -531,13 +565,16 @@ bepugpu_status Scene::UploadFlow(Context* ctx, const int32_t* a, const int32_t* 
         }
         if (!any) break;
     }
-    std::vector<int2> chunks = FlowChunks(manifoldOffsets);
-    flow.chunkCount = (int)chunks.size();
-    flow.groupChunkCount = (int)groupChunks.size();
+    std::vector<int2> chunks;
+    if (n) chunks = FlowChunks(manifoldOffsets);
+    const size_t sweepChunks = chunks.size();
     chunks.insert(chunks.end(), groupChunks.begin(), groupChunks.end());
-    bepugpu_status st = UploadFlowChunks(ctx, chunks, groupPlan.slotOf.size());
+    st = UploadFlowChunks(ctx, chunks, groupPlan.slotOf.size());
+    if (st != BEPUGPU_OK) return st;
     CK(cudaStreamSynchronize(stream));
-    return st;
+    flow.chunkCount = (int)sweepChunks;
+    flow.groupChunkCount = (int)groupChunks.size();
+    return BEPUGPU_OK;
 }
 
 // The caller keeps the chunks until the stream has passed the copy.
@@ -571,6 +608,10 @@ bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool grou
         f.chunks += f.chunkCount;
         f.chunkCount = f.groupChunkCount;
     }
+    if (f.chunkCount == 0) {
+        ctx->SetError("solve sweeps: no tables (the last constraint upload failed)");
+        return BEPUGPU_INVALID_OPERATION;
+    }
     const int resident = s->flowBlocksPerSm * ctx->smCount;
     if (resident < 1) {
         ctx->SetError("solve sweeps: no resident CTA (%d an SM of %d)", s->flowBlocksPerSm, ctx->smCount);
@@ -581,7 +622,7 @@ bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool grou
     if (launches) (*launches)++;
     cudaLaunchConfig_t cfg = {};
     // a warp per chunk on its own CTA while the CTAs last
-    cfg.gridDim = dim3((unsigned)std::max(1, std::min(resident, f.chunkCount)));
+    cfg.gridDim = dim3((unsigned)std::min(resident, f.chunkCount));
     cfg.blockDim = dim3(kFlowThreads);
     cfg.stream = s->stream;
     cudaLaunchAttribute attr[1];

@@ -652,6 +652,10 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
             return e == cudaErrorMemoryAllocation ? BEPUGPU_OUT_OF_MEMORY : BEPUGPU_CUDA_ERROR;
         }
     }
+    if (nPairs) {
+        bepugpu_status fs = s->NeedFlow(ctx);
+        if (fs != BEPUGPU_OK) return fs;
+    }
     Carve cv{(char*)P.block};
     const int T = 256;
     auto* table = cv.take<unsigned long long>(tableSlots);
@@ -725,10 +729,10 @@ extern "C" bepugpu_status bepugpu_update_pairs(bepugpu_context* c, int32_t id, f
     s->colouringOnDevice = true;
     s->colouringEntries = n;
     s->manifoldOffsets = col.offsets;
-    s->flow.chunkCount = (int)chunks.size();
-    s->flow.groupChunkCount = 0;
+    s->flow.chunkCount = s->flow.groupChunkCount = 0;
     bepugpu_status fs = s->UploadFlowChunks(ctx, chunks, (size_t)n);
     if (fs != BEPUGPU_OK) return fs;
+    s->flow.chunkCount = (int)chunks.size();
     s->jointOffsets.assign(col.colours + 1, 0);
     s->m.count = n;
     s->generatedCount = n;

@@ -203,7 +203,7 @@ struct Server {
     void LendSpillBuffers(Scene* only) {
         for (Slot& sl : slots) {
             if (!sl.live || (only && sl.s != only) || sl.s->spillHost) continue;
-            sl.s->LendSpillBuffer(hostPool.Take(sl.s->arenaBytes));
+            sl.s->LendSpillBuffer(hostPool.Take(sl.s->SpillBytes()));
         }
     }
 

@@ -125,3 +125,32 @@ def test_sweep_scenes_and_towers_in_one_wave(gpu_context):
         _assert_same(_state(sp, b, m), _state(alone, b, m))
         alone.close()
         sp.close()
+
+
+def test_scenes_without_sweeps_hold_no_tables(gpu_context):
+    """The sweeps' tables, 24 bytes a manifold and 40 a body, come with the first
+    constraints that need them and stay."""
+    gpu_context.set_settings(default_settings())
+    b, m = scenes.make_tower(150, seed=6)[:2]  # one island group by default
+
+    def bytes_of(make):
+        before = gpu_context.memory_usage()[1]
+        sp = make()
+        return sp, gpu_context.memory_usage()[1] - before
+
+    grouped, none = bytes_of(lambda: GpuSpace(gpu_context, b, m))
+    swept, tables = bytes_of(lambda: GpuSpace(gpu_context, b, m, group_policy=SWEEPS))
+    extra = tables - none
+    assert 24 * len(m) + 40 * len(b) <= extra < 24 * len(m) + 40 * len(b) + 8192
+    before = gpu_context.memory_usage()[1]
+    grouped.set_group_policy(*SWEEPS)
+    for _ in range(2):
+        grouped.upload_constraints(m)
+        assert gpu_context.memory_usage()[1] - before == extra
+    for sp in (grouped, swept):
+        for _ in range(3):
+            sp.step(DT)
+    _assert_same(_state(grouped, b, m), _state(swept, b, m))
+    grouped.close()
+    swept.close()
+    assert gpu_context.memory_usage()[1] == before - none - tables
