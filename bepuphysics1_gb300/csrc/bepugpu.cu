@@ -1684,10 +1684,7 @@ bepugpu_status bepugpu_upload_constraints(bepugpu_context* c, int32_t id, const 
         bepugpu_status gst = s->UploadGroups(ctx);
         if (gst != BEPUGPU_OK) return gst;
     }
-    {
-        bepugpu_status fst = s->UploadFlow(ctx, a.data() + nj, bb.data() + nj);
-        if (fst != BEPUGPU_OK) return fst;
-    }
+    s->flow.chunkCount = s->flow.groupChunkCount = 0;  // until their tables are there
     s->hostSlotOf = plan.slotOf;
     s->maxBodyReferenced = -1;
     for (uint32_t u = 0; u < nm + nj; u++) s->maxBodyReferenced = std::max(s->maxBodyReferenced, std::max(a[u], bb[u]));
@@ -1699,7 +1696,8 @@ bepugpu_status bepugpu_upload_constraints(bepugpu_context* c, int32_t id, const 
         bepugpu_status gst = PrepareGenerated(ctx, s, man, nm, s->hostSlotOf);
         if (gst != BEPUGPU_OK) return gst;
     }
-    return UploadManifoldRecords(ctx, s, man, nm);
+    bepugpu_status st = UploadManifoldRecords(ctx, s, man, nm);
+    return st == BEPUGPU_OK ? s->UploadFlow(ctx) : st;
 }
 
 bepugpu_status bepugpu_update_manifolds(bepugpu_context* c, int32_t id, const bepugpu_manifold* man, uint32_t n) {

@@ -40,7 +40,12 @@ struct SortDigits {
     int passes;
     int shift[10], bits[10];
 };
-constexpr int kSortBlocks = 64, kSortHistWords = kSortBlocks * 512;
+constexpr int kSortBlocks = 64, kSortBins = 512, kSortHistWords = kSortBlocks * kSortBins;
+// CTAs of a sort of at most `capacity` keys; it uses kSortBins words of hist for each.
+constexpr size_t SortBlocks(size_t capacity) {
+    const size_t blocks = (capacity + 2047) / 2048;
+    return blocks < 1 ? 1 : (blocks < (size_t)kSortBlocks ? blocks : (size_t)kSortBlocks);
+}
 // The sorted keys end in `keys`; `odd` allows a number of passes that ends in `other`.
 SortDigits SortPlan(int lowFrom, int lowBits, int highBits, bool odd = false);
 int BitsFor(size_t values);  // bits that tell `values` values apart
@@ -221,7 +226,8 @@ struct FlowTables {
     int32_t* degree;          // per body: visits of a sweep
     int32_t* csrBegin;        // per body: its entries of csr, bodies + 1
     int32_t* csr;             // slot << 1 | end (0 A, 1 B), ascending
-    float4 *lin, *ang;        // per body: velocity, w = visits so far (bits)
+    int32_t* sort;            // words of the upload's sort, then its status
+    float4 *lin, *ang;        // per body: velocity, w = tag (bits): the visit whose turn it is and the active set
     int* error;               // Scene::flowStatus, as the device sees it
     int chunkCount;
     int groupChunkCount;      // chunks after those: the slots of FlowGroups
@@ -385,7 +391,7 @@ struct Scene {
         return g;
     }
     FlowTables flow{};
-    // The tables' block, for the scene's capacity: 24 bytes a manifold and 40 a
+    // The tables' block, for the scene's capacity: 26 bytes a manifold and 40 a
     // body, from the first constraints that flow on.  A scene of island groups
     // that fit a CTA has none.
     void* flowBlock = nullptr;
@@ -397,9 +403,9 @@ struct Scene {
     int flowBlocksPerSm = 0;
     StatusWords* words = nullptr;  // the owning context's
     int* flowStatus = nullptr;     // page-locked: a wait of the scene's sweeps ran out (FlowStatus)
-    // flow.cu: the tables from the constraint upload's records (bodies a, b
-    // per manifold record), or from update_pairs' sorted (body, entry) keys.
-    bepugpu_status UploadFlow(Context* ctx, const int32_t* a, const int32_t* b);
+    // flow.cu: the tables from the constraint upload's slots, or from
+    // update_pairs' sorted (body, entry) keys.
+    bepugpu_status UploadFlow(Context* ctx);
     bepugpu_status UploadFlowChunks(Context* ctx, const std::vector<int2>& chunks, size_t slots);
     bepugpu_status BuildFlowOnDevice(Context* ctx, const unsigned long long* entries, int count, const int2* ends,
                                      const int* slots, const int* status);

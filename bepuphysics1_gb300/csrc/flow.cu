@@ -441,12 +441,38 @@ __global__ void __launch_bounds__(kFlowThreads, 4) k_flow(ManifoldSoA m, BodySoA
         }
 }
 
-// update_pairs' side of the tables, from its (dynamic body, entry) keys
-// sorted by body: where each body's entries start, and the entries as
-// slot << 1 | end in slot order.  Nothing when the slots' sort gave up (*err).
+// The body of sorted entry k: -1 before the first, `bodies` past the last.
 __device__ __forceinline__ int BodyOfEntry(const unsigned long long* __restrict__ entries, int count, int bodies, int k) {
     return k < 0 ? -1 : (k < count && entries[k] != ~0ull ? (int)(entries[k] >> 32) : bodies);
 }
+// The tables from the constraint upload's slots [0, n) and those from g0 on: a
+// (dynamic body, slot << 1 | end) entry for each end, ~0 without one, sorted by
+// body.  The slots ascend and the sort is stable, so a body's entries end in
+// slot order.  Nothing when the sort gave up (*err).
+__global__ void k_flow_entries(ManifoldSoA m, BodySoA b, int n, int g0, int slots, unsigned long long* entries) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= slots) return;
+    const int s = i < n ? i : g0 + i - n;
+    const int4 h = m.head[s];
+    const auto entry = [&](int body, int end) {
+        const bool moves = body >= 0 && b.pos[body].w != 0.f;
+        return moves ? ((unsigned long long)(unsigned)body << 32) | (unsigned)(s << 1 | end) : ~0ull;
+    };
+    entries[2 * (size_t)i] = entry(h.x, 0);
+    entries[2 * (size_t)i + 1] = entry(h.y, 1);
+}
+__global__ void k_flow_slots(const unsigned long long* __restrict__ entries, int count, int bodies, FlowTables f,
+                             const int* __restrict__ err) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k > count || *err) return;
+    const int body = BodyOfEntry(entries, count, bodies, k);
+    for (int i = BodyOfEntry(entries, count, bodies, k - 1) + 1; i <= body; i++) f.csrBegin[i] = k;
+    if (body < bodies) f.csr[k] = (int)(entries[k] & 0xffffffffu);
+}
+
+// update_pairs' side of the tables, from its (dynamic body, entry) keys
+// sorted by body: where each body's entries start, and the entries as
+// slot << 1 | end in slot order.  Nothing when the slots' sort gave up (*err).
 __global__ void k_flow_csr(const unsigned long long* __restrict__ entries, int count, int bodies,
                            const int2* __restrict__ ends, const int* __restrict__ slotOf, FlowTables f,
                            const int* __restrict__ err) {
@@ -503,6 +529,7 @@ size_t Scene::RebaseFlow() {
     take(flow.csr, 2 * M);
     take(flow.degree, B);
     take(flow.csrBegin, B + 1);
+    take(flow.sort, SortBlocks(2 * M) * kSortBins + 1);
     take(flow.lin, B);
     take(flow.ang, B);
     return bytes;
@@ -521,7 +548,10 @@ bepugpu_status Scene::NeedFlow(Context* ctx) {
     return BEPUGPU_OK;
 }
 
-bepugpu_status Scene::UploadFlow(Context* ctx, const int32_t* a, const int32_t* b) {
+// After the records' upload, whose heads and staging buffer it uses.  On the
+// host, two walks over the records in slot order were a twelfth of the upload of
+// a pile of 65,536 boxes: 14.8 ms, 13.7 this way.
+bepugpu_status Scene::UploadFlow(Context* ctx) {
     // slots [0, n) and [g0, g1); beside joints the sweep path runs colour by colour
     const int n = groupPlan.jointGlobalCount ? 0 : groupPlan.globalCount;
     const GroupClass* large = FlowGroups(groupPlan);
@@ -530,27 +560,6 @@ bepugpu_status Scene::UploadFlow(Context* ctx, const int32_t* a, const int32_t* 
     if (n == 0 && g1 == g0) return BEPUGPU_OK;
     bepugpu_status st = NeedFlow(ctx);
     if (st != BEPUGPU_OK) return st;
-    std::vector<int32_t> recordOf(groupPlan.slotOf.size(), -1);
-    for (size_t i = 0; i < groupPlan.slotOf.size(); i++) recordOf[groupPlan.slotOf[i]] = (int32_t)i;
-    const int nb = this->b.count;
-    std::vector<int32_t> begin(nb + 1, 0);
-    auto moving = [&](int32_t e) { return e >= 0 && hostDynamic[e]; };
-    auto slots = [&](auto visit) {
-        for (int s = 0; s < n; s++) visit(s, a[recordOf[s]], b[recordOf[s]]);
-        for (int s = g0; s < g1; s++) visit(s, a[recordOf[s]], b[recordOf[s]]);
-    };
-    slots([&](int, int32_t x, int32_t y) {
-        if (moving(x)) begin[x + 1]++;
-        if (moving(y)) begin[y + 1]++;
-    });
-    for (int i = 0; i < nb; i++) begin[i + 1] += begin[i];
-    std::vector<int32_t> at(begin.begin(), begin.end() - 1), csr(begin[nb]);
-    slots([&](int s, int32_t x, int32_t y) {
-        if (moving(x)) csr[at[x]++] = s << 1;
-        if (moving(y)) csr[at[y]++] = (s << 1) | 1;
-    });
-    CK(cudaMemcpyAsync(flow.csrBegin, begin.data(), sizeof(int32_t) * begin.size(), cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(flow.csr, csr.data(), sizeof(int32_t) * csr.size(), cudaMemcpyHostToDevice, stream));
     // the groups' chunks colour by colour over all of them
     std::vector<int2> groupChunks;
     for (int c = 0; large; c++) {
@@ -571,7 +580,27 @@ bepugpu_status Scene::UploadFlow(Context* ctx, const int32_t* a, const int32_t* 
     chunks.insert(chunks.end(), groupChunks.begin(), groupChunks.end());
     st = UploadFlowChunks(ctx, chunks, groupPlan.slotOf.size());
     if (st != BEPUGPU_OK) return st;
+    const int slots = n + g1 - g0, T = 256;
+    const size_t keys = 2 * (size_t)slots;
+    auto* entries = (unsigned long long*)staging;  // 32 bytes a slot; a manifold record is larger
+    static_assert(sizeof(bepugpu_manifold) >= 32, "the entries and the sort's second buffer fit the staged records");
+    int* status = flow.sort + SortBlocks(keys) * kSortBins;
+    CK(cudaMemsetAsync(status, 0, sizeof(int), stream));
+    CK(MarkExpired(status, BEPUGPU_WAIT_TABLES));
+    k_flow_entries<<<(slots + T - 1) / T, T, 0, stream>>>(m, b, n, g0, slots, entries);
+    CK(cudaGetLastError());
+    CK(RadixSort(this, entries, entries + keys, nullptr, keys, SortPlan(0, 0, BitsFor((size_t)b.count + 1)),
+                 (unsigned*)flow.sort, status, stream));
+    k_flow_slots<<<(int)((keys + T) / T), T, 0, stream>>>(entries, (int)keys, b.count, flow, status);
+    CK(cudaGetLastError());
+    int gaveUp = 0;
+    CK(cudaMemcpyAsync(&gaveUp, status, sizeof(int), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
+    if (gaveUp) {
+        CK(cudaMemsetAsync(SortCounter(), 0, sizeof(unsigned), stream));
+        ctx->SetError("upload_constraints: the sort of the sweeps' visits did not finish");
+        return BEPUGPU_TIMEOUT;
+    }
     flow.chunkCount = (int)sweepChunks;
     flow.groupChunkCount = (int)groupChunks.size();
     return BEPUGPU_OK;

@@ -27,7 +27,8 @@ namespace bepugpu {
 namespace {
 
 constexpr int kSortThreads = 1024, kSortWarps = kSortThreads / 32;
-constexpr int kSortDigitBits = 9, kSortBins = 1 << kSortDigitBits;
+constexpr int kSortDigitBits = 9;
+static_assert(kSortBins == 1 << kSortDigitBits, "a digit's values");
 
 __global__ void __launch_bounds__(kSortThreads) k_radix_sort(unsigned long long* keys, unsigned long long* other,
                                                              const unsigned* __restrict__ count, unsigned capacity,
@@ -129,7 +130,7 @@ int BitsFor(size_t values) {
 cudaError_t RadixSort(const Scene* s, unsigned long long* keys, unsigned long long* other, const unsigned* count,
                       size_t capacity, const SortDigits& digits, unsigned* hist, int* err, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)std::min<size_t>(kSortBlocks, std::max<size_t>(1, (capacity + 2047) / 2048)));
+    cfg.gridDim = dim3((unsigned)SortBlocks(capacity));
     cfg.blockDim = dim3(kSortThreads);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];

@@ -577,9 +577,9 @@ bepugpu_status bepugpu_check_finite(bepugpu_context* ctx, int32_t scene, int32_t
  * context stays usable.  No reference counterpart. */
 bepugpu_status bepugpu_probe_bounded_wait(bepugpu_context* ctx, uint32_t spin_limit);
 /* Tests what follows a device-side wait that ran out, without one: the status
- * words of the named waits read as such a wait leaves them, once each.  The
- * first three when the scene's calls next come to them: those calls return
- * TIMEOUT and leave the scene as it was.  The last two at once. */
+ * words of the named waits read as such a wait leaves them, once each: those of
+ * a call when the scene next comes to them -- that call returns TIMEOUT and, but
+ * for the upload's, leaves the scene as it was -- those of a step at once. */
 #define BEPUGPU_WAIT_COLOURING 1u /* bepugpu_update_pairs: the entries' sort and the colouring */
 #define BEPUGPU_WAIT_SLOTS 2u     /* bepugpu_update_pairs: the sort of the entries into slots */
 #define BEPUGPU_WAIT_BROAD_PHASE 4u /* the broad phase's sorts (bepugpu_broad_phase, bepugpu_update_pairs) */
@@ -587,7 +587,9 @@ bepugpu_status bepugpu_probe_bounded_wait(bepugpu_context* ctx, uint32_t spin_li
                                       for bepugpu_synchronize to report */
 #define BEPUGPU_WAIT_SWEEPS 16u /* a step before this call whose sweeps wait visit by visit; INVALID_OPERATION
                                    for a scene without them */
-#define BEPUGPU_WAIT_ALL 31u
+#define BEPUGPU_WAIT_TABLES 32u /* bepugpu_upload_constraints: the sort of the sweeps' visits; the scene then takes
+                                   no step until its constraints are uploaded again */
+#define BEPUGPU_WAIT_ALL 63u
 bepugpu_status bepugpu_probe_expired_wait(bepugpu_context* ctx, int32_t scene, uint32_t where);
 
 /* Self-test of the device's float results of the reference's double-precision

@@ -15,7 +15,7 @@ from parity import DT
 
 pytestmark = pytest.mark.gpu
 FLAGS = N.STEP_ALL | N.STEP_COLLIDE
-COLOURING, SLOTS, BROAD_PHASE, PERSISTENT, SWEEPS = 1, 2, 4, 8, 16
+COLOURING, SLOTS, BROAD_PHASE, PERSISTENT, SWEEPS, TABLES = 1, 2, 4, 8, 16, 32
 
 
 def _expire(sp, where):
@@ -190,6 +190,22 @@ def test_a_served_requests_completion_reports_its_sweeps(gpu_context):
     srv.release(o)
     srv.close()
     gpu_context.synchronize()
+    a.close()
+    o.close()
+
+
+def test_upload_that_gave_up(gpu_context):
+    gpu_context.set_settings(default_settings())
+    (a, _, m), (o, _, _) = _flowing(gpu_context, 3), _flowing(gpu_context, 3)
+    _expire(a, TABLES)
+    assert "upload_constraints" in _timeout(a.upload_constraints, m)
+    with pytest.raises(N.InvalidOperationException):
+        a.step(DT)
+    a.upload_constraints(m)
+    o.upload_constraints(m)
+    for sp in (a, o):
+        sp.step(DT)
+    np.testing.assert_array_equal(a.download_bodies(), o.download_bodies())
     a.close()
     o.close()
 

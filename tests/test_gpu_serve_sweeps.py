@@ -128,7 +128,7 @@ def test_sweep_scenes_and_towers_in_one_wave(gpu_context):
 
 
 def test_scenes_without_sweeps_hold_no_tables(gpu_context):
-    """The sweeps' tables, 24 bytes a manifold and 40 a body, come with the first
+    """The sweeps' tables, 26 bytes a manifold and 40 a body, come with the first
     constraints that need them and stay."""
     gpu_context.set_settings(default_settings())
     b, m = scenes.make_tower(150, seed=6)[:2]  # one island group by default
