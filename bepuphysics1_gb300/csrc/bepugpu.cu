@@ -558,7 +558,7 @@ __device__ __forceinline__ void WarmJointSlot(const JointSoA& j, const BodySoA& 
     if (!(st.x & kGroupActive)) return;
     int4 h = j.head[s];
     BodyState A, B;
-    LoadVisit(GlobalBodies{b}, h.x, h.y, st.x, A, B);
+    LoadVisit<true>(GlobalBodies{b}, h.x, h.y, st.x, A, B);
     WarmJoint<kAdded>(j, s, A, B, st.x, h.z & 0xff);
     StoreVisit(GlobalBodies{b}, h.x, h.y, st.x, A, B);
 }
@@ -568,7 +568,7 @@ __device__ __forceinline__ void SolveJointSlot(const JointSoA& j, const BodySoA&
     if (!(st.x & kGroupActive)) return;
     int4 h = j.head[s];
     BodyState A, B;
-    LoadVisit(GlobalBodies{b}, h.x, h.y, st.x, A, B);
+    LoadVisit<true>(GlobalBodies{b}, h.x, h.y, st.x, A, B);
     SolveJoint<kAdded>(j, s, A, B, st, h.z & 0xff, p);
     StoreVisit(GlobalBodies{b}, h.x, h.y, st.x, A, B);
     j.state[s] = st;
