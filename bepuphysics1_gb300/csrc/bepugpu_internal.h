@@ -241,11 +241,12 @@ bepugpu_status LaunchFlow(Context* ctx, Scene* s, const StepParams& p, bool grou
 // Scenes of more chunks than this (four for each of the 16 warps a GB300 SM
 // holds of k_flow) warm-start in a launch per colour.  Such a step has more
 // launches than colours, as callers of bepugpu_last_step_launches know the
-// sweep path (a test of the packed 65,536-box pile holds it to that).  A step
-// with the warm start in the flow launch against per colour: 188,667 manifolds
-// 285 and 305 us, 425,999 650 and 657 us, 757,861 1,190 and 1,178 us; in
-// smaller scenes the colours' launches cost more (82,000 manifolds of 16
-// colours: 45 us a step).
+// sweep path (a test of the packed 65,536-box pile holds it to that): the line
+// lies there for them, not for speed.  A step with the warm start in the flow
+// launch against per colour: 188,667 manifolds 285 and 305 us, 425,999 650 and
+// 657 us, 757,861 1,190 and 1,178 us, so by time alone it would lie near
+// 700,000 manifolds; in smaller scenes the colours' launches cost more (82,000
+// manifolds of 16 colours: 45 us a step).
 constexpr int kFlowWarmChunks = 9728;
 // TIMEOUT when a wait of one of the scene's finished flow launches ran out (and
 // clears it).  For each call that hands the scene's results out.

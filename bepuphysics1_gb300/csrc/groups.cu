@@ -31,7 +31,7 @@ namespace bepugpu {
 // of those slots into the global solve lanes.  One thread per manifold or
 // body fills the GPU where a group CTA runs its few threads over them in turn;
 // the group kernel then copies the lanes into shared memory
-// (GroupStep's `prestepped`).  The same device routines as the colour-sweep
+// (GroupStep's kPrestepped).  The same device routines as the colour-sweep
 // path's k_refresh_force_list and k_prestep.
 __global__ void k_group_refresh_force(ManifoldSoA m, BodySoA b, StepParams p, const int32_t* __restrict__ list, int n,
                                       int s0, int s1, uint32_t flags) {

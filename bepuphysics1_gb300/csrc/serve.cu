@@ -713,7 +713,7 @@ bepugpu_status bepugpu_server_add_scene(bepugpu_server* h, int32_t scene) {
         return BEPUGPU_INVALID_OPERATION;
     }
     if (sc->mode != BEPUGPU_MODE_GRAPH) {
-        // a cooperative launch beside other waves' kernels could not count on co-residency
+        // its grid barriers would hold the SMs for whole steps between the waves' launches
         s->SetError("scene " + std::to_string(scene) + " is in persistent mode; serving takes graph-mode scenes");
         return BEPUGPU_INVALID_OPERATION;
     }

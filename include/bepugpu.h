@@ -710,10 +710,13 @@ bepugpu_status bepugpu_batch_step_each(bepugpu_context* ctx, const int32_t* scen
 bepugpu_status bepugpu_set_batch_threads(bepugpu_context* ctx, int32_t threads);
 
 /* Per-phase device times of one step run as separate launches, each bracketed
- * by CUDA events on the scene's stream (an instrumented copy of bepugpu_step:
- * it advances the scene like bepugpu_step does).  The solve census counts,
- * before each solve sweep, the manifolds still active and their algorithmic
- * bytes 76*d + 136 + 48*c (c contacts, d dynamic bodies). */
+ * by CUDA events on the scene's stream.  It advances the scene like
+ * bepugpu_step does, bit for bit, but not in the same launches: the sweep path
+ * goes colour by colour and every island group runs in one CTA, so that the
+ * solve census can count, before each solve sweep, the manifolds still active
+ * and their algorithmic bytes 76*d + 136 + 48*c (c contacts, d dynamic bodies).
+ * The census is the step's own; for its times see bepugpu_last_step_ms and
+ * bepugpu_last_step_phase_ms where bepugpu_step sweeps visit by visit. */
 typedef struct bepugpu_phase_times {
     float refresh_ms, force_ms, prestep_ms, warm_ms, solve_ms, position_ms;
     uint32_t solve_launches, warm_launches;
