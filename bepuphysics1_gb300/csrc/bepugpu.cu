@@ -1641,11 +1641,18 @@ bepugpu_status bepugpu_upload_constraints(bepugpu_context* c, int32_t id, const 
             return BEPUGPU_INVALID_ARGUMENT;
         }
     }
-    if (!ColourSolverList(a.data(), bb.data(), (int32_t)(nm + nj), s->hostDynamic.data(), nb, s->colouring,
+    Colouring colouring;
+    if (!ColourSolverList(a.data(), bb.data(), (int32_t)(nm + nj), s->hostDynamic.data(), nb, colouring,
                           follows.data())) {
         ctx->SetError("a constraint references a body outside [0, %d)", nb);
         return BEPUGPU_INVALID_ARGUMENT;
     }
+    {
+        bepugpu_status gst = CheckGenerated(ctx, s, man, nm);
+        if (gst != BEPUGPU_OK) return gst;
+    }
+    // The records are accepted: the scene changes from here on.
+    s->colouring = std::move(colouring);
     s->colouringOnDevice = false;
     // Manifold and joint slots: the colour-sweep part in colour-major order,
     // then the island groups (groups.cu); the persistent mode keeps everything

@@ -567,9 +567,11 @@ struct Context {
 Scene* FindScene(Context* ctx, int32_t id);
 bepugpu_status SceneMissing(Context* ctx, int32_t id);
 
-// Narrow phase (collide.cu).  Checks the GENERATED manifolds of a constraint
-// upload against the scene's shapes and their contact_order fields, and
+// Narrow phase (collide.cu).  CheckGenerated checks the GENERATED manifolds of a
+// constraint upload (their bodies in range) against the scene's shapes and their
+// contact_order fields, before the upload changes anything; PrepareGenerated
 // stores their slots; LaunchCollide runs the narrow phase over them.
+bepugpu_status CheckGenerated(Context* ctx, const Scene* s, const bepugpu_manifold* man, uint32_t nm);
 bepugpu_status PrepareGenerated(Context* ctx, Scene* s, const bepugpu_manifold* man, uint32_t nm,
                                 const std::vector<int32_t>& slotOf);
 cudaError_t LaunchCollide(Scene* s, const StepParams& p, cudaStream_t stream);

@@ -59,10 +59,7 @@ bool PairShapesFit(const bepugpu_shape& a, const bepugpu_shape& b) {
 
 }  // namespace
 
-bepugpu_status PrepareGenerated(Context* ctx, Scene* s, const bepugpu_manifold* man, uint32_t nm,
-                                const std::vector<int32_t>& slotOf) {
-    std::vector<int32_t> slots;
-    std::vector<int2> pairs;
+bepugpu_status CheckGenerated(Context* ctx, const Scene* s, const bepugpu_manifold* man, uint32_t nm) {
     for (uint32_t i = 0; i < nm; i++) {
         const bepugpu_manifold& r = man[i];
         if (!(r.flags & BEPUGPU_MANIFOLD_GENERATED)) continue;
@@ -94,10 +91,19 @@ bepugpu_status PrepareGenerated(Context* ctx, Scene* s, const bepugpu_manifold* 
                           r.contact_count);
             return BEPUGPU_INVALID_ARGUMENT;
         }
-        slots.push_back(slotOf[i]);
-        pairs.push_back(make_int2(r.body_a, r.body_b));
     }
-    s->hostGenPairs = pairs;
+    return BEPUGPU_OK;
+}
+
+bepugpu_status PrepareGenerated(Context* ctx, Scene* s, const bepugpu_manifold* man, uint32_t nm,
+                                const std::vector<int32_t>& slotOf) {
+    std::vector<int32_t> slots;
+    s->hostGenPairs.clear();
+    for (uint32_t i = 0; i < nm; i++) {
+        if (!(man[i].flags & BEPUGPU_MANIFOLD_GENERATED)) continue;
+        slots.push_back(slotOf[i]);
+        s->hostGenPairs.push_back(make_int2(man[i].body_a, man[i].body_b));
+    }
     std::sort(slots.begin(), slots.end());  // ascending slots: neighbouring threads read neighbouring lanes
     s->generatedCount = (int32_t)slots.size();
     if (!slots.empty()) {
