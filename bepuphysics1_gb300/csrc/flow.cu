@@ -682,6 +682,7 @@ cudaError_t StatusWords::Take(int** word) {
         const cudaError_t e = cudaHostAlloc((void**)&page, sizeof(int) * kWords, cudaHostAllocMapped);
         if (e != cudaSuccess) return e;
         pages_.push_back(page);
+        free_.reserve(kWords * pages_.size());  // Give never allocates
         for (int k = kWords - 1; k >= 0; k--) free_.push_back(page + k);
     }
     *word = free_.back();

@@ -637,7 +637,8 @@ bepugpu_status bepugpu_colour_list(const int32_t* body_a, const int32_t* body_b,
  * the first of the scene's calls that hand out results returns TIMEOUT, with
  * the state as the step left it (bepugpu_step_state, bepugpu_step_host, the
  * download calls, bepugpu_get_islands, bepugpu_batch_step; bepugpu_synchronize
- * for all scenes; the completion of a served request). */
+ * for all scenes; the completion of a served request).  In the persistent mode
+ * a wait that ran out is reported by bepugpu_synchronize alone. */
 bepugpu_status bepugpu_step(bepugpu_context* ctx, int32_t scene, float dt, uint32_t flags);
 bepugpu_status bepugpu_set_solve_mode(bepugpu_context* ctx, int32_t scene, int32_t mode);
 /* Island groups.  An island (dynamic bodies connected through constraints)

@@ -132,6 +132,7 @@ def test_scenes_without_sweeps_hold_no_tables(gpu_context):
     constraints that need them and stay."""
     gpu_context.set_settings(default_settings())
     b, m = scenes.make_tower(150, seed=6)[:2]  # one island group by default
+    GpuSpace(gpu_context, b, m).close()  # blocks that an earlier test's spills left pending are reclaimed here
 
     def bytes_of(make):
         before = gpu_context.memory_usage()[1]
